@@ -8,8 +8,8 @@
 // the origin's plain `linear` (origin/model.py:108-120).
 //
 // Same skeleton as the FP8 and NVFP4 GEMMs of this library: swap-AB (UMMA M = 128 weight rows,
-// UMMA N = padded M), stream-K over the flat (weight tile, 64-wide K block) list, one TMA
-// instruction per unit (weight tile and activation tile, one lane each), four
+// UMMA N = padded M), stream-K over the flat (weight tile, 64-wide K block) list, an elected thread starts
+// a unit's two copies (weight tile and activation tile), four
 // tcgen05.mma kind::f16 (K = 16) per unit.  Nothing is rescaled between K blocks, so a tile
 // accumulates over its whole K range in TMEM and the epilogue runs once per segment; two issuer
 // threads take units alternately into two TMEM tiles that the epilogue adds.  Partial tiles go
@@ -29,7 +29,7 @@ namespace gemm16 {
 constexpr int kTileN = 128;          // weight rows per tile (UMMA M)
 constexpr int kBlockK = 64;          // K elements per unit = 128 bytes per row
 constexpr int kRowBytes = 128;
-constexpr int kProducers = 4;        // warps 0..3: starting a unit's copies costs a warp several hundred cycles
+constexpr int kProducers = 4;        // warps 0..3
 constexpr int kIssuers = 2;          // warps 2, 3: each accumulates its own units into its own TMEM tile
 constexpr int kFirstEpiWarp = 8;     // warps 8..11 (6 and 7 idle: the TMEM lane quarter of a warp is warp % 4)
 constexpr int kEpiWarps = 4;
@@ -165,15 +165,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
             const int s = ring.idx;
             alive = mbar_wait_lane0(empty + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty);
             if (!alive) break;
-            if (lane == 0) mbar_arrive_expect_tx(full + s * 8, L::kStageBytes);
-            __syncwarp();
-            // one instruction, two lanes: lane 0 fetches the weight tile, lane 1 the activations
             const uint32_t stage = base + s * L::kStageBytes;
-            const uint32_t dst = stage + (lane == 1 ? kWBytes : 0);
-            const void* map = lane == 1 ? static_cast<const void*>(&a_map) : static_cast<const void*>(&w_map);
-            if (lane < 2)
-                tma_load_2d_hint(dst, map, full + s * 8, kb * kBlockK, lane == 1 ? 0 : tile * kTileN,
-                                 lane == 1 ? keep_policy : stream_policy);
+            if (elect_one()) {
+                mbar_arrive_expect_tx(full + s * 8, L::kStageBytes);
+                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kBlockK, tile * kTileN, stream_policy);
+                tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, kb * kBlockK, 0, keep_policy);
+            }
+            __syncwarp();
             ring.step(kProd, S);
             kb += kProd;
             while (kb >= p.kb) {
@@ -186,7 +184,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constan
         // Issuer i takes units n with n % 2 == i and accumulates them into its own TMEM tile; the
         // epilogue adds the two tiles.  (Two threads must not chain accumulations into one tile:
         // only operations of one thread are ordered.)
-        if (lane == 0) {
+        if (elect_one()) {
             const int me = warp - kIssuer0;
             // kind::f16 with BF16 operands (format 1), fp32 accumulator, both operands K-major
             constexpr uint32_t idesc = umma_idesc(kTileN, M_PAD, 1, 1);

@@ -19,7 +19,7 @@
 //    a range that does not start a tile's K range writes its fp32 partial to the CTA's own
 //    scratch slot in global memory and raises a flag; the CTA holding the start of the
 //    range adds the partials in CTA order (deterministic) and writes the bf16 tile;
-//  * per unit: one TMA instruction fetches the weight tile (128 x 128 B) and the
+//  * per unit: an elected thread fetches the weight tile (128 x 128 B) and the
 //    activation tile (M_PAD x 128 B), four tcgen05.mma kind::f8f6f4 fill a fresh TMEM
 //    stage, and an epilogue warpgroup adds the stage, times the unit's scales, to its register
 //    accumulators.  One unit's epilogue is a chain of waits (scales, TMEM stage, tcgen05.ld), so
@@ -246,34 +246,28 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         int tile = static_cast<int>((u0 + me) / p.kb), kb = static_cast<int>((u0 + me) % p.kb);
         bool alive = true;
         if (resident && count > 0) {
-            // this producer's share of the activation tiles (K blocks me, me + kProducers, ..), one lane
-            // per tile in a single instruction
+            // this producer's share of the activation tiles (K blocks me, me + kProducers, ..)
             const int mine = me < p.kb ? (p.kb - me + kProducers - 1) / kProducers : 0;
-            if (lane == 0) {
+            if (elect_one()) {
                 if (mine > 0) mbar_arrive_expect_tx(a_full, static_cast<uint32_t>(mine) * L::kABytes);
                 else mbar_arrive(a_full);
+                for (int kbj = me; kbj < p.kb; kbj += kProducers)
+                    tma_load_2d_hint(a_res + kbj * L::kABytes, &a_map, a_full, kbj * kBlockK, 0, keep_policy);
             }
             __syncwarp();
-            for (int j0 = 0; j0 < mine; j0 += 32) {
-                const int j = j0 + static_cast<int>(lane);
-                const int kbj = me + j * kProducers;
-                if (j < mine) tma_load_2d_hint(a_res + kbj * L::kABytes, &a_map, a_full, kbj * kBlockK, 0, keep_policy);
-            }
         }
-        const uint32_t lanes_loading = resident ? 1u : 2u;
         for (int n = me; n < count && alive; n += kProducers) {
             const int s = ring.idx;
             alive = mbar_wait_lane0(empty + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty);
             if (!alive) break;
-            if (lane == 0) mbar_arrive_expect_tx(full + s * 8, stage_bytes);
-            __syncwarp();
-            // one instruction, two lanes: lane 0 fetches the weight tile, lane 1 the activations
-            const uint32_t dst = base + s * stage_bytes + (lane == 1 ? kWBytes : 0);
-            const void* map = lane == 1 ? static_cast<const void*>(&a_map) : static_cast<const void*>(&w_map);
+            const uint32_t stage = base + s * stage_bytes;
             const int a_x = kb * kBlockK + (p.group_tiles ? (tile / p.group_tiles) * p.K : 0);
-            if (lane < lanes_loading)
-                tma_load_2d_hint(dst, map, full + s * 8, lane == 1 ? a_x : kb * kBlockK, lane == 1 ? 0 : tile * kTileN,
-                                 lane == 1 ? keep_policy : stream_policy);
+            if (elect_one()) {
+                mbar_arrive_expect_tx(full + s * 8, stage_bytes);
+                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kBlockK, tile * kTileN, stream_policy);
+                if (!resident) tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, a_x, 0, keep_policy);
+            }
+            __syncwarp();
             ring.step(kProducers, S);
             kb += kProducers;
             while (kb >= p.kb) {
@@ -283,7 +277,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         }
     } else if (warp < kProducers + kIssuers) {
         // ------------------------------------------------------------ UMMA issuers (one thread each)
-        if (lane == 0) {
+        if (elect_one()) {
             const int me = warp - kProducers;
             constexpr uint32_t idesc = umma_idesc(kTileN, M_PAD, 0, 0);
             Ring ring, tring;

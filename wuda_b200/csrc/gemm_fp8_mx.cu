@@ -13,7 +13,7 @@
 // segment.
 //
 // Skeleton as in the other GEMMs of this library: swap-AB (UMMA M = 128 weight rows, UMMA N = padded M), stream-K
-// over the flat (weight tile, K block) list, one TMA instruction per unit, two issuer warps that take units
+// over the flat (weight tile, K block) list, two issuer warps that take units
 // alternately into their own TMEM tiles, partial tiles through per-CTA scratch slots added in CTA order, bounded
 // waits.  New here:
 //   * The scale images.  A unit (128 x 128 bytes) is four MMAs of K = 32; their scale bytes are the four bytes
@@ -274,10 +274,12 @@ gemm_fp8_mx_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         float a_now[kRowsPerLane], a_next[kRowsPerLane];
         load_scales(tile, kb, a_now);
         if (RES && me == 0 && count > 0) {   // the whole activation matrix, once (plain form: one group)
-            if (lane == 0) mbar_arrive_expect_tx(a_full, p.kb * L::kABytes);
+            if (elect_one()) {
+                mbar_arrive_expect_tx(a_full, p.kb * L::kABytes);
+                for (int k = 0; k < p.kb; ++k)
+                    tma_load_2d_hint(a_res + k * L::kABytes, &a_map, a_full, k * kRowBytes, 0, keep_policy);
+            }
             __syncwarp();
-            for (int k = static_cast<int>(lane); k < p.kb; k += 32)
-                tma_load_2d_hint(a_res + k * L::kABytes, &a_map, a_full, k * kRowBytes, 0, keep_policy);
         }
         for (int n = me; n < count && alive; n += kProd) {
             const int s = ring.idx;
@@ -289,17 +291,15 @@ gemm_fp8_mx_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
             load_scales(tile_next, kb_next, a_next);
             alive = mbar_wait_lane0(empty + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty);
             if (!alive) break;
-            if (lane == 0) mbar_arrive_expect_tx(full + s * 8, (W4 ? kWBytes / 2 : kWBytes) + (RES ? 0 : L::kABytes));
-            __syncwarp();
-            // one instruction, two lanes: lane 0 fetches the weight tile, lane 1 the activations of the tile's group
             const uint32_t stage = base + s * L::kStageBytes;
             uint8_t* stage_ptr = base_ptr + s * L::kStageBytes;
             const int group = tile / p.tiles_per_group;
-            const uint32_t dst = stage + (lane == 1 ? kWBytes : 0);
-            const void* map = lane == 1 ? static_cast<const void*>(&a_map) : static_cast<const void*>(&w_map);
-            if (lane < (RES ? 1u : 2u))
-                tma_load_2d_hint(dst, map, full + s * 8, (lane == 1 ? group * p.kb + kb : kb) * kRowBytes, lane == 1 ? 0 : tile * kTileN,
-                                 lane == 1 ? keep_policy : stream_policy);
+            if (elect_one()) {   // the weight tile and the activations of the tile's group
+                mbar_arrive_expect_tx(full + s * 8, (W4 ? kWBytes / 2 : kWBytes) + (RES ? 0 : L::kABytes));
+                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kRowBytes, tile * kTileN, stream_policy);
+                if (!RES) tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, (group * p.kb + kb) * kRowBytes, 0, keep_policy);
+            }
+            __syncwarp();
             // scale images: lane l writes row l of each (16 bytes: the words of rows l, l + 32, l + 64, l + 96)
             if constexpr (W4) {
                 cp_async_wait<kSfDepth - 1>();      // this unit's words have landed (a lane reads only what it fetched)
@@ -337,7 +337,7 @@ gemm_fp8_mx_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         // Issuer i takes units n with n % 2 == i and accumulates them into its own TMEM tile; the epilogue adds the
         // two tiles.  (Two threads must not chain accumulations into one tile: only operations of one thread are
         // ordered.)
-        if (lane == 0) {
+        if (elect_one()) {
             const int me = warp - kIssuer0;
             const uint32_t sfw_t = tmem_base + L::kAccCols + me * 16;
             const uint32_t sfa_t = sfw_t + 8;

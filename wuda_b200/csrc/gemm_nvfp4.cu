@@ -12,8 +12,8 @@
 // them from TMEM, where tcgen05.cp puts them from shared memory, so a tile accumulates over its whole
 // K range in TMEM and the epilogue runs once per tile (times gs_a * gs_w, to bf16).  Everything else
 // follows the FP8 GEMM of this library: swap-AB (UMMA M = 128 weight rows, UMMA N = padded M),
-// stream-K over the flat (weight tile, 256-wide K block) list, one TMA instruction per unit (weights,
-// activations and both scale blocks, one lane each), partial tiles through per-CTA scratch slots
+// stream-K over the flat (weight tile, 256-wide K block) list, an elected thread starts a unit's four copies (weights,
+// activations and both scale blocks), partial tiles through per-CTA scratch slots
 // added in CTA order, bounded waits.
 //
 // Scale layout in global memory ("packed"): per 128 rows x 256 K one 2 KB block
@@ -34,7 +34,7 @@ namespace gemm4 {
 constexpr int kTileN = 128;          // weight rows per tile (UMMA M)
 constexpr int kBlockK = 256;         // K elements per unit = 128 bytes per row
 constexpr int kRowBytes = 128;
-constexpr int kProducers = 4;        // warps 0..3: a warp needs ~1000 cycles to start a unit's four copies, a unit lasts ~800
+constexpr int kProducers = 4;        // warps 0..3
 constexpr int kIssuers = 2;          // warps 2, 3: each accumulates its own units into its own TMEM tile
 constexpr int kFirstEpiWarp = 8;     // warps 8..11 (6 and 7 idle: the TMEM lane quarter of a warp is warp % 4)
 constexpr int kEpiWarps = 4;
@@ -189,12 +189,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             const int s = ring.idx;
             alive = mbar_wait_lane0(empty + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty);
             if (!alive) break;
-            if (lane == 0) mbar_arrive_expect_tx(full + s * 8, L::kStageBytes);
-            __syncwarp();
-            // one instruction, four lanes: weights, activations, weight scales, activation scales
             const uint32_t stage = base + s * L::kStageBytes;
-            uint32_t dst = stage;
-            const void* map = &w_map;
             // grouped: `tile` is the flat index; the weight tile is the expert's, the activations the group's
             // (the group's expert is looked up only when the group changes: a dependent global load per
             // unit would sit in the producer's critical path)
@@ -209,26 +204,15 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
             } else if (!grouped) {
                 wtile = tile;
             }
-            int c0 = kb * kRowBytes, c1 = wtile * kTileN;
-            uint64_t policy = stream_policy;
-            if (lane == 1) {
-                dst = stage + kWBytes;
-                map = &a_map;
-                c1 = grp * M_PAD;
-                policy = keep_policy;
-            } else if (lane == 2) {
-                dst = stage + kWBytes + L::kABytes;
-                map = &wsf_map;
-                c0 = 0;
-                c1 = (wtile * p.kb + kb) * 4;
-            } else if (lane == 3) {
-                dst = stage + kWBytes + L::kABytes + kSfBytes;
-                map = &asf_map;
-                c0 = 0;
-                c1 = (grp * p.kb + kb) * 4;
-                policy = keep_policy;
+            if (elect_one()) {
+                mbar_arrive_expect_tx(full + s * 8, L::kStageBytes);
+                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kRowBytes, wtile * kTileN, stream_policy);
+                tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, kb * kRowBytes, grp * M_PAD, keep_policy);
+                tma_load_2d_hint(stage + kWBytes + L::kABytes, &wsf_map, full + s * 8, 0, (wtile * p.kb + kb) * 4, stream_policy);
+                tma_load_2d_hint(stage + kWBytes + L::kABytes + kSfBytes, &asf_map, full + s * 8, 0, (grp * p.kb + kb) * 4,
+                                 keep_policy);
             }
-            if (lane < 4) tma_load_2d_hint(dst, map, full + s * 8, c0, c1, policy);
+            __syncwarp();
             ring.step(kProd, S);
             kb += kProd;
             while (kb >= p.kb) {
@@ -241,7 +225,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_consta
         // Issuer i takes units n with n % 2 == i and accumulates them into its own TMEM tile; the
         // epilogue adds the two tiles.  (Two threads must not chain accumulations into one tile:
         // only operations of one thread are ordered.)
-        if (lane == 0) {
+        if (elect_one()) {
             const int me = warp - kIssuer0;
             // kind::mxf4nvf4: formats e2m1 (1), scale format ue4m3 (0), both operands K-major
             constexpr uint32_t idesc = umma_idesc_block_scaled(kTileN, M_PAD, 1, 1, 0, 0, 0);

@@ -378,20 +378,16 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     // walks on to the end of the range so that it enters (and thereby releases) every request in it.
     if (warp < kProducers) {
         // ------------------------------------------------------------ producers
-        // All copies of an item (key rows and scale words of every page) go out as ONE tensor-copy instruction
-        // with one lane per copy.
+        // An elected thread starts all copies of an item (key rows and scale words of every page); the page numbers
+        // come to it by shuffles.
         const int me = warp;
         const uint64_t stream_policy = policy_evict_first();
+        constexpr int kMaxPages = 8;
         const int ppi = kItem / p.epb;                   // pages per item: 8, 4, 2 or 1
         const int ppi_shift = ppi == 8 ? 3 : (ppi == 4 ? 2 : (ppi == 2 ? 1 : 0));
         const uint32_t page_bytes = p.epb * kRowBytes;
         const uint32_t page_scale_bytes = p.epb * 4;
         const int pg = static_cast<int>(lane) & (ppi - 1);   // this lane's page inside the item
-        const bool is_scale = static_cast<int>(lane) >= ppi;
-        const bool copier = static_cast<int>(lane) < 2 * ppi;
-        const void* my_map = is_scale ? static_cast<const void*>(&sf_map) : static_cast<const void*>(&kv_map);
-        const uint32_t my_dst = (is_scale ? lin_smem + pg * page_scale_bytes : kv_smem + pg * page_bytes);
-        const uint32_t my_stage_bytes = is_scale ? kLinBytes : kKvBytes;
         int qc = 0, pages_b = 0;
         int64_t bt_row = 0;
         // block-table window: 32 entries in use, the next 32 already requested
@@ -402,7 +398,7 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             if (me == 0 && alive) {
                 const int qs = qc & 1;
                 alive = mbar_wait_lane0(empty_q + qs * 8, ((qc >> 1) & 1) ^ 1, abort_flag, p.status, kDevTimeoutEmptyQ);
-                if (alive && lane == 0) {
+                if (alive && elect_one()) {
                     mbar_arrive_expect_tx(full_q + qs * 8, kQBytes + kWBytes);
                     tma_load_2d(q_smem + qs * kQBytes, &q_map, full_q + qs * 8, 0, c.b * kHeads);
                     bulk_load(w_smem + qs * kWBytes, p.weights + static_cast<int64_t>(c.b) * kHeads, kWBytes,
@@ -437,7 +433,7 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 nxt_val = (e1 < pages_b && e1 < p.bt_stride) ? __ldg(p.block_table + bt_row + e1) : -1;
             }
             int phys = __shfl_sync(0xffffffffu, win_val, (first_page + pg - win_base) & 31);
-            const bool mine = copier && pg < valid;
+            const bool mine = static_cast<int>(lane) < valid;
             if (mine && (phys < 0 || phys >= p.num_blocks)) {
                 if (p.status) atomicCAS(p.status, 0, kDevBadPageIndex);
                 phys = 0;
@@ -445,10 +441,20 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             const int s = ring.idx;
             alive = mbar_wait_lane0(empty_kv + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutEmptyKv);
             if (!alive) break;
-            if (lane == 0) mbar_arrive_expect_tx(full_kv + s * 8, valid * (page_bytes + page_scale_bytes));
+            int page[kMaxPages];
+#pragma unroll
+            for (int i = 0; i < kMaxPages; ++i) page[i] = __shfl_sync(0xffffffffu, phys, i);
+            if (elect_one()) {
+                mbar_arrive_expect_tx(full_kv + s * 8, valid * (page_bytes + page_scale_bytes));
+                const uint32_t kv_dst = kv_smem + s * kKvBytes, sf_dst = lin_smem + s * kLinBytes;
+#pragma unroll
+                for (int i = 0; i < kMaxPages; ++i) {
+                    if (i >= valid) break;
+                    tma_load_3d_hint(kv_dst + i * page_bytes, &kv_map, full_kv + s * 8, 0, 0, page[i], stream_policy);
+                    tma_load_3d_hint(sf_dst + i * page_scale_bytes, &sf_map, full_kv + s * 8, 0, 0, page[i], stream_policy);
+                }
+            }
             __syncwarp();
-            if (mine)
-                tma_load_3d_hint(my_dst + s * my_stage_bytes, my_map, full_kv + s * 8, 0, 0, phys, stream_policy);
             ring.step(kProducers, S);
         }
         if (alive && nitems > 0 && at < nitems - 1)
@@ -456,7 +462,7 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     } else if (warp < kFirstScaleWarp) {
         // ------------------------------------------------------------ issuers
         // One thread per warp runs the whole loop; issuer e owns the items n with n % 2 == e and item stage e.
-        if (lane == 0) {
+        if (elect_one()) {
             const int me = warp - kProducers;
             const uint32_t acc = tmem_base + me * 2 * kHeads;
             const uint32_t sfa = tmem_base + kColSfaBase + me * 8;

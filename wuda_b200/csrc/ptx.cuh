@@ -58,6 +58,12 @@ __device__ __forceinline__ uint32_t lane_id() {
     return l;
 }
 
+// The lane that issues a warp's tensor copies and MMAs.  Such an instruction takes its operands from warp-uniform
+// registers: behind `elect.sync` the compiler knows that one lane is active and moves them there directly, behind
+// `lane == 0` (or with operands that differ from lane to lane) it has to walk the active lanes in a loop, which cost
+// about a hundred cycles per instruction.  Measured with nothing else changed: FP8 x FP4 24576 x 7168 at 64 rows
+// 41.1 -> 32.0 us, the whole decode layer at batch 64 / 128 1257 -> 1201 / 1584 -> 1516 us, sparse attention at batch
+// 64 92.3 -> 88.2 us, MXFP4 logits + top-k at batch 64 57.1 -> 53.7 us; results bit-identical.
 __device__ __forceinline__ bool elect_one() {
     uint32_t pred;
     asm volatile(

@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
                                             kDevTimeoutMlaScoresRead);   // the block before, the other issuer's
                 if (!alive) break;
                 tc_fence_after();
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t own_addr = base + kOffOwn + s * kHalfStageBytes, oth_addr = base + kOffOth + t * kHalfStageBytes;
                     // descriptors differ only in their 14-bit address field: one add per MMA
                     const uint64_t own_desc = umma_smem_desc_sw128(own_addr), oth_desc = umma_smem_desc_sw128(oth_addr);
@@ -395,8 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         }
     } else if (warp == kIssuerWarpPV) {
         // ------------------------------------------------------------ weighted-sum issuer
-        // A thread issues an MMA about every hundred cycles whatever its size; with the weighted sums on a thread of
-        // their own the score issuer goes straight on to the next block.
+        // With the weighted sums on a thread of their own the score issuer goes straight on to the next block.
         constexpr uint32_t idesc_pv = umma_idesc_b_mn(kRows, kHalf, 0, 0);
         bool alive = true;
         for (int j = 0; j < blocks && alive; ++j) {
@@ -404,7 +403,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
             alive = mbar_wait_lane0(p_full + t * 8, (j >> 1) & 1u, abort_flag, p.status, kDevTimeoutMlaProbs);
             if (!alive) break;
             tc_fence_after();
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t p_addr = base + kOffP + t * kPBytes;
                 const uint32_t v_addr = base + kOffOwn + s * kHalfStageBytes;
 #pragma unroll
