@@ -1,0 +1,760 @@
+// The GEMM of this library whose accumulation stays in tensor memory, for decode-sized M on sm_100a:
+//
+//   C[M, N] = A[M, K] x W[N, K]^T,   M <= 256
+//
+// in four operand kinds: FP8 or 4-bit weights with power-of-two scales applied by the tensor core (gemm_fp8_mx.cu),
+// NVFP4 (gemm_nvfp4.cu) and BF16 (gemm_bf16.cu); those files describe the formats and hold the entry points.  The FP8
+// GEMM with general scales promotes every K block on CUDA cores and is a kernel of its own (gemm_fp8.cu).
+//
+// What bounds it: the weight stream.  A unit is one weight tile, 128 rows x 128 bytes of K, and the activation rows of
+// the same K range.  A probe that only streams units (TMA, no MMA) brings 24576 x 7168 bytes in 28-30 us (5.8-6.2 TB/s)
+// beside 0 to 128 activation rows and in 32.8 us beside 256: an SM takes in up to 110 bytes per ns, so re-reading the
+// activations from L2 with every weight tile is cheap and nothing is kept resident or shared between CTAs.
+//
+//   * swap-AB: weight rows are the MMA's M = 128, activation rows (rounded up to 16, not to a power of two) its N.
+//   * one elected thread fetches (as many stages as fit, 4 to 12), one issues the MMAs into one accumulator, which is
+//     double-buffered up to 128 rows; all rows up to 256 go in ONE pass over the weights.
+//   * block scales of the FP8 / 4-bit kinds are exponent bytes in tensor memory.  A 32-bit scale column holds four
+//     consecutive K blocks (the MMA's scale id picks one), so two warps build ONE image per four units, from scales
+//     they requested sixteen units earlier; the fetching and the issuing thread never wait for scale arithmetic.
+//   * work split.  Weight tiles enough for every SM: stream-K, i.e. the flat unit list in equal contiguous ranges; a
+//     range that starts inside a tile leaves its partial sums in its scratch slot and the CTA with the tile's start
+//     adds them in CTA order - it comes to that tile last, the partial was finished first.  Few tiles ("split"): the
+//     same number of CTAs for every tile, each with one K range; all leave their partial sums, and once the tile's
+//     counter is complete each CTA adds one slice of the tile over all partials, in order - instead of one CTA adding
+//     seven or more whole partials one after the other.  Both orders are fixed: results do not depend on timing.
+//   * before it waits for the kernel ahead (programmatic launch) a CTA asks L2 for its first weight tiles, so a chain
+//     of small kernels hides the start of the weight stream.  A prefetch into L2 is a hint: it reads nothing into the
+//     SM, so weights written by an earlier kernel of the chain are still seen.
+// Every wait is bounded.
+#pragma once
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include "host.h"
+#include "ptx.cuh"
+
+namespace wuda {
+namespace gemmtc {
+
+enum class Kind { kMx8, kMx8W4, kNv4, kBf16 };
+
+constexpr int kTileN = 128;                   // weight rows per tile (UMMA M)
+constexpr int kRowBytes = 128;                // K bytes of a unit: 128 e4m3, 256 e2m1, 64 bf16
+constexpr int kWBytes = kTileN * kRowBytes;   // 16 KB
+constexpr int kMaxStages = 12;
+// The grouped form streams for hundreds of microseconds, and there more copies in flight cost bandwidth: routed experts of
+// 64 tokens (5.65 GB) 924 us with 10 stages, 892 with 8, 877 with 6, 905 with 5, 939 with 4.  The dense calls are too short
+// for that (24576 x 7168 NVFP4 at 8 rows 20.8 us with 8 to 10 stages, 21.8 with 6).
+constexpr int kGroupedStages = 6;
+constexpr int kImgSlots = 4;
+constexpr int kImgBlock = 512;                // scale bytes of 128 rows, four bytes each: [row % 32][row / 32]
+constexpr int kNvSfBytes = 2048;              // NVFP4: packed scales of 128 rows x 256 K
+constexpr int kMaxGrid = 192;
+constexpr int kMaxTileSplit = 32;
+constexpr int64_t kFlagBytes = 1024;          // the flags lead the scratch, whatever the shape (kernels share scratches)
+
+struct Params {
+    void* c;
+    int c_is_fp32;
+    float* scratch;            // [grid] partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]
+    int32_t* flags;            // stream-K: one flag per CTA; split: one counter per weight tile
+    int32_t* status;
+    int M, N, kb, n_tiles;     // kb = units per weight tile
+    int a_rows;                // M rounded up to 16
+    int stages;
+    int split;                 // CTAs per weight tile, 0 = stream-K
+    // power-of-two scaled kinds
+    const float* a_scales;     // [M, scale_cols]
+    const float* w_scales;     // [n_tiles, kb] (FP8 weights)
+    const uint8_t* w_sf;       // 4-bit weights: [N, sf_stride] exponent bytes, one per weight row and 32 K-elements
+    int sf_stride;
+    int tiles_per_group;       // tile t reads the activations from K block (t / tiles_per_group) * kb on
+    int scale_cols;
+    int vec_scales;            // rows of a_scales (and w_sf) can be read 16 bytes at a time
+    // NVFP4
+    float out_scale;
+    const int32_t* group_expert;   // grouped form (routed experts): [num_groups], else NULL; see gemm_nvfp4.cu
+    const int32_t* row_token;
+    const int32_t* num_groups;
+    const float* expert_scale;
+};
+
+template <Kind KIND, int M_PAD>
+struct Layout {
+    static constexpr bool kMx = KIND == Kind::kMx8 || KIND == Kind::kMx8W4;
+    static constexpr int kBlocks = (M_PAD + 127) / 128;               // 128-row blocks of activation scales
+    static constexpr int kBuffers = M_PAD <= 128 ? 2 : 1;
+    static constexpr int kEpiWarps = M_PAD >= 128 ? 8 : 4;
+    static constexpr int kThreads = 32 * (4 + kEpiWarps);
+    static constexpr int kCols = M_PAD / (kEpiWarps / 4);             // accumulator columns per epilogue thread
+    // scale columns of one set (two sets alternate)
+    static constexpr int kSfwCols = kMx ? 4 : (KIND == Kind::kNv4 ? 16 : 0);
+    static constexpr int kSfaCols = kSfwCols * kBlocks;
+    static constexpr int kAccCols = kBuffers * M_PAD;
+    static constexpr int kUsedCols = kAccCols + 2 * (kSfwCols + kSfaCols);
+    static constexpr int kTmemCols = kUsedCols <= 32 ? 32 : (kUsedCols <= 64 ? 64 : (kUsedCols <= 128 ? 128 : (kUsedCols <= 256 ? 256 : 512)));
+    static constexpr int kImgW = KIND == Kind::kMx8W4 ? 4 * kImgBlock : kImgBlock;    // weight part of an image slot
+    static constexpr int kImgBytes = kMx ? kImgW + kBlocks * kImgBlock : 0;
+    static __host__ __device__ constexpr int stage_bytes(int a_rows) {
+        return kWBytes + a_rows * kRowBytes + (KIND == Kind::kNv4 ? kNvSfBytes * (1 + kBlocks) : 0);
+    }
+    static __host__ __device__ constexpr int img_off(int stages, int a_rows) { return stages * stage_bytes(a_rows); }
+    static __host__ __device__ constexpr int bar_off(int stages, int a_rows) { return img_off(stages, a_rows) + kImgSlots * kImgBytes; }
+    // barriers: full[12] empty[12] img_full[4] img_empty[4] full_tm[2] empty_tm[2]
+    static constexpr int kBars = 2 * kMaxStages + 2 * kImgSlots + 4;
+    static __host__ __device__ constexpr int misc_off(int stages, int a_rows) { return bar_off(stages, a_rows) + kBars * 8; }
+    static __host__ __device__ constexpr int total(int stages, int a_rows) { return misc_off(stages, a_rows) + 16 + 1024; }
+};
+
+__device__ __forceinline__ void st_release_gpu(int32_t* p, int v) {
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_acquire_gpu(const int32_t* p) {
+    int v;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ int add_acq_rel_gpu(int32_t* p, int v) {
+    int old;
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    return old;
+}
+__device__ __forceinline__ long long range_begin(long long units, int c, int grid) { return units * c / grid; }
+__device__ __forceinline__ int cta_of(long long units, long long u, int grid) {
+    int c = static_cast<int>(u * grid / units);
+    while (c + 1 < grid && range_begin(units, c + 1, grid) <= u) ++c;
+    while (c > 0 && range_begin(units, c, grid) > u) --c;
+    return c;
+}
+
+// Exponent byte of a power-of-two fp32 scale; anything else is reported and truncated to the power of two below.
+__device__ __forceinline__ uint32_t exponent_byte(float scale, int32_t* status) {
+    const uint32_t bits = __float_as_uint(scale);
+    if (((bits & 0x807fffffu) != 0u || (bits >> 23) == 0xffu) && scale != 0.f && status)
+        atomicCAS(status, 0, static_cast<int>(kDevScaleNotPow2));
+    const uint32_t e = (bits >> 23) & 0xffu;
+    return e == 0xffu ? 0xfeu : e;
+}
+
+__device__ __forceinline__ void umma_mxf8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem,
+                                          uint32_t sfb_tmem, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t"
+        ".reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale.scale_vec::1X "
+        "[%0], %1, %2, %3, [%5], [%6], p;\n\t"
+        "}\n"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(sfa_tmem), "r"(sfb_tmem)
+        : "memory");
+}
+
+template <Kind KIND>
+__device__ __forceinline__ uint32_t to_bf16x2(float a, float b, float scale) {
+    if (KIND == Kind::kNv4) a *= scale, b *= scale;
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return reinterpret_cast<const uint32_t&>(v);
+}
+// Four lanes (rows r = lane & 3) hold columns 0..3 as two pairs of 16 bits; lane r leaves with column r of the four rows.
+__device__ __forceinline__ void transpose4(uint32_t c01, uint32_t c23, uint32_t lane, uint32_t& rows01, uint32_t& rows23) {
+    const bool up = (lane & 2u) != 0u, odd = (lane & 1u) != 0u;
+    const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? c01 : c23, 2);
+    const uint32_t near = up ? got : c01, far = up ? c23 : got;     // this lane's column pair of rows (r & 1) and (r & 1) + 2
+    const uint32_t low = __byte_perm(near, far, 0x5410), high = __byte_perm(near, far, 0x7632);
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, odd ? low : high, 1);
+    const uint32_t even_rows = odd ? other : low, odd_rows = odd ? high : other;   // rows (0, 2) and (1, 3) of the lane's column
+    rows01 = __byte_perm(even_rows, odd_rows, 0x5410);
+    rows23 = __byte_perm(even_rows, odd_rows, 0x7632);
+}
+
+// One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter).
+template <typename Pred>
+__device__ __forceinline__ void await_word(const int32_t* word, Pred done, volatile int* abort_flag, int32_t* status) {
+    if (done(ld_acquire_gpu(word))) return;
+    const unsigned long long start = globaltimer_ns();
+    uint32_t spins = 0;
+    while (!done(ld_acquire_gpu(word))) {
+        if ((++spins & 255u) == 0u && (*abort_flag || globaltimer_ns() - start > kWaitLimitNs)) {
+            *abort_flag = 1;
+            if (status) atomicCAS(status, 0, static_cast<int>(kDevTimeoutPeerFlag));
+            break;
+        }
+    }
+}
+
+template <Kind KIND, int M_PAD>
+__global__ void __launch_bounds__(Layout<KIND, M_PAD>::kThreads, 1)
+gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
+               const __grid_constant__ CUtensorMap wsf_map, const __grid_constant__ CUtensorMap asf_map, const Params p) {
+    using L = Layout<KIND, M_PAD>;
+    constexpr bool kMx = L::kMx;
+    constexpr int kBuffers = L::kBuffers;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - raw_addr);
+    const int S = p.stages;
+    const uint32_t stage_bytes = L::stage_bytes(p.a_rows);
+    const uint32_t bars = base + L::bar_off(S, p.a_rows);
+    const uint32_t full = bars, empty = full + kMaxStages * 8, img_full = empty + kMaxStages * 8, img_empty = img_full + kImgSlots * 8,
+                   full_tm = img_empty + kImgSlots * 8, empty_tm = full_tm + 16;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, p.a_rows));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 4);
+
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+    const uint32_t lane = lane_id();
+
+    if (threadIdx.x == 0) {
+        *abort_flag = 0;
+        for (int i = 0; i < S; ++i) {
+            mbar_init(full + i * 8, 1);
+            mbar_init(empty + i * 8, 1);
+        }
+        for (int i = 0; i < kImgSlots; ++i) {
+            mbar_init(img_full + i * 8, 1);
+            mbar_init(img_empty + i * 8, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(full_tm + b * 8, 1);               // a segment's accumulator is complete
+            mbar_init(empty_tm + b * 8, L::kEpiWarps);   // the epilogue has read it
+        }
+        fence_mbar_init();
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), L::kTmemCols);
+        tmem_relinquish();
+    }
+    const bool grouped = KIND == Kind::kNv4 && p.group_expert != nullptr;
+    // the unit range of this CTA (the grouped form learns its number of units from the kernel ahead)
+    long long units = static_cast<long long>(p.n_tiles) * p.kb, u0 = 0;
+    int grid = static_cast<int>(gridDim.x), count = 0;
+    if (!grouped) {
+        if (p.split > 0) {
+            const int tile = static_cast<int>(blockIdx.x) / p.split, j = static_cast<int>(blockIdx.x) - tile * p.split;
+            const int k0 = p.kb * j / p.split;
+            u0 = static_cast<long long>(tile) * p.kb + k0;
+            count = p.kb * (j + 1) / p.split - k0;
+        } else {
+            u0 = range_begin(units, blockIdx.x, grid);
+            count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
+        }
+    }
+    if (warp == 0 && elect_one()) {
+        prefetch_tmap(&w_map);
+        prefetch_tmap(&a_map);
+        if constexpr (KIND == Kind::kNv4) {
+            prefetch_tmap(&wsf_map);
+            prefetch_tmap(&asf_map);
+        }
+        if constexpr (KIND != Kind::kMx8W4) {
+            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+            for (int n = 0; n < count && n < S; ++n) {
+                tma_prefetch_2d(&w_map, kb * (KIND == Kind::kBf16 ? kRowBytes / 2 : kRowBytes), tile * kTileN);
+                if (++kb == p.kb) kb = 0, ++tile;
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    // all of the above ran while the kernel ahead was still finishing; its results are read from here on
+    pdl_launch_dependents();
+    pdl_wait();
+
+    if (grouped) {
+        // Only the first min(grid, units) CTAs take part: every participating CTA then owns at least one unit, which
+        // the fix-up relies on when it waits for the CTAs that share a tile.
+        units *= *p.num_groups;
+        if (units < grid) grid = static_cast<int>(units);
+        if (static_cast<int>(blockIdx.x) < grid) {
+            u0 = range_begin(units, blockIdx.x, grid);
+            count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
+        }
+    }
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ copies
+        if (elect_one()) {
+            const uint64_t stream_policy = policy_evict_first();
+            const uint64_t keep_policy = policy_evict_last();
+            const uint32_t tx = stage_bytes - (KIND == Kind::kMx8W4 ? kWBytes / 2 : 0);   // packed weights: the padding is not counted
+            int s = 0;
+            uint32_t phase = 1;
+            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+            int seen_tile = -1, grp = grouped ? -1 : 0, expert = 0, wtile = 0;
+            for (int n = 0; n < count; ++n) {
+                // grouped: `tile` is the flat index; the weight tile is the expert's, the activations the group's
+                // (looked up only when the tile changes)
+                if (grouped && tile != seen_tile) {
+                    seen_tile = tile;
+                    const int g_now = tile / p.n_tiles;
+                    if (g_now != grp) {
+                        grp = g_now;
+                        expert = __ldcg(p.group_expert + grp);   // written by the dispatch kernel of the same chain
+                    }
+                    wtile = expert * p.n_tiles + (tile - grp * p.n_tiles);
+                } else if (!grouped) {
+                    wtile = tile;
+                }
+                if (!mbar_wait(empty + s * 8, phase, abort_flag, p.status, kDevTimeoutGemmEmpty)) break;
+                const uint32_t stage = base + s * stage_bytes, bar = full + s * 8, a_bytes = p.a_rows * kRowBytes;
+                mbar_arrive_expect_tx(bar, tx);
+                if constexpr (kMx) {
+                    tma_load_2d_hint(stage, &w_map, bar, kb * kRowBytes, wtile * kTileN, stream_policy);
+                    tma_load_2d_hint(stage + kWBytes, &a_map, bar, ((tile / p.tiles_per_group) * p.kb + kb) * kRowBytes, 0, keep_policy);
+                } else if constexpr (KIND == Kind::kNv4) {
+                    tma_load_2d_hint(stage, &w_map, bar, kb * kRowBytes, wtile * kTileN, stream_policy);
+                    tma_load_2d_hint(stage + kWBytes, &a_map, bar, kb * kRowBytes, grp * M_PAD, keep_policy);
+                    const uint32_t sf = stage + kWBytes + a_bytes;
+                    tma_load_2d_hint(sf, &wsf_map, bar, 0, (wtile * p.kb + kb) * 4, stream_policy);
+#pragma unroll
+                    for (int b = 0; b < L::kBlocks; ++b)   // (a second block exists only where rows beyond 128 do: M_PAD = 256)
+                        tma_load_2d_hint(sf + (1 + b) * kNvSfBytes, &asf_map, bar, 0, ((grp + b) * p.kb + kb) * 4, keep_policy);
+                } else {
+                    tma_load_2d_hint(stage, &w_map, bar, kb * (kRowBytes / 2), wtile * kTileN, stream_policy);
+                    tma_load_2d_hint(stage + kWBytes, &a_map, bar, kb * (kRowBytes / 2), 0, keep_policy);
+                }
+                if (++s == S) s = 0, phase ^= 1u;
+                if (++kb == p.kb) kb = 0, ++tile;
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMAs
+        if (elect_one()) {
+            int s = 0;
+            uint32_t phase = 0, seg = 0, img = 0, nv_set = 0;   // img: images taken so far
+            int kb = static_cast<int>(u0 % p.kb);
+            const uint32_t sf_cols = tmem_base + L::kAccCols;
+            bool alive = true;
+            for (int n = 0; n < count && alive;) {
+                const int seg_len = min(p.kb - kb, count - n);
+                const uint32_t buf = kBuffers == 2 ? (seg & 1u) : 0u;
+                if (seg >= static_cast<uint32_t>(kBuffers)) {   // the epilogue must have drained this buffer's previous segment
+                    if (!mbar_wait(empty_tm + buf * 8, (seg / kBuffers - 1u) & 1u, abort_flag, p.status, kDevTimeoutGemmTmemEmpty)) break;
+                    tc_fence_after();
+                }
+                const uint32_t d = tmem_base + buf * M_PAD;
+                for (int u = 0; u < seg_len; ++u) {
+                    const int k = kb + u;
+                    const uint32_t slot = img & (kImgSlots - 1);
+                    const uint32_t img_addr = base + L::img_off(S, p.a_rows) + slot * L::kImgBytes;
+                    const uint32_t set = (kMx ? img & 1u : nv_set) * (L::kSfwCols + L::kSfaCols);
+                    const uint32_t sfw = sf_cols + set, sfa = sfw + L::kSfwCols;
+                    if constexpr (kMx) {
+                        if (u == 0 || (k & 3) == 0) {   // the first unit of a scale image
+                            if (!mbar_wait(img_full + slot * 8, (img / kImgSlots) & 1u, abort_flag, p.status, kDevTimeoutGemmFull)) {
+                                alive = false;
+                                break;
+                            }
+                            tc_fence_after();
+                            if (KIND == Kind::kMx8) tmem_cp_32x128b_warpx4(sfw, umma_smem_desc_noswz(img_addr, 16, 128));
+#pragma unroll
+                            for (int b = 0; b < L::kBlocks; ++b)
+                                tmem_cp_32x128b_warpx4(sfa + b * 4, umma_smem_desc_noswz(img_addr + L::kImgW + b * kImgBlock, 16, 128));
+                        }
+                    }
+                    if (!mbar_wait(full + s * 8, phase, abort_flag, p.status, kDevTimeoutGemmFull)) {
+                        alive = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t w_addr = base + s * stage_bytes, a_addr = w_addr + kWBytes;
+                    if constexpr (KIND == Kind::kMx8W4)   // every unit has its own weight scales: four bytes per row
+                        tmem_cp_32x128b_warpx4(sfw, umma_smem_desc_noswz(img_addr + (k & 3) * kImgBlock, 16, 128));
+                    if constexpr (KIND == Kind::kNv4) {
+                        const uint32_t sf = a_addr + p.a_rows * kRowBytes;
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {   // 32 rows x 16 bytes per K/64 step; 8-row groups 128 bytes apart
+                            tmem_cp_32x128b_warpx4(sfw + i * 4, umma_smem_desc_noswz(sf + i * 512, 16, 128));
+#pragma unroll
+                            for (int b = 0; b < L::kBlocks; ++b)
+                                tmem_cp_32x128b_warpx4(sfa + (i * L::kBlocks + b) * 4,
+                                                       umma_smem_desc_noswz(sf + (1 + b) * kNvSfBytes + i * 512, 16, 128));
+                        }
+                    }
+                    const uint64_t w_desc = umma_smem_desc_sw128(w_addr), a_desc = umma_smem_desc_sw128(a_addr);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t acc = (u > 0 || i > 0) ? 1u : 0u;
+                        if constexpr (kMx) {
+                            // weights e4m3 (format 0) or e2m1 (5) x e4m3, ue8m0 scales (1)
+                            const uint32_t idesc = umma_idesc_block_scaled(kTileN, p.a_rows, KIND == Kind::kMx8W4 ? 5 : 0, 0, 1,
+                                                                           KIND == Kind::kMx8W4 ? i : (k & 3), k & 3);
+                            umma_mxf8(d, w_desc + i * 2, a_desc + i * 2, idesc, sfw, sfa, acc);
+                        } else if constexpr (KIND == Kind::kNv4) {
+                            const uint32_t idesc = umma_idesc_block_scaled(kTileN, p.a_rows, 1, 1, 0, 0, 0);
+                            umma_nvf4(d, w_desc + i * 2, a_desc + i * 2, idesc, sfw + i * 4, sfa + i * L::kBlocks * 4, acc);
+                        } else {
+                            umma_f16(d, w_desc + i * 2, a_desc + i * 2, umma_idesc(kTileN, p.a_rows, 1, 1), acc);
+                        }
+                    }
+                    umma_commit(empty + s * 8);     // the stage's bytes are consumed once these retire
+                    if (kMx && (u + 1 == seg_len || (k & 3) == 3)) {
+                        umma_commit(img_empty + slot * 8);
+                        ++img;
+                    }
+                    nv_set ^= 1u;
+                    if (++s == S) s = 0, phase ^= 1u;
+                }
+                if (!alive) break;
+                umma_commit(full_tm + buf * 8);     // the segment is complete
+                n += seg_len;
+                kb += seg_len;
+                if (kb == p.kb) kb = 0;
+                ++seg;
+            }
+        }
+    } else if (warp < 4) {
+        // ------------------------------------------------------------ scale images, one per (tile, four K blocks)
+        if constexpr (kMx) {
+            constexpr int kQ = (M_PAD + 31) / 32;      // activation rows of a lane: lane, lane + 32, ..
+            const uint32_t me = warp - 2;
+            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb), n = 0;
+            auto advance = [&](int times) {
+                for (; times > 0; --times) {
+                    const int len = min(4 - (kb & 3), p.kb - kb);
+                    n += len, kb += len;
+                    if (kb == p.kb) kb = 0, ++tile;
+                }
+            };
+            struct Raw {
+                float4 a[kQ];
+                float4 w;               // FP8 weights: the four K blocks' scales
+                uint4 wsf[4];           // 4-bit weights: rows lane + 32 q, four words of four exponent bytes
+            };
+            auto load = [&](Raw& r) {
+                const int k0 = kb & ~3;
+                const int col = (tile / p.tiles_per_group) * p.kb + k0;
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) {
+                    const int row = q * 32 + static_cast<int>(lane);
+                    r.a[q] = make_float4(1.f, 1.f, 1.f, 1.f);      // rows beyond M: zeros times 2^0
+                    if (row < p.M) {
+                        const float* src = p.a_scales + static_cast<int64_t>(row) * p.scale_cols + col;
+                        if (p.vec_scales) {
+                            r.a[q] = __ldcg(reinterpret_cast<const float4*>(src));
+                        } else {
+                            r.a[q].x = __ldcg(src);
+                            if (k0 + 1 < p.kb) r.a[q].y = __ldcg(src + 1);
+                            if (k0 + 2 < p.kb) r.a[q].z = __ldcg(src + 2);
+                            if (k0 + 3 < p.kb) r.a[q].w = __ldcg(src + 3);
+                        }
+                    }
+                }
+                if constexpr (KIND == Kind::kMx8) {
+                    const float* src = p.w_scales + static_cast<int64_t>(tile) * p.kb + k0;
+                    r.w.x = __ldg(src);
+                    r.w.y = k0 + 1 < p.kb ? __ldg(src + 1) : 1.f;
+                    r.w.z = k0 + 2 < p.kb ? __ldg(src + 2) : 1.f;
+                    r.w.w = k0 + 3 < p.kb ? __ldg(src + 3) : 1.f;
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int row = tile * kTileN + q * 32 + static_cast<int>(lane);
+                        r.wsf[q] = make_uint4(0u, 0u, 0u, 0u);     // rows beyond N: zeros times 2^-127
+                        if (row < p.N) {
+                            const uint8_t* src = p.w_sf + static_cast<int64_t>(row) * p.sf_stride + k0 * 4;
+                            if (p.vec_scales) {
+                                r.wsf[q] = __ldg(reinterpret_cast<const uint4*>(src));
+                            } else {
+                                const uint32_t* words = reinterpret_cast<const uint32_t*>(src);
+                                r.wsf[q].x = __ldg(words);
+                                if (k0 + 1 < p.kb) r.wsf[q].y = __ldg(words + 1);
+                                if (k0 + 2 < p.kb) r.wsf[q].z = __ldg(words + 2);
+                                if (k0 + 3 < p.kb) r.wsf[q].w = __ldg(words + 3);
+                            }
+                        }
+                    }
+                }
+            };
+            auto pack = [&](float4 v) {
+                return exponent_byte(v.x, p.status) | exponent_byte(v.y, p.status) << 8 | exponent_byte(v.z, p.status) << 16 |
+                       exponent_byte(v.w, p.status) << 24;
+            };
+            // Two images are in registers and each is refilled as soon as it is written out, four images ahead of the
+            // one under way: a copy from one to the other would wait for the loads.
+            Raw raw[2];
+            uint32_t seq = me;                  // the image this warp writes next; (tile, kb, n) is the one it loads next
+            int n_write[2];
+            auto fill = [&](int h) {
+                n_write[h] = n;
+                if (n < count) load(raw[h]);
+                advance(2);
+            };
+            auto write = [&](const Raw& now) -> bool {
+                const uint32_t slot = seq & (kImgSlots - 1);
+                if (!mbar_wait_lane0(img_empty + slot * 8, ((seq / kImgSlots) & 1u) ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty))
+                    return false;
+                uint4* img = reinterpret_cast<uint4*>(base_ptr + L::img_off(S, p.a_rows) + slot * L::kImgBytes) + lane;
+                if constexpr (KIND == Kind::kMx8) {
+                    const uint32_t ew = pack(now.w);
+                    img[0] = make_uint4(ew, ew, ew, ew);
+                } else {
+                    img[0] = make_uint4(now.wsf[0].x, now.wsf[1].x, now.wsf[2].x, now.wsf[3].x);
+                    img[kImgBlock / 16] = make_uint4(now.wsf[0].y, now.wsf[1].y, now.wsf[2].y, now.wsf[3].y);
+                    img[2 * kImgBlock / 16] = make_uint4(now.wsf[0].z, now.wsf[1].z, now.wsf[2].z, now.wsf[3].z);
+                    img[3 * kImgBlock / 16] = make_uint4(now.wsf[0].w, now.wsf[1].w, now.wsf[2].w, now.wsf[3].w);
+                }
+#pragma unroll
+                for (int b = 0; b < L::kBlocks; ++b) {
+                    uint32_t word[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (b * 4 + q < kQ) word[q] = pack(now.a[b * 4 + q]);
+                    img[(L::kImgW + b * kImgBlock) / 16] = make_uint4(word[0], word[1], word[2], word[3]);
+                }
+                fence_proxy_async_smem();       // the images are read by tcgen05.cp
+                __syncwarp();
+                if (lane == 0) mbar_arrive(img_full + slot * 8);
+                seq += 2;
+                return true;
+            };
+            advance(me);
+            fill(0);
+            fill(1);
+            while (n_write[0] < count) {
+                if (!write(raw[0])) break;
+                fill(0);
+                if (n_write[1] >= count || !write(raw[1])) break;
+                fill(1);
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue
+        constexpr int kEpi = 32 * L::kEpiWarps, kCols = L::kCols;
+        auto epi_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpi) : "memory"); };
+        const int et = static_cast<int>(threadIdx.x) - 128;
+        const int row = et & 127, col0 = (et >> 7) * kCols;      // weight row inside the tile, first column
+        const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+        bool alive = true;
+        int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+        uint32_t seg = 0;
+        const int64_t slot_floats = static_cast<int64_t>(M_PAD) * kTileN;
+        int grp = 0, seen_grp = -1;
+        float scale = p.out_scale;
+        uint32_t stored = 0xffffffffu;       // grouped rows without a token are padding: nobody reads them
+        for (int n = 0; n < count;) {
+            // the segment [kb, kb_end) of `tile`
+            const int seg_len = min(p.kb - kb, count - n);
+            const bool from_zero = (kb == 0), to_end = (kb + seg_len == p.kb);
+            const uint32_t buf = kBuffers == 2 ? (seg & 1u) : 0u;
+            if constexpr (KIND == Kind::kNv4 && M_PAD == 16) {
+                // a group's scale and row mask, once per group and before the wait: read per tile behind it, the two
+                // dependent loads made the epilogue longer than a tile of eight units (w2 of the routed experts 266 -> 288 us)
+                if (grouped) grp = tile / p.n_tiles;
+                if (grouped && grp != seen_grp) {
+                    seen_grp = grp;
+                    scale = p.out_scale * __ldg(p.expert_scale + __ldcg(p.group_expert + grp));
+                    if (p.row_token) {
+                        const int tok = lane < M_PAD ? __ldcg(p.row_token + grp * M_PAD + lane) : -1;
+                        stored = __ballot_sync(0xffffffffu, tok >= 0);
+                    }
+                }
+            }
+            if (alive) alive = mbar_wait_warp_fast(full_tm + buf * 8, (seg / kBuffers) & 1u, abort_flag, p.status, kDevTimeoutGemmTmemFull);
+            float acc[kCols];
+            if (alive) {
+                tc_fence_after();
+                const uint32_t t0 = tmem_base + lane_base + buf * M_PAD + col0;
+                uint32_t(&raw)[kCols] = reinterpret_cast<uint32_t(&)[kCols]>(acc);
+#pragma unroll
+                for (int c = 0; c < kCols; c += 16) tmem_ld_32x16(t0 + c, reinterpret_cast<uint32_t(&)[16]>(raw[c]));
+                tmem_ld_wait();
+                tc_fence_before();
+            } else {
+#pragma unroll
+                for (int i = 0; i < kCols; ++i) acc[i] = 0.f;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(empty_tm + buf * 8);
+
+            const int nrow0 = (tile - grp * p.n_tiles) * kTileN;
+            if (!(from_zero && to_end) && (p.split > 0 || !from_zero)) {   // partial sums to this CTA's slot
+                float4* slot = reinterpret_cast<float4*>(p.scratch + static_cast<int64_t>(blockIdx.x) * slot_floats) + row;
+                if (alive) {
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 4)
+                        if (col0 + c < p.M) __stcg(slot + (col0 + c) / 4 * kTileN, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
+                }
+                __threadfence();
+                epi_sync();
+            }
+            if (p.split > 0) {
+                // every CTA of the tile adds one slice of it over all partials, in K order
+                int32_t* counter = p.flags + tile;
+                if (et == 0 && alive) {
+                    add_acq_rel_gpu(counter, 1);
+                    await_word(counter, [&](int v) { return (v & 0xffff) == p.split; }, abort_flag, p.status);
+                }
+                epi_sync();
+                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                if (alive) {
+                    // a thread adds four activation rows of a weight row, eight partials in flight
+                    const int j = static_cast<int>(blockIdx.x) - tile * p.split, quads = (p.M + 3) / 4 * kTileN;
+                    const float4* part = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(tile) * p.split * slot_floats);
+                    const int end = quads * (j + 1) / p.split;
+                    for (int e = quads * j / p.split + et; e < end; e += kEpi) {
+                        float4 v = __ldcg(part + e);
+                        for (int q0 = 1; q0 < p.split; q0 += 8) {
+                            float4 x[8];
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) x[q] = __ldcg(part + min(q0 + q, p.split - 1) * (slot_floats / 4) + e);
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                if (q0 + q < p.split) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
+                        }
+                        const float out[4] = {v.x, v.y, v.z, v.w};
+                        const int m = e / kTileN * 4, nr = nrow0 + e % kTileN;
+                        if (nr < p.N) {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                if (m + i < p.M) {
+                                    const int64_t at = static_cast<int64_t>(m + i) * p.N + nr;
+                                    const float o = KIND == Kind::kNv4 ? out[i] * p.out_scale : out[i];
+                                    if (KIND == Kind::kBf16 && p.c_is_fp32) static_cast<float*>(p.c)[at] = o;
+                                    else static_cast<__nv_bfloat16*>(p.c)[at] = __float2bfloat16_rn(o);
+                                }
+                        }
+                    }
+                }
+                epi_sync();
+                // the last to leave puts the counter back to zero
+                if (et == 0 && alive && (add_acq_rel_gpu(counter, 0x10000) >> 16) == p.split - 1) st_release_gpu(counter, 0);
+            } else if (!from_zero) {
+                if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
+            } else {
+                if (!to_end) {
+                    const long long t_end = static_cast<long long>(tile + 1) * p.kb - 1;
+                    const int last = cta_of(units, t_end, grid);
+                    // every contributor's flag is awaited by a thread of its own, then the partials are added in CTA order
+                    for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
+                        await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
+                    epi_sync();
+                    alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                    if (alive) {
+                        for (int c = blockIdx.x + 1; c <= last; ++c) {
+                            const float4* peer = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * slot_floats) + row;
+                            // (pieces of 32 columns, eight 16-byte loads in flight each: a condition per load would wait for
+                            // every one by itself; the slot of a CTA has room for M_PAD columns)
+                            constexpr int kPiece = kCols < 32 ? kCols : 32;
+#pragma unroll
+                            for (int c0 = 0; c0 < kCols; c0 += kPiece)
+                                if (col0 + c0 < p.M) {
+                                    float4 v[kPiece / 4];
+#pragma unroll
+                                    for (int i = 0; i < kPiece / 4; ++i) v[i] = __ldcg(peer + ((col0 + c0) / 4 + i) * kTileN);
+#pragma unroll
+                                    for (int i = 0; i < kPiece / 4; ++i) {
+                                        acc[c0 + 4 * i] += v[i].x, acc[c0 + 4 * i + 1] += v[i].y;
+                                        acc[c0 + 4 * i + 2] += v[i].z, acc[c0 + 4 * i + 3] += v[i].w;
+                                    }
+                                }
+                        }
+                    }
+                    epi_sync();
+                    if (alive)
+                        for (int c = blockIdx.x + 1 + et; c <= last; c += kEpi) p.flags[c] = 0;
+                }
+                const int nrow = nrow0 + row;
+                // Rows of C that take 8-byte stores: the four lanes that hold four neighbouring weight rows exchange their
+                // values so that each stores one activation row's four - a quarter of the store instructions.
+                const bool wide = M_PAD > 16 && !(KIND == Kind::kBf16 && p.c_is_fp32) && (p.N & 3) == 0 &&
+                                  (reinterpret_cast<uintptr_t>(p.c) & 7u) == 0;
+                if (wide) {
+                    if (alive) {
+                        __nv_bfloat16* c = static_cast<__nv_bfloat16*>(p.c) + nrow0 + (row & ~3);
+                        const bool in_n = nrow < p.N;    // (N is a multiple of four: the four lanes agree)
+#pragma unroll
+                        for (int i = 0; i < kCols; i += 4)
+                            if (col0 + i < p.M) {
+                                uint32_t rows01, rows23;
+                                transpose4(to_bf16x2<KIND>(acc[i], acc[i + 1], p.out_scale), to_bf16x2<KIND>(acc[i + 2], acc[i + 3], p.out_scale),
+                                           lane, rows01, rows23);
+                                const int m = col0 + i + static_cast<int>(lane & 3);
+                                if (m < p.M && in_n) *reinterpret_cast<uint2*>(c + static_cast<int64_t>(m) * p.N) = make_uint2(rows01, rows23);
+                            }
+                    }
+                } else if (alive && nrow < p.N) {
+                    const int64_t c_off = static_cast<int64_t>(grp) * M_PAD * p.N;
+#pragma unroll
+                    for (int i = 0; i < kCols; ++i)
+                        if (col0 + i < p.M && (M_PAD > 16 || ((stored >> i) & 1u))) {
+                            const int64_t at = c_off + static_cast<int64_t>(col0 + i) * p.N + nrow;
+                            const float v = KIND == Kind::kNv4 ? acc[i] * scale : acc[i];
+                            if (KIND == Kind::kBf16 && p.c_is_fp32) static_cast<float*>(p.c)[at] = v;
+                            else static_cast<__nv_bfloat16*>(p.c)[at] = __float2bfloat16_rn(v);
+                        }
+                }
+            }
+            n += seg_len;
+            kb += seg_len;
+            if (kb == p.kb) kb = 0, ++tile;
+            ++seg;
+        }
+    }
+
+    __syncthreads();
+    if (*abort_flag) abort_drain_sleep();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, L::kTmemCols);
+    }
+}
+
+// CTAs per weight tile: as many as the SMs hold when that is at least three (one CTA adding up to six whole partials at
+// the end costs more than the SMs that the division leaves idle), none (stream-K) otherwise.
+inline int tile_split(int n_tiles, int kb, int sms) {
+    int split = sms / n_tiles;
+    if (split > kb) split = kb;
+    if (split > kMaxTileSplit) split = kMaxTileSplit;
+    return split >= 3 ? split : 0;
+}
+
+template <Kind KIND, int M_PAD>
+int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap& wsf_map, const CUtensorMap& asf_map, Params& p,
+           const DeviceInfo& dev, cudaStream_t stream) {
+    using L = Layout<KIND, M_PAD>;
+    int stages = p.group_expert ? kGroupedStages : kMaxStages;
+    while (stages > 2 && L::total(stages, p.a_rows) > dev.smem_optin) --stages;
+    if (L::total(stages, p.a_rows) > dev.smem_optin)
+        return fail(WUDA_ERR_UNSUPPORTED, "device offers %d bytes of shared memory per block; the kernel needs more", dev.smem_optin);
+    p.stages = stages;
+    auto kernel = gemm_tc_kernel<KIND, M_PAD>;
+    WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(stages, p.a_rows)));
+    const int sms = gemm_sms(dev);
+    const long long units = static_cast<long long>(p.n_tiles) * p.kb;
+    // (grouped: the number of groups is only known on the device; one CTA per SM, idle ones return at once)
+    p.split = p.group_expert ? 0 : tile_split(p.n_tiles, p.kb, sms);
+    int grid = sms;
+    if (p.split > 0) grid = p.n_tiles * p.split;
+    else if (!p.group_expert && units < sms) grid = static_cast<int>(units);
+    WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(L::kThreads), L::total(stages, p.a_rows), stream, w_map, a_map, wsf_map, asf_map, p));
+    return WUDA_OK;
+}
+
+// The kernel for m activation rows.
+template <Kind KIND>
+int launch_for(int m, const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap& wsf_map, const CUtensorMap& asf_map,
+               Params& p, const DeviceInfo& dev, cudaStream_t stream) {
+    if (m <= 16) return launch<KIND, 16>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
+    if (m <= 32) return launch<KIND, 32>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
+    if (m <= 64) return launch<KIND, 64>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
+    if constexpr (KIND != Kind::kBf16)      // (BF16 takes at most 128 rows)
+        if (m > 128) return launch<KIND, 256>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
+    return launch<KIND, 128>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
+}
+
+// Bytes of scratch a call with m rows wants: the flags and a partial-tile slot per CTA.
+inline int64_t scratch_bytes(int m) {
+    int m_pad = 16;
+    while (m_pad < m) m_pad *= 2;
+    return kFlagBytes + static_cast<int64_t>(kMaxGrid) * m_pad * kTileN * 4;
+}
+inline int rows_of(int m) { return (m + 15) / 16 * 16; }
+
+}  // namespace gemmtc
+}  // namespace wuda
