@@ -12,8 +12,8 @@
 // activations from L2 with every weight tile is cheap and nothing is kept resident or shared between CTAs.
 //
 //   * swap-AB: weight rows are the MMA's M = 128, activation rows (rounded up to 16, not to a power of two) its N.
-//   * one elected thread fetches (as many stages as fit, 4 to 12), one issues the MMAs into one accumulator, which is
-//     double-buffered up to 128 rows; all rows up to 256 go in ONE pass over the weights.
+//   * one elected thread fetches (as many stages as fit, 4 to 12), one issues the MMAs into an accumulator that is
+//     double-buffered where tensor memory has the room; all rows up to 256 go in ONE pass over the weights.
 //   * block scales of the FP8 / 4-bit kinds are exponent bytes in tensor memory.  A 32-bit scale column holds four
 //     consecutive K blocks (the MMA's scale id picks one), so two warps build ONE image per four units, from scales
 //     they requested sixteen units earlier; the fetching and the issuing thread never wait for scale arithmetic.
@@ -85,14 +85,18 @@ template <Kind KIND, int M_PAD>
 struct Layout {
     static constexpr bool kMx = KIND == Kind::kMx8 || KIND == Kind::kMx8W4;
     static constexpr int kBlocks = (M_PAD + 127) / 128;               // 128-row blocks of activation scales
-    static constexpr int kBuffers = M_PAD <= 128 ? 2 : 1;
+    // FP8 x FP8 up to 128 rows keeps two sums, of the even and of the odd units of a range, added at the end.  The order of
+    // the additions is part of the layer's results: another order moves single bf16 roundings of the projections, and the
+    // 4-bit activations of the experts behind them turn those into 1e-2 of the layer's output.
+    static constexpr int kAccs = KIND == Kind::kMx8 && M_PAD <= 128 ? 2 : 1;
+    static constexpr int kBuffers = kAccs * M_PAD <= 128 ? 2 : 1;
     static constexpr int kEpiWarps = M_PAD >= 128 ? 8 : 4;
     static constexpr int kThreads = 32 * (4 + kEpiWarps);
     static constexpr int kCols = M_PAD / (kEpiWarps / 4);             // accumulator columns per epilogue thread
     // scale columns of one set (two sets alternate)
     static constexpr int kSfwCols = kMx ? 4 : (KIND == Kind::kNv4 ? 16 : 0);
     static constexpr int kSfaCols = kSfwCols * kBlocks;
-    static constexpr int kAccCols = kBuffers * M_PAD;
+    static constexpr int kAccCols = kBuffers * kAccs * M_PAD;
     static constexpr int kUsedCols = kAccCols + 2 * (kSfwCols + kSfaCols);
     static constexpr int kTmemCols = kUsedCols <= 32 ? 32 : (kUsedCols <= 64 ? 64 : (kUsedCols <= 128 ? 128 : (kUsedCols <= 256 ? 256 : 512)));
     static constexpr int kImgW = KIND == Kind::kMx8W4 ? 4 * kImgBlock : kImgBlock;    // weight part of an image slot
@@ -336,7 +340,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     if (!mbar_wait(empty_tm + buf * 8, (seg / kBuffers - 1u) & 1u, abort_flag, p.status, kDevTimeoutGemmTmemEmpty)) break;
                     tc_fence_after();
                 }
-                const uint32_t d = tmem_base + buf * M_PAD;
+                const uint32_t d_buf = tmem_base + buf * (L::kAccs * M_PAD);
                 for (int u = 0; u < seg_len; ++u) {
                     const int k = kb + u;
                     const uint32_t slot = img & (kImgSlots - 1);
@@ -375,10 +379,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                                                        umma_smem_desc_noswz(sf + (1 + b) * kNvSfBytes + i * 512, 16, 128));
                         }
                     }
+                    const uint32_t d = d_buf + (L::kAccs == 2 ? ((n + u) & 1) * M_PAD : 0);
                     const uint64_t w_desc = umma_smem_desc_sw128(w_addr), a_desc = umma_smem_desc_sw128(a_addr);
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
-                        const uint32_t acc = (u > 0 || i > 0) ? 1u : 0u;
+                        const uint32_t acc = (u >= L::kAccs || i > 0) ? 1u : 0u;
                         if constexpr (kMx) {
                             // weights e4m3 (format 0) or e2m1 (5) x e4m3, ue8m0 scales (1)
                             const uint32_t idesc = umma_idesc_block_scaled(kTileN, p.a_rows, KIND == Kind::kMx8W4 ? 5 : 0, 0, 1,
@@ -558,11 +563,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             float acc[kCols];
             if (alive) {
                 tc_fence_after();
-                const uint32_t t0 = tmem_base + lane_base + buf * M_PAD + col0;
+                const uint32_t t0 = tmem_base + lane_base + buf * (L::kAccs * M_PAD) + col0;
                 uint32_t(&raw)[kCols] = reinterpret_cast<uint32_t(&)[kCols]>(acc);
+                if constexpr (L::kAccs == 2) {
+                    const uint32_t first = (n & 1) * M_PAD;      // a segment of one unit has only this sum
 #pragma unroll
-                for (int c = 0; c < kCols; c += 16) tmem_ld_32x16(t0 + c, reinterpret_cast<uint32_t(&)[16]>(raw[c]));
-                tmem_ld_wait();
+                    for (int c = 0; c < kCols; c += 16) {
+                        uint32_t v0[16], v1[16];
+                        tmem_ld_32x16(t0 + first + c, v0);
+                        if (seg_len >= 2) tmem_ld_32x16(t0 + (M_PAD - first) + c, v1);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) acc[c + i] = __uint_as_float(v0[i]) + (seg_len >= 2 ? __uint_as_float(v1[i]) : 0.f);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < kCols; c += 16) tmem_ld_32x16(t0 + c, reinterpret_cast<uint32_t(&)[16]>(raw[c]));
+                    tmem_ld_wait();
+                }
                 tc_fence_before();
             } else {
 #pragma unroll
