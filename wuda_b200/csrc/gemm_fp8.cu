@@ -11,24 +11,23 @@
 // block-scale path, so the promotion happens in registers.
 //
 // Design: decode GEMMs are bound by the weight stream (N*K bytes once from HBM), so
-//  * swap-AB: the UMMA M dimension (128) is a tile of weight rows, the UMMA N dimension
-//    is the padded activation count (16..256); the activations (a few MB at most) are
-//    re-read from L2 for every weight tile;
-//  * stream-K: the flat list of (weight tile, K block) units is cut into one equal
-//    contiguous range per SM, so every SM streams the same number of bytes whatever N is;
-//    a range that does not start a tile's K range writes its fp32 partial to the CTA's own
-//    scratch slot in global memory and raises a flag; the CTA holding the start of the
-//    range adds the partials in CTA order (deterministic) and writes the bf16 tile;
-//  * per unit: an elected thread fetches the weight tile (128 x 128 B) and the
-//    activation tile (M_PAD x 128 B), four tcgen05.mma kind::f8f6f4 fill a fresh TMEM
-//    stage, and an epilogue warpgroup adds the stage, times the unit's scales, to its register
-//    accumulators.  One unit's epilogue is a chain of waits (scales, TMEM stage, tcgen05.ld), so
-//    the two epilogue warpgroups take units alternately and their chains overlap; the two
-//    accumulator sets are added when a tile's segment ends.  (Above 64 activation rows a thread
-//    cannot hold all columns; the groups then split the columns and both take every unit.);
-//  * roles are replicated (2 producers, 2 issuers) and take units round-robin; stage
-//    counts are multiples of the role counts; every wait is bounded and reports through
-//    the status word.
+//  * swap-AB: the UMMA M dimension (128) is a tile of weight rows, the UMMA N dimension is the activation count rounded
+//    up to 16; the activations (a few MB at most) are re-read from L2 for every weight tile (gemm_tc.cuh says why that
+//    is cheap);
+//  * the work split is gemm_tc.cuh's: stream-K, or for few weight tiles the same number of CTAs per tile;
+//  * per unit: an elected thread fetches the weight tile (128 x 128 B) and the activation tile, another issues four
+//    tcgen05.mma kind::f8f6f4 into a fresh TMEM stage, and an epilogue warpgroup adds the stage, times the unit's scales,
+//    to its register accumulators.  The scales of a stage, already multiplied (a_s * w_s), are written beside it by a
+//    warp that requested them four K blocks at a time, eight units earlier, and arrives on the stage's barrier: an
+//    epilogue thread waits once per unit.  The two epilogue warpgroups take units alternately and their chains overlap; the
+//    two accumulator sets are added when a tile's segment ends.  (Above 64 activation rows a thread cannot hold all
+//    columns; the groups then split the columns and both take every unit.)
+// Measured (CUDA-graph replays, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
+// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 37.1,
+// 43.9 -> 38.4, 62.7 -> 46.8, 122.5 -> 91.1 (two passes); 7168 x 16384 at 64 rows 32.5 -> 29.5; 2112 x 7168 at 1 / 64 rows
+// 12.3 -> 10.3, 15.3 -> 12.3.  Where the split is stream-K (more than a third of the SMs hold tiles) the results are
+// bit-identical to those of the earlier form: the order of the additions is the same.
+// Every wait is bounded and reports through the status word.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -36,36 +35,43 @@
 #include <cstring>
 #include <mutex>
 
+#include "gemm_tc.cuh"
 #include "host.h"
 #include "ptx.cuh"
 
 namespace wuda {
 namespace gemm8 {
 
-constexpr int kTileN = 128;          // weight rows per tile (UMMA M)
-constexpr int kBlockK = 128;         // K per unit
-constexpr int kProducers = 2;        // warps 0, 1
-constexpr int kIssuers = 2;          // warps 2, 3
-constexpr int kFirstEpiWarp = 4;     // warps 4..11: two warpgroups, half the columns each
+using gemmtc::add_acq_rel_gpu;
+using gemmtc::await_word;
+using gemmtc::cta_of;
+using gemmtc::kRowBytes;
+using gemmtc::kTileN;
+using gemmtc::kWBytes;
+using gemmtc::ld_acquire_gpu;
+using gemmtc::range_begin;
+using gemmtc::st_release_gpu;
+
+constexpr int kFirstEpiWarp = 4;     // warp 0 copies, 1 issues MMAs, 2 prepares scales, 3 is idle, 4..11 are two epilogue warpgroups
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 32 * (kFirstEpiWarp + kEpiWarps);
-constexpr int kWBytes = kTileN * kBlockK;   // 16 KB
-constexpr int kScaleSlots = 8;       // scale ring depth
-constexpr int kScaleAhead = 6;       // units of look-ahead of the scale fetch (< kScaleSlots - 1)
+constexpr int kMaxStages = 12;
 
 struct Params {
-    const float* a_scales;     // [M, K/128]
+    const float* a_scales;     // [M, a_kb_total]
     const float* w_scales;     // [ceil(N/128), K/128]
     __nv_bfloat16* c;          // [M, N]
-    float* scratch;            // [grid][M_PAD][128] fp32: one partial-tile slot per CTA
-    int32_t* flags;            // [grid]: slot c is published; zero between calls
+    float* scratch;            // [grid] partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]
+    int32_t* flags;            // stream-K: one flag per CTA; split: one counter per weight tile; zero between calls
     int32_t* status;
     int M, N, K, kb;           // kb = K / 128
     int n_tiles;
+    int a_rows;                // M rounded up to 16
     int stages;
-    int a_resident = 0;        // the whole activation matrix stays in shared memory (see Smem)
+    int split;                 // CTAs per weight tile, 0 = stream-K
+    int vec_scales;            // rows of a_scales can be read 16 bytes at a time
     // grouped form: weight tile t belongs to group t / group_tiles and reads the activations'
-    // columns [group * K, (group + 1) * K); a_kb_total = K blocks in an activation row (0: kb)
+    // columns [group * K, (group + 1) * K); a_kb_total = K blocks in an activation row
     int group_tiles = 0;
     int a_kb_total = 0;
     // two-rank tensor parallelism (K split across two GPUs): peer exchange of fp32 tiles
@@ -80,66 +86,24 @@ struct Params {
 
 template <int M_PAD>
 struct Smem {
-    static constexpr int kABytes = M_PAD * kBlockK;
-    static constexpr int kStageBytes = kWBytes + kABytes;
-    static constexpr int kTmemStages = M_PAD <= 128 ? 4 : 2;
-    static constexpr int kTmemCols = kTmemStages * M_PAD < 32 ? 32 : kTmemStages * M_PAD;
-    // Two layouts.  Streaming: every stage holds a weight tile and the matching activation tile.
-    // Resident: when the padded activation matrix (kb tiles of kABytes) fits beside at least six
-    // weight stages it is loaded once per CTA and the stages hold weight tiles only - a CTA then
-    // ingests 16 KB per unit instead of 16 KB + kABytes, which is what bounds decode shapes with
-    // many rows and a short K.
-    static __host__ __device__ constexpr int stage_bytes(bool resident) { return resident ? kWBytes : kStageBytes; }
-    static __host__ __device__ constexpr int scale_off(int stages, int resident_kb = 0) {
-        return stages * stage_bytes(resident_kb > 0) + resident_kb * kABytes;
-    }
+    static constexpr int kTmemStages = M_PAD <= 64 ? 8 : 4;
+    static constexpr int kTmemCols = kTmemStages * M_PAD;
     // Up to M_PAD = 64 the two epilogue warpgroups take units alternately (all columns each) and add
     // their accumulators through a [M_PAD][128] fp32 buffer when a tile's segment ends; above that a
     // thread cannot hold M_PAD accumulators and the groups split the columns instead.
     static constexpr bool kAlternate = M_PAD <= 64;
     static constexpr int kCombineBytes = kAlternate ? M_PAD * kTileN * 4 : 0;
-    // scale rings, one set per epilogue group: kScaleSlots x (M_PAD activation scales) + kScaleSlots
-    // weight scales
-    static constexpr int kRingFloats = kScaleSlots * M_PAD + kScaleSlots;
-    static __host__ __device__ constexpr int comb_off(int stages, int resident_kb = 0) {
-        return scale_off(stages, resident_kb) + 2 * kRingFloats * 4;
-    }
-    static __host__ __device__ constexpr int bar_off(int stages, int resident_kb = 0) {
-        return comb_off(stages, resident_kb) + kCombineBytes;
-    }
-    // barriers: full[16] empty[16] full_tm[4] empty_tm[4] a_full[1]
-    static __host__ __device__ constexpr int misc_off(int stages, int resident_kb = 0) {
-        return bar_off(stages, resident_kb) + 48 * 8;
-    }
-    static __host__ __device__ constexpr int total(int stages, int resident_kb = 0) {
-        return misc_off(stages, resident_kb) + 32 + 1024;
-    }
-};
-
-struct Ring {
-    int idx = 0;
-    uint32_t phase = 0;
-    __device__ __forceinline__ void step(int n, int size) {   // n <= size
-        idx += n;
-        if (idx >= size) {
-            idx -= size;
-            phase ^= 1u;
-        }
-    }
+    static __host__ __device__ constexpr int stage_bytes(int a_rows) { return kWBytes + a_rows * kRowBytes; }
+    // one row of scale products per TMEM stage
+    static __host__ __device__ constexpr int scale_off(int stages, int a_rows) { return stages * stage_bytes(a_rows); }
+    static __host__ __device__ constexpr int comb_off(int stages, int a_rows) { return scale_off(stages, a_rows) + kTmemStages * M_PAD * 4; }
+    static __host__ __device__ constexpr int bar_off(int stages, int a_rows) { return comb_off(stages, a_rows) + kCombineBytes; }
+    // barriers: full[12] empty[12] full_tm[8] empty_tm[8]
+    static __host__ __device__ constexpr int misc_off(int stages, int a_rows) { return bar_off(stages, a_rows) + (2 * kMaxStages + 16) * 8; }
+    static __host__ __device__ constexpr int total(int stages, int a_rows) { return misc_off(stages, a_rows) + 32 + 1024; }
 };
 
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
-__device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void st_release_gpu(int32_t* p, int v) {
-    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 __device__ __forceinline__ void st_release_sys(int32_t* p, int v) {
     asm volatile("st.release.sys.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -153,21 +117,6 @@ __device__ __forceinline__ float ld_volatile_f32(const float* p) {   // written 
     asm volatile("ld.volatile.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ int ld_acquire_gpu(const int32_t* p) {
-    int v;
-    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Range boundary of CTA c in the flat unit list.
-__device__ __forceinline__ long long range_begin(long long units, int c, int grid) { return units * c / grid; }
-// The CTA whose range holds unit u.
-__device__ __forceinline__ int cta_of(long long units, long long u, int grid) {
-    int c = static_cast<int>(u * grid / units);
-    while (c + 1 < grid && range_begin(units, c + 1, grid) <= u) ++c;
-    while (c > 0 && range_begin(units, c, grid) > u) --c;
-    return c;
-}
 
 template <int M_PAD>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -175,27 +124,22 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 const Params p) {
     using L = Smem<M_PAD>;
     constexpr int kTS = L::kTmemStages;
-    constexpr int kHalf = M_PAD / 2;                 // columns per epilogue warpgroup
+    constexpr int kHalf = M_PAD / 2;                 // columns a warpgroup finishes
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base = (raw_addr + 1023u) & ~1023u;
     uint8_t* base_ptr = smem_raw + (base - raw_addr);
     const int S = p.stages;
-    const bool resident = p.a_resident != 0;
-    const int rkb = resident ? p.kb : 0;
-    const int stage_bytes = L::stage_bytes(resident);
-    const uint32_t a_res = base + S * stage_bytes;      // resident activations: kb tiles of kABytes
-    const uint32_t bars = base + L::bar_off(S, rkb);
-    const uint32_t full = bars, empty = bars + 16 * 8, full_tm = bars + 32 * 8, empty_tm = bars + 36 * 8;
-    const uint32_t a_full = bars + 40 * 8;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, rkb));
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, rkb) + 4);
-    float* rings = reinterpret_cast<float*>(base_ptr + L::scale_off(S, rkb));
-    float* comb = reinterpret_cast<float*>(base_ptr + L::comb_off(S, rkb));
+    const uint32_t stage_bytes = L::stage_bytes(p.a_rows);
+    const uint32_t bars = base + L::bar_off(S, p.a_rows);
+    const uint32_t full = bars, empty = full + kMaxStages * 8, full_tm = empty + kMaxStages * 8, empty_tm = full_tm + 8 * 8;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, p.a_rows));
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 4);
+    float* products = reinterpret_cast<float*>(base_ptr + L::scale_off(S, p.a_rows));     // [kTS][M_PAD]: a_s * w_s
+    float* comb = reinterpret_cast<float*>(base_ptr + L::comb_off(S, p.a_rows));
     constexpr bool kAlt = L::kAlternate;
-    constexpr bool kPreScale = M_PAD >= 64;   // multiply activation and weight scales once per column, not per thread
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
     const uint32_t lane = lane_id();
 
     if (threadIdx.x == 0) {
@@ -205,25 +149,42 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             mbar_init(empty + i * 8, 1);          // released by the UMMA commit
         }
         for (int i = 0; i < kTS; ++i) {
-            mbar_init(full_tm + i * 8, 1);
+            mbar_init(full_tm + i * 8, 2);        // the MMAs have retired and the scale products are written
             mbar_init(empty_tm + i * 8, kAlt ? kEpiWarps / 2 : kEpiWarps);   // the warps that read a stage
         }
-        mbar_init(a_full, kProducers);
         fence_mbar_init();
     }
-    if (warp == kProducers) {   // first issuer warp owns the TMEM allocation
+    if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), L::kTmemCols);
         tmem_relinquish();
     }
-    if (warp == 0 && lane == 0) {
+    const long long units = static_cast<long long>(p.n_tiles) * p.kb;
+    long long u0;
+    int count;
+    if (p.split > 0) {
+        const int tile = static_cast<int>(blockIdx.x) / p.split, j = static_cast<int>(blockIdx.x) - tile * p.split;
+        const int k0 = p.kb * j / p.split;
+        u0 = static_cast<long long>(tile) * p.kb + k0;
+        count = p.kb * (j + 1) / p.split - k0;
+    } else {
+        u0 = range_begin(units, blockIdx.x, gridDim.x);
+        count = static_cast<int>(range_begin(units, blockIdx.x + 1, gridDim.x) - u0);
+    }
+    const int tile0 = static_cast<int>(u0 / p.kb), kb0 = static_cast<int>(u0 % p.kb);
+    if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
+        int tile = tile0, kb = kb0;
+        for (int n = 0; n < count && n < S; ++n) {
+            tma_prefetch_2d(&w_map, kb * kRowBytes, tile * kTileN);
+            if (++kb == p.kb) kb = 0, ++tile;
+        }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // the prologue above ran while the kernel ahead was still finishing; global memory from here on
+    // all of the above ran while the kernel ahead was still finishing; its results are read from here on
     pdl_launch_dependents();
     pdl_wait();
 
@@ -231,207 +192,173 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     // finished call's (the word is rewritten only after every CTA of this call has read it)
     const int tp_epoch = (p.tp_peer_inbox && p.tp_epoch == 0) ? ld_acquire_gpu(p.tp_ctrl) + 1 : p.tp_epoch;
 
-    const long long units = static_cast<long long>(p.n_tiles) * p.kb;
-    const long long u0 = range_begin(units, blockIdx.x, gridDim.x);
-    const long long u1 = range_begin(units, blockIdx.x + 1, gridDim.x);
-    const int count = static_cast<int>(u1 - u0);
-
-    if (warp < kProducers) {
-        // ------------------------------------------------------------ TMA producers
-        const int me = warp;
-        const uint64_t stream_policy = policy_evict_first();
-        const uint64_t keep_policy = policy_evict_last();
-        Ring ring;
-        ring.step(me, S);
-        int tile = static_cast<int>((u0 + me) / p.kb), kb = static_cast<int>((u0 + me) % p.kb);
-        bool alive = true;
-        if (resident && count > 0) {
-            // this producer's share of the activation tiles (K blocks me, me + kProducers, ..)
-            const int mine = me < p.kb ? (p.kb - me + kProducers - 1) / kProducers : 0;
-            if (elect_one()) {
-                if (mine > 0) mbar_arrive_expect_tx(a_full, static_cast<uint32_t>(mine) * L::kABytes);
-                else mbar_arrive(a_full);
-                for (int kbj = me; kbj < p.kb; kbj += kProducers)
-                    tma_load_2d_hint(a_res + kbj * L::kABytes, &a_map, a_full, kbj * kBlockK, 0, keep_policy);
-            }
-            __syncwarp();
-        }
-        for (int n = me; n < count && alive; n += kProducers) {
-            const int s = ring.idx;
-            alive = mbar_wait_lane0(empty + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmEmpty);
-            if (!alive) break;
-            const uint32_t stage = base + s * stage_bytes;
-            const int a_x = kb * kBlockK + (p.group_tiles ? (tile / p.group_tiles) * p.K : 0);
-            if (elect_one()) {
-                mbar_arrive_expect_tx(full + s * 8, stage_bytes);
-                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kBlockK, tile * kTileN, stream_policy);
-                if (!resident) tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, a_x, 0, keep_policy);
-            }
-            __syncwarp();
-            ring.step(kProducers, S);
-            kb += kProducers;
-            while (kb >= p.kb) {
-                kb -= p.kb;
-                ++tile;
-            }
-        }
-    } else if (warp < kProducers + kIssuers) {
-        // ------------------------------------------------------------ UMMA issuers (one thread each)
+    if (warp == 0) {
+        // ------------------------------------------------------------ copies
         if (elect_one()) {
-            const int me = warp - kProducers;
-            constexpr uint32_t idesc = umma_idesc(kTileN, M_PAD, 0, 0);
-            Ring ring, tring;
-            ring.step(me, S);
-            tring.step(me, kTS);
-            int kbi = static_cast<int>((u0 + me) % p.kb);   // K block of this issuer's next unit
-            bool a_ready = !resident || count <= me ||
-                           mbar_wait(a_full, 0u, abort_flag, p.status, kDevTimeoutGemmFull);
-            for (int n = me; n < count && a_ready; n += kIssuers) {
-                const int s = ring.idx, ts = tring.idx;
-                if (!mbar_wait(full + s * 8, ring.phase, abort_flag, p.status, kDevTimeoutGemmFull)) break;
-                if (!mbar_wait(empty_tm + ts * 8, tring.phase ^ 1u, abort_flag, p.status, kDevTimeoutGemmTmemEmpty)) break;
+            const uint64_t stream_policy = policy_evict_first();
+            const uint64_t keep_policy = policy_evict_last();
+            int s = 0, tile = tile0, kb = kb0;
+            uint32_t phase = 1;
+            for (int n = 0; n < count; ++n) {
+                const int a_x = kb * kRowBytes + (p.group_tiles ? (tile / p.group_tiles) * p.K : 0);
+                if (!mbar_wait(empty + s * 8, phase, abort_flag, p.status, kDevTimeoutGemmEmpty)) break;
+                const uint32_t stage = base + s * stage_bytes;
+                mbar_arrive_expect_tx(full + s * 8, stage_bytes);
+                tma_load_2d_hint(stage, &w_map, full + s * 8, kb * kRowBytes, tile * kTileN, stream_policy);
+                tma_load_2d_hint(stage + kWBytes, &a_map, full + s * 8, a_x, 0, keep_policy);
+                if (++s == S) s = 0, phase ^= 1u;
+                if (++kb == p.kb) kb = 0, ++tile;
+            }
+        }
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMAs
+        if (elect_one()) {
+            const uint32_t idesc = umma_idesc(kTileN, p.a_rows, 0, 0);
+            int s = 0;
+            uint32_t phase = 0;
+            for (int n = 0; n < count; ++n) {
+                const int ts = n % kTS;
+                if (!mbar_wait(empty_tm + ts * 8, ((n / kTS) & 1) ^ 1, abort_flag, p.status, kDevTimeoutGemmTmemEmpty)) break;
+                if (!mbar_wait(full + s * 8, phase, abort_flag, p.status, kDevTimeoutGemmFull)) break;
                 tc_fence_after();
                 const uint32_t w_addr = base + s * stage_bytes;
-                const uint32_t a_addr = resident ? a_res + kbi * L::kABytes : w_addr + kWBytes;
-                kbi += kIssuers;
-                while (kbi >= p.kb) kbi -= p.kb;
-                const uint32_t d_addr = tmem_base + ts * M_PAD;
+                const uint64_t w_desc = umma_smem_desc_sw128(w_addr), a_desc = umma_smem_desc_sw128(w_addr + kWBytes);
 #pragma unroll
-                for (int k = 0; k < kBlockK / 32; ++k)
-                    umma_f8f6f4(d_addr, umma_smem_desc_sw128(w_addr + k * 32), umma_smem_desc_sw128(a_addr + k * 32),
-                                idesc, k > 0 ? 1u : 0u);
+                for (int k = 0; k < 4; ++k)
+                    umma_f8f6f4(tmem_base + ts * M_PAD, w_desc + k * 2, a_desc + k * 2, idesc, k > 0 ? 1u : 0u);
                 umma_commit(full_tm + ts * 8);
                 umma_commit(empty + s * 8);      // the stage's bytes are consumed once the UMMAs retire
-                ring.step(kIssuers, S);
-                tring.step(kIssuers, kTS);
+                if (++s == S) s = 0, phase ^= 1u;
             }
         }
-    } else {
-        // ------------------------------------------------------------ epilogue warps
-        // Thread = one weight row (TMEM lane) x half of the activation columns.
-        const int ew = warp - kFirstEpiWarp;            // 0..7
-        const int grp = ew >> 2;                        // epilogue warpgroup
-        const int half = grp;                           // the half of the columns this group finishes
-        const int et = (ew * 32 + lane);                // 0..255 among epilogue threads
-        const int gt = et & 127;                        // 0..127 inside the group
-        const int row_in_tile = (warp & 3) * 32 + lane;
+    } else if (warp == 2) {
+        // ------------------------------------------------------------ scale products
+        // In groups of four K blocks of a tile (aligned to four, cut at the ends of the range).  A lane holds the scales of
+        // rows lane, lane + 32, ..; two groups are in registers, each refilled when it has been written out.  (One warp: it
+        // sees every phase of the barriers it waits on.)
+        constexpr int kQ = (M_PAD + 31) / 32;
+        int tile = tile0, kb = kb0, n = 0;
+        struct Raw {
+            float4 a[kQ], w;
+            int n, k, len;          // first unit, its K block modulo four, units
+        };
+        auto group_len = [&] { return min(min(4 - (kb & 3), p.kb - kb), count - n); };
+        auto fill = [&](Raw& r) {
+            r.n = n, r.k = kb & 3, r.len = group_len();
+            if (n < count) {
+                const int k0 = kb & ~3, col = k0 + (p.group_tiles ? (tile / p.group_tiles) * p.kb : 0);
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) {
+                    const int row = q * 32 + static_cast<int>(lane);
+                    r.a[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (row < p.M) {
+                        const float* src = p.a_scales + static_cast<int64_t>(row) * p.a_kb_total + col;
+                        if (p.vec_scales) {
+                            r.a[q] = __ldcg(reinterpret_cast<const float4*>(src));
+                        } else {
+                            r.a[q].x = __ldcg(src);
+                            if (k0 + 1 < p.kb) r.a[q].y = __ldcg(src + 1);
+                            if (k0 + 2 < p.kb) r.a[q].z = __ldcg(src + 2);
+                            if (k0 + 3 < p.kb) r.a[q].w = __ldcg(src + 3);
+                        }
+                    }
+                }
+                const float* src = p.w_scales + static_cast<int64_t>(tile) * p.kb + k0;
+                r.w.x = __ldg(src);
+                r.w.y = k0 + 1 < p.kb ? __ldg(src + 1) : 0.f;
+                r.w.z = k0 + 2 < p.kb ? __ldg(src + 2) : 0.f;
+                r.w.w = k0 + 3 < p.kb ? __ldg(src + 3) : 0.f;
+                const int len = group_len();
+                n += len, kb += len;
+                if (kb == p.kb) kb = 0, ++tile;
+            }
+        };
+        auto of = [](const float4& v, int i) { return i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)); };
+        auto write = [&](const Raw& r) -> bool {
+            for (int i = 0; i < r.len; ++i) {
+                const int u = r.n + i, ts = u % kTS;
+                const float w = of(r.w, r.k + i);
+                float v[kQ];
+#pragma unroll
+                for (int q = 0; q < kQ; ++q) v[q] = __fmul_rn(of(r.a[q], r.k + i), w);
+                if (!mbar_wait_warp_fast(empty_tm + ts * 8, ((u / kTS) & 1) ^ 1, abort_flag, p.status, kDevTimeoutGemmTmemEmpty))
+                    return false;
+#pragma unroll
+                for (int q = 0; q < kQ; ++q)
+                    if (q * 32 + static_cast<int>(lane) < M_PAD) products[ts * M_PAD + q * 32 + lane] = v[q];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_tm + ts * 8);
+            }
+            return true;
+        };
+        Raw a, b;
+        fill(a);
+        fill(b);
+        while (a.n < count) {
+            if (!write(a)) break;
+            fill(a);
+            if (b.n >= count || !write(b)) break;
+            fill(b);
+        }
+    } else if (warp >= kFirstEpiWarp) {
+        // ------------------------------------------------------------ epilogue
+        const int ew = warp - kFirstEpiWarp;
+        const int grp = ew >> 2, half = grp;
+        const int et = ew * 32 + static_cast<int>(lane);      // 0..255
+        const int row_in_tile = (warp & 3) * 32 + static_cast<int>(lane);
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         // kAlt: this group takes the units with (n & 1) == grp and accumulates every column;
         // otherwise both groups take every unit and half of the columns each.
         constexpr int kCols = kAlt ? M_PAD : kHalf;
         const int col0 = kAlt ? 0 : half * kHalf;
-        constexpr int kStep = kAlt ? 2 : 1;
-        const int first = kAlt ? grp : 0;               // this group's first unit
-        __align__(8) float acc[kCols];
+        __align__(16) float acc[kCols];
 #pragma unroll
         for (int i = 0; i < kCols; ++i) acc[i] = 0.f;
-        Ring tring;
-        tring.step(first, kTS);
         bool alive = true;
-        int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+        int tile = tile0, kb = kb0;
         int seg_kb0 = kb;                               // first K block of the running segment
-
-        // Scales of a unit (activation scales a_s[:, kb], weight scale w_s[tile, kb]) are fetched
-        // kScaleAhead of the group's units early with 4-byte asynchronous copies into the group's rings
-        // of kScaleSlots slots, so their L2 latency never sits between two units.
-        float* a_ring = rings + (kAlt ? grp * L::kRingFloats : 0);   // one ring per group, or one shared
-        float* w_ring = a_ring + kScaleSlots * M_PAD;
-        const int fetcher = kAlt ? gt : et;             // thread index among those that share the rings
-        const int fetchers = kAlt ? 128 : 256;
-        int ftile = static_cast<int>((u0 + first) / p.kb), fkb = static_cast<int>((u0 + first) % p.kb);
-        auto fetch_scales = [&](int j) {                // j-th unit of this group
-            if (first + j * kStep < count) {
-                const int slot = j & (kScaleSlots - 1);
-                const int a_stride = p.a_kb_total ? p.a_kb_total : p.kb;
-                const int a_col = fkb + (p.group_tiles ? (ftile / p.group_tiles) * p.kb : 0);
-                for (int r = fetcher; r < p.M; r += fetchers)
-                    cp_async4(smem_u32(a_ring + slot * M_PAD + r), p.a_scales + static_cast<int64_t>(r) * a_stride + a_col);
-                if (fetcher == fetchers - 1)
-                    cp_async4(smem_u32(w_ring + slot), p.w_scales + static_cast<int64_t>(ftile) * p.kb + fkb);
-                fkb += kStep;
-                while (fkb >= p.kb) {
-                    fkb -= p.kb;
-                    ++ftile;
-                }
-            }
-            cp_async_commit();                           // one group per unit, empty or not
-        };
-        for (int j = 0; j < kScaleAhead; ++j) fetch_scales(j);
-        auto ring_sync = [&]() {                         // the threads that share this group's rings
-            if constexpr (kAlt) {
-                if (grp == 0) asm volatile("bar.sync 2, 128;" ::: "memory");
-                else asm volatile("bar.sync 3, 128;" ::: "memory");
-            } else {
-                epi_bar_sync();
-            }
-        };
+        constexpr int64_t kSlotFloats = static_cast<int64_t>(M_PAD) * kTileN;
 
         // An aborting CTA keeps walking the loop (every wait then fails at once) so that all
         // 256 epilogue threads reach every named barrier; it only skips the arithmetic.
-        int j = 0;                                       // units this group has taken
         for (int n = 0; n < count; ++n) {
             if (!kAlt || (n & 1) == grp) {
-            fetch_scales(j + kScaleAhead);
-            cp_async_wait<kScaleAhead>();                // this thread's copies for the unit have landed
-            ring_sync();                                 // ... and so have everybody else's
-            if constexpr (kPreScale) {   // the unit's scale products a_s[c] * w_s, once per column
-                const int slot = j & (kScaleSlots - 1);
-                if (fetcher < M_PAD) a_ring[slot * M_PAD + fetcher] = __fmul_rn(a_ring[slot * M_PAD + fetcher], w_ring[slot]);
-                ring_sync();
-            }
-            const int ts = tring.idx;
-            if (alive)
-                alive = mbar_wait_warp_fast(full_tm + ts * 8, tring.phase, abort_flag, p.status, kDevTimeoutGemmTmemFull);
-            if (alive) {
-                tc_fence_after();
-                const int slot = j & (kScaleSlots - 1);
-                const float wsc = kPreScale ? 1.0f : w_ring[slot];   // wide tiles hold a_s[c] * w_s already
-                const float* sc = a_ring + slot * M_PAD + col0;
-                const uint32_t taddr = tmem_base + lane_base + ts * M_PAD + col0;
-                // acc[c] += v[c] * (a_s[c] * w_s): the products come as 16-byte shared-memory loads, the
-                // sums as packed fp32x2 operations (one instruction per two columns)
-                float2* acc2 = reinterpret_cast<float2*>(acc);
-                const float2 w2 = make_float2(wsc, wsc);
-                if constexpr (kCols >= 32) {
-                    uint32_t v[2][32];
-                    tmem_ld_32x32(taddr, v[0]);
+                const int ts = n % kTS;
+                if (alive)
+                    alive = mbar_wait_warp_fast(full_tm + ts * 8, (n / kTS) & 1, abort_flag, p.status, kDevTimeoutGemmTmemFull);
+                if (alive) {
+                    tc_fence_after();
+                    const float* sc = products + ts * M_PAD + col0;
+                    const uint32_t taddr = tmem_base + lane_base + ts * M_PAD + col0;
+                    // acc[c] += v[c] * (a_s[c] * w_s): the products come as 16-byte shared-memory loads, the
+                    // sums as packed fp32x2 operations (one instruction per two columns)
+                    float2* acc2 = reinterpret_cast<float2*>(acc);
+                    constexpr int kPiece = kCols < 32 ? 16 : 32;
+                    uint32_t v[2][kPiece];
+                    auto load = [&](int c, uint32_t (&dst)[kPiece]) {
+                        if constexpr (kPiece == 32) tmem_ld_32x32(taddr + c, dst);
+                        else tmem_ld_32x16(taddr + c, dst);
+                    };
+                    load(0, v[0]);
 #pragma unroll
-                    for (int c = 0; c < kCols; c += 32) {
+                    for (int c = 0; c < kCols; c += kPiece) {
                         tmem_ld_wait();
-                        if (c + 32 < kCols) tmem_ld_32x32(taddr + c + 32, v[((c >> 5) + 1) & 1]);
-                        const uint32_t* x = v[(c >> 5) & 1];
+                        if (c + kPiece < kCols) load(c + kPiece, v[(c / kPiece + 1) & 1]);
+                        const uint32_t* x = v[(c / kPiece) & 1];
                         const float4* s4 = reinterpret_cast<const float4*>(sc + c);
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4) {
+                        for (int i = 0; i < kPiece; i += 4) {
                             const float4 sv = s4[i >> 2];
-                            const float2 s01 = kPreScale ? make_float2(sv.x, sv.y) : __fmul2_rn(make_float2(sv.x, sv.y), w2);
-                            const float2 s23 = kPreScale ? make_float2(sv.z, sv.w) : __fmul2_rn(make_float2(sv.z, sv.w), w2);
                             acc2[(c + i) >> 1] = __ffma2_rn(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])),
-                                                            s01, acc2[(c + i) >> 1]);
-                            acc2[((c + i) >> 1) + 1] = __ffma2_rn(
-                                make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), s23,
-                                acc2[((c + i) >> 1) + 1]);
+                                                            make_float2(sv.x, sv.y), acc2[(c + i) >> 1]);
+                            acc2[((c + i) >> 1) + 1] = __ffma2_rn(make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])),
+                                                                  make_float2(sv.z, sv.w), acc2[((c + i) >> 1) + 1]);
                         }
                     }
-                } else if constexpr (kCols == 16) {
-                    uint32_t v[16];
-                    tmem_ld_32x16(taddr, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) acc[i] = fmaf(__uint_as_float(v[i]), sc[i] * wsc, acc[i]);
-                } else {
-                    uint32_t v[8];
-                    tmem_ld_32x8(taddr, v);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc[i] = fmaf(__uint_as_float(v[i]), sc[i] * wsc, acc[i]);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(empty_tm + ts * 8);
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(empty_tm + ts * 8);
-            }
-            tring.step(kStep, kTS);
-            ++j;
             }
 
             // ---- end of a segment: the tile's K range ended, or this CTA's range did
@@ -459,19 +386,35 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                     }
                     epi_bar_sync();                      // the buffer is free for the next segment
                 }
+                const int c0 = half * kHalf;             // this thread finishes columns c0 .. c0 + kHalf - 1
                 const int nrow = tile * kTileN + row_in_tile;
                 const bool from_zero = (seg_kb0 == 0), to_end = (kb + 1 == p.kb);
-                if (!from_zero) {
-                    // A partial that does not start the tile's K range goes to this CTA's slot;
-                    // the CTA that holds the start of the range collects it.  Layout
-                    // [column][row]: a warp's 32 rows are contiguous.
-                    float* slot = p.scratch + static_cast<int64_t>(blockIdx.x) * (M_PAD * kTileN) + row_in_tile;
+                if (p.split > 0 || !from_zero) {
+                    // partial sums to this CTA's slot, 16 bytes = four columns of a row
+                    float4* slot = reinterpret_cast<float4*>(p.scratch + static_cast<int64_t>(blockIdx.x) * kSlotFloats) + row_in_tile;
                     if (alive) {
 #pragma unroll
-                        for (int i = 0; i < kHalf; ++i) __stcg(slot + (half * kHalf + i) * kTileN, acc[i]);
+                        for (int i = 0; i < kHalf; i += 4)
+                            if (c0 + i < p.M) __stcg(slot + (c0 + i) / 4 * kTileN, make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]));
                     }
                     __threadfence();
                     epi_bar_sync();
+                }
+                if (p.split > 0) {
+                    // every CTA of the tile adds one slice of it over all partials, in K order
+                    int32_t* counter = p.flags + tile;
+                    if (et == 0 && alive) {
+                        add_acq_rel_gpu(counter, 1);
+                        await_word(counter, [&](int v) { return (v & 0xffff) == p.split; }, abort_flag, p.status);
+                    }
+                    epi_bar_sync();
+                    alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                    if (alive)
+                        gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile, p.split, et, 32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
+                    epi_bar_sync();
+                    // the last to leave puts the counter back to zero
+                    if (et == 0 && alive && (add_acq_rel_gpu(counter, 0x10000) >> 16) == p.split - 1) st_release_gpu(counter, 0);
+                } else if (!from_zero) {
                     if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
                 } else {
                     if (!to_end) {
@@ -480,27 +423,27 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                         // partials in CTA order, so the sum does not depend on timing.
                         const long long t_end = static_cast<long long>(tile + 1) * p.kb - 1;
                         const int last = cta_of(units, t_end, gridDim.x);
-                        // every contributor's flag is awaited by a thread of its own, then the partials are
-                        // added in CTA order (the loads of different partials overlap)
-                        for (int c = blockIdx.x + 1 + et; c <= last && alive; c += 32 * kEpiWarps) {
-                            const unsigned long long start = globaltimer_ns();
-                            uint32_t spins = 0;
-                            while (ld_acquire_gpu(p.flags + c) == 0) {
-                                if ((++spins & 255u) == 0u && (*abort_flag || globaltimer_ns() - start > kWaitLimitNs)) {
-                                    *abort_flag = 1;
-                                    if (p.status) atomicCAS(p.status, 0, kDevTimeoutPeerFlag);
-                                    break;
-                                }
-                                __nanosleep(64);
-                            }
-                        }
+                        // every contributor's flag is awaited by a thread of its own
+                        for (int c = blockIdx.x + 1 + et; c <= last && alive; c += 32 * kEpiWarps)
+                            await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
                         epi_bar_sync();
-                        alive = alive && !*abort_flag;
+                        alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                         if (alive) {
                             for (int c = blockIdx.x + 1; c <= last; ++c) {
-                                const float* peer = p.scratch + static_cast<int64_t>(c) * (M_PAD * kTileN) + row_in_tile;
+                                const float4* peer = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * kSlotFloats) + row_in_tile;
+                                constexpr int kPiece = kHalf < 32 ? kHalf : 32;
 #pragma unroll
-                                for (int i = 0; i < kHalf; ++i) acc[i] += __ldcg(peer + (half * kHalf + i) * kTileN);
+                                for (int i0 = 0; i0 < kHalf; i0 += kPiece)
+                                    if (c0 + i0 < p.M) {
+                                        float4 v[kPiece / 4];
+#pragma unroll
+                                        for (int i = 0; i < kPiece / 4; ++i) v[i] = __ldcg(peer + ((c0 + i0) / 4 + i) * kTileN);
+#pragma unroll
+                                        for (int i = 0; i < kPiece / 4; ++i) {
+                                            acc[i0 + 4 * i] += v[i].x, acc[i0 + 4 * i + 1] += v[i].y;
+                                            acc[i0 + 4 * i + 2] += v[i].z, acc[i0 + 4 * i + 3] += v[i].w;
+                                        }
+                                    }
                             }
                         }
                         epi_bar_sync();
@@ -520,7 +463,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                         if (alive) {
 #pragma unroll
                             for (int i = 0; i < kHalf; ++i)
-                                p.tp_peer_inbox[tile_off + (half * kHalf + i) * kTileN] = acc[i];
+                                p.tp_peer_inbox[tile_off + (c0 + i) * kTileN] = acc[i];
                         }
                         __threadfence_system();
                         epi_bar_sync();
@@ -538,18 +481,31 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                             }
                         }
                         epi_bar_sync();
-                        alive = alive && !*abort_flag;
+                        alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                         if (alive) {
 #pragma unroll
                             for (int i = 0; i < kHalf; ++i)
-                                acc[i] += ld_volatile_f32(p.tp_my_inbox + tile_off + (half * kHalf + i) * kTileN);
+                                acc[i] += ld_volatile_f32(p.tp_my_inbox + tile_off + (c0 + i) * kTileN);
                         }
                     }
-                    if (alive && nrow < p.N) {
+                    if (alive) {
+                        if ((p.N & 3) == 0 && (reinterpret_cast<uintptr_t>(p.c) & 7u) == 0) {
+                            // four lanes with neighbouring weight rows exchange, so that each stores 8 bytes of one activation row
+                            __nv_bfloat16* c = p.c + tile * kTileN + (row_in_tile & ~3);
 #pragma unroll
-                        for (int i = 0; i < kHalf; ++i) {
-                            const int m = half * kHalf + i;
-                            if (m < p.M) p.c[static_cast<int64_t>(m) * p.N + nrow] = __float2bfloat16_rn(acc[i]);
+                            for (int i = 0; i < kHalf; i += 4)
+                                if (c0 + i < p.M) {
+                                    uint32_t rows01, rows23;
+                                    gemmtc::transpose4(gemmtc::to_bf16x2(acc[i], acc[i + 1]), gemmtc::to_bf16x2(acc[i + 2], acc[i + 3]), lane,
+                                                       rows01, rows23);
+                                    const int m = c0 + i + static_cast<int>(lane & 3);
+                                    if (m < p.M && nrow < p.N)
+                                        *reinterpret_cast<uint2*>(c + static_cast<int64_t>(m) * p.N) = make_uint2(rows01, rows23);
+                                }
+                        } else if (nrow < p.N) {
+#pragma unroll
+                            for (int i = 0; i < kHalf; ++i)
+                                if (c0 + i < p.M) p.c[static_cast<int64_t>(c0 + i) * p.N + nrow] = __float2bfloat16_rn(acc[i]);
                         }
                     }
                 }
@@ -562,13 +518,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 ++tile;
             }
         }
-        cp_async_wait<0>();
     }
 
     __syncthreads();
     if (*abort_flag) abort_drain_sleep();
     __syncthreads();
-    if (warp == kProducers) {
+    if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, L::kTmemCols);
     }
@@ -586,30 +541,23 @@ template <int M_PAD>
 static int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, Params& p, const DeviceInfo& dev,
                   cudaStream_t stream) {
     using L = Smem<M_PAD>;
-    // resident activations if they leave room for six or more weight stages (96 KB in flight)
-    int stages = 16, rkb = p.kb;
-    while (stages > 6 && L::total(stages, rkb) > dev.smem_optin) stages -= 2;
-    if (p.group_tiles || L::total(stages, rkb) > dev.smem_optin) {   // groups read different activation columns
-        rkb = 0;
-        stages = 16;
-        while (stages > 2 && L::total(stages) > dev.smem_optin) stages -= 2;
-    }
-    const int smem = L::total(stages, rkb);
+    int stages = kMaxStages;
+    while (stages > 2 && L::total(stages, p.a_rows) > dev.smem_optin) --stages;
+    const int smem = L::total(stages, p.a_rows);
     if (smem > dev.smem_optin)
         return fail(WUDA_ERR_UNSUPPORTED, "device offers %d bytes of shared memory per block; the kernel needs more",
                     dev.smem_optin);
     p.stages = stages;
-    p.a_resident = rkb > 0;
     auto kernel = gemm_fp8_kernel<M_PAD>;
     WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
     const long long units = static_cast<long long>(p.n_tiles) * p.kb;
-    // at most kMaxSplit CTAs share one weight tile: the tile's owner adds the others' partials one after
-    // the other, which costs more than it saves when a few tiles are cut into a hundred pieces
-    // (adding one partial costs the owner about as much as streaming M_PAD / 64 units, so wide tiles split less)
-    constexpr int kMaxSplit = M_PAD <= 16 ? 16 : (M_PAD == 32 ? 12 : (M_PAD == 64 ? 8 : 6));
     const int sms = gemm_sms(dev);
+    // (the two-rank form needs a finished tile in one CTA; the owner of a tile then adds at most kMaxSplit partials)
+    constexpr int kMaxSplit = M_PAD <= 16 ? 16 : (M_PAD == 32 ? 12 : (M_PAD == 64 ? 8 : 6));
+    p.split = p.tp_peer_inbox ? 0 : gemmtc::tile_split(p.n_tiles, p.kb, sms);
     int grid = units < sms ? static_cast<int>(units) : sms;
-    if (static_cast<long long>(p.n_tiles) * kMaxSplit < grid) grid = p.n_tiles * kMaxSplit;
+    if (p.split > 0) grid = p.n_tiles * p.split;
+    else if (static_cast<long long>(p.n_tiles) * kMaxSplit < grid) grid = p.n_tiles * kMaxSplit;
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem, stream, w_map, a_map, p));
     return WUDA_OK;
 }
@@ -688,6 +636,9 @@ int gemm_fp8_setup_and_launch(const GemmCall& g) {
     p.n_tiles = (n_all + 127) / 128;
     p.group_tiles = g.groups > 1 ? g.n / 128 : 0;
     p.a_kb_total = g.groups * (g.k / 128);
+    p.a_rows = gemmtc::rows_of(g.m);
+    p.vec_scales = p.kb % 4 == 0 && aligned16(g.a_scales);
+    p.split = 0;
     p.scratch = g.slots;
     p.flags = g.flags;
     p.stages = 0;
@@ -713,7 +664,7 @@ int gemm_fp8_setup_and_launch(const GemmCall& g) {
     {
         const uint64_t dims[2] = {static_cast<uint64_t>(g.k) * g.groups, static_cast<uint64_t>(g.m)};
         const uint64_t strides[1] = {static_cast<uint64_t>(g.k) * g.groups};
-        const uint32_t box[2] = {128u, static_cast<uint32_t>(m_pad)};
+        const uint32_t box[2] = {128u, static_cast<uint32_t>(p.a_rows)};
         st = encode_tensor_map(&a_map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, g.a, dims, strides, box,
                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
         if (st != WUDA_OK) return st;

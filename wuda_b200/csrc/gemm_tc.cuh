@@ -155,9 +155,7 @@ __device__ __forceinline__ void umma_mxf8(uint32_t d_tmem, uint64_t a_desc, uint
         : "memory");
 }
 
-template <Kind KIND>
-__device__ __forceinline__ uint32_t to_bf16x2(float a, float b, float scale) {
-    if (KIND == Kind::kNv4) a *= scale, b *= scale;
+__device__ __forceinline__ uint32_t to_bf16x2(float a, float b) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
     return reinterpret_cast<const uint32_t&>(v);
 }
@@ -171,6 +169,39 @@ __device__ __forceinline__ void transpose4(uint32_t c01, uint32_t c23, uint32_t 
     const uint32_t even_rows = odd ? other : low, odd_rows = odd ? high : other;   // rows (0, 2) and (1, 3) of the lane's column
     rows01 = __byte_perm(even_rows, odd_rows, 0x5410);
     rows23 = __byte_perm(even_rows, odd_rows, 0x7632);
+}
+
+// This CTA's slice of a weight tile shared by `split` CTAs: the sum over all partials, in K order, scaled and stored.
+// A thread adds four activation rows of a weight row, eight partials in flight.
+template <Kind KIND>
+__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, int split, int thread, int threads, int M,
+                                          int N, float out_scale, int c_is_fp32, void* c) {
+    const int j = static_cast<int>(blockIdx.x) - tile * split, quads = (M + 3) / 4 * kTileN;
+    const float4* part = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(tile) * split * slot_floats);
+    const int end = quads * (j + 1) / split;
+    for (int e = quads * j / split + thread; e < end; e += threads) {
+        float4 v = __ldcg(part + e);
+        for (int q0 = 1; q0 < split; q0 += 8) {
+            float4 x[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) x[q] = __ldcg(part + min(q0 + q, split - 1) * (slot_floats / 4) + e);
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if (q0 + q < split) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
+        }
+        const float out[4] = {v.x, v.y, v.z, v.w};
+        const int m = e / kTileN * 4, nr = tile * kTileN + e % kTileN;
+        if (nr < N) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (m + i < M) {
+                    const int64_t at = static_cast<int64_t>(m + i) * N + nr;
+                    const float o = KIND == Kind::kNv4 ? out[i] * out_scale : out[i];
+                    if (KIND == Kind::kBf16 && c_is_fp32) static_cast<float*>(c)[at] = o;
+                    else static_cast<__nv_bfloat16*>(c)[at] = __float2bfloat16_rn(o);
+                }
+        }
+    }
 }
 
 // One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter).
@@ -609,35 +640,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 }
                 epi_sync();
                 alive = __all_sync(0xffffffffu, alive && !*abort_flag);
-                if (alive) {
-                    // a thread adds four activation rows of a weight row, eight partials in flight
-                    const int j = static_cast<int>(blockIdx.x) - tile * p.split, quads = (p.M + 3) / 4 * kTileN;
-                    const float4* part = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(tile) * p.split * slot_floats);
-                    const int end = quads * (j + 1) / p.split;
-                    for (int e = quads * j / p.split + et; e < end; e += kEpi) {
-                        float4 v = __ldcg(part + e);
-                        for (int q0 = 1; q0 < p.split; q0 += 8) {
-                            float4 x[8];
-#pragma unroll
-                            for (int q = 0; q < 8; ++q) x[q] = __ldcg(part + min(q0 + q, p.split - 1) * (slot_floats / 4) + e);
-#pragma unroll
-                            for (int q = 0; q < 8; ++q)
-                                if (q0 + q < p.split) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
-                        }
-                        const float out[4] = {v.x, v.y, v.z, v.w};
-                        const int m = e / kTileN * 4, nr = nrow0 + e % kTileN;
-                        if (nr < p.N) {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i)
-                                if (m + i < p.M) {
-                                    const int64_t at = static_cast<int64_t>(m + i) * p.N + nr;
-                                    const float o = KIND == Kind::kNv4 ? out[i] * p.out_scale : out[i];
-                                    if (KIND == Kind::kBf16 && p.c_is_fp32) static_cast<float*>(p.c)[at] = o;
-                                    else static_cast<__nv_bfloat16*>(p.c)[at] = __float2bfloat16_rn(o);
-                                }
-                        }
-                    }
-                }
+                if (alive)
+                    add_slice<KIND>(p.scratch, slot_floats, tile, p.split, et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32, p.c);
                 epi_sync();
                 // the last to leave puts the counter back to zero
                 if (et == 0 && alive && (add_acq_rel_gpu(counter, 0x10000) >> 16) == p.split - 1) st_release_gpu(counter, 0);
@@ -683,13 +687,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                                   (reinterpret_cast<uintptr_t>(p.c) & 7u) == 0;
                 if (wide) {
                     if (alive) {
+                        const float out = KIND == Kind::kNv4 ? p.out_scale : 1.f;
                         __nv_bfloat16* c = static_cast<__nv_bfloat16*>(p.c) + nrow0 + (row & ~3);
                         const bool in_n = nrow < p.N;    // (N is a multiple of four: the four lanes agree)
 #pragma unroll
                         for (int i = 0; i < kCols; i += 4)
                             if (col0 + i < p.M) {
                                 uint32_t rows01, rows23;
-                                transpose4(to_bf16x2<KIND>(acc[i], acc[i + 1], p.out_scale), to_bf16x2<KIND>(acc[i + 2], acc[i + 3], p.out_scale),
+                                transpose4(to_bf16x2(acc[i] * out, acc[i + 1] * out), to_bf16x2(acc[i + 2] * out, acc[i + 3] * out),
                                            lane, rows01, rows23);
                                 const int m = col0 + i + static_cast<int>(lane & 3);
                                 if (m < p.M && in_n) *reinterpret_cast<uint2*>(c + static_cast<int64_t>(m) * p.N) = make_uint2(rows01, rows23);
