@@ -23,8 +23,8 @@
 //    two accumulator sets are added when a tile's segment ends.  (Above 64 activation rows a thread cannot hold all
 //    columns; the groups then split the columns and both take every unit.)
 // Measured (CUDA-graph replays, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
-// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 37.1,
-// 43.9 -> 38.4, 62.7 -> 46.8, 122.5 -> 91.1 (two passes); 7168 x 16384 at 64 rows 32.5 -> 29.5; 2112 x 7168 at 1 / 64 rows
+// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 35.9,
+// 43.9 -> 37.9, 62.7 -> 45.7, 122.5 -> 89.5 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.7; 2112 x 7168 at 1 / 64 rows
 // 12.3 -> 10.3, 15.3 -> 12.3.  Where the split is stream-K (more than a third of the SMs hold tiles) the results are
 // bit-identical to those of the earlier form: the order of the additions is the same.
 // Every wait is bounded and reports through the status word.
@@ -55,7 +55,8 @@ using gemmtc::st_release_gpu;
 constexpr int kFirstEpiWarp = 4;     // warp 0 copies, 1 issues MMAs, 2 prepares scales, 3 is idle, 4..11 are two epilogue warpgroups
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 32 * (kFirstEpiWarp + kEpiWarps);
-constexpr int kMaxStages = 12;
+// (more copies in flight cost DRAM efficiency: 24576 x 7168 at 16 rows 35.9 us with 6 stages, 37.3 with 10)
+constexpr int kMaxStages = 6;
 
 struct Params {
     const float* a_scales;     // [M, a_kb_total]
@@ -98,7 +99,7 @@ struct Smem {
     static __host__ __device__ constexpr int scale_off(int stages, int a_rows) { return stages * stage_bytes(a_rows); }
     static __host__ __device__ constexpr int comb_off(int stages, int a_rows) { return scale_off(stages, a_rows) + kTmemStages * M_PAD * 4; }
     static __host__ __device__ constexpr int bar_off(int stages, int a_rows) { return comb_off(stages, a_rows) + kCombineBytes; }
-    // barriers: full[12] empty[12] full_tm[8] empty_tm[8]
+    // barriers: full[6] empty[6] full_tm[8] empty_tm[8]
     static __host__ __device__ constexpr int misc_off(int stages, int a_rows) { return bar_off(stages, a_rows) + (2 * kMaxStages + 16) * 8; }
     static __host__ __device__ constexpr int total(int stages, int a_rows) { return misc_off(stages, a_rows) + 32 + 1024; }
 };
