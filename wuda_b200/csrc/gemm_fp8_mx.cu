@@ -19,9 +19,9 @@
 // reads as 2^-127.
 // Measured (CUDA-graph replays, us; before = scale images built unit by unit by the fetching warps, two accumulators,
 // passes of 128 rows, partials added by one CTA per tile):
-//   24576 x 7168 at 64 rows 41.0 -> 36.0; 7168 x 16384 at 256 rows 69.5 -> 43.9; 73728 x 1536 at 64 rows (the q
-//   projection; before with the activations resident in shared memory) 28.8 -> 28.1; 4096 x 7168 at 16 rows 14.4 -> 12.5;
-//   4-bit weights: 24576 x 7168 at 64 rows 32.0 -> 30.8, 7168 x 16384 at 200 rows 76 -> 43
+//   24576 x 7168 at 64 rows 41.0 -> 35.1; 7168 x 16384 at 256 rows 69.5 -> 40.3; 73728 x 1536 at 64 rows (the q
+//   projection; before with the activations resident in shared memory) 28.8 -> 25.8; 4096 x 7168 at 64 rows 20.5 -> 14.7;
+//   4-bit weights: 24576 x 7168 at 64 rows 32.0 -> 28.7, 7168 x 16384 at 200 rows 76 -> 39
 #include "gemm_tc.cuh"
 
 namespace wuda {

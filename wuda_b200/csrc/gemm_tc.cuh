@@ -90,7 +90,11 @@ struct Layout {
     // 4-bit activations of the experts behind them turn those into 1e-2 of the layer's output.
     static constexpr int kAccs = KIND == Kind::kMx8 && M_PAD <= 128 ? 2 : 1;
     static constexpr int kBuffers = kAccs * M_PAD <= 128 ? 2 : 1;
-    static constexpr int kEpiWarps = M_PAD >= 128 ? 8 : 4;
+    // Epilogue warps: behind the last copy they move partial sums and results with the bytes in flight that they have, so
+    // 256 rows take sixteen (7168 x 16384 FP8 43.8 -> 40.4 us; not with 4-bit weights, whose scale images need the
+    // registers).  At 128 rows sixteen gain 0.4 us of 24.8 alone but leave no registers for the next kernel of a chain to
+    // set itself up beside this one: the layer at batch 128 takes 1452 instead of 1438 us.
+    static constexpr int kEpiWarps = M_PAD == 256 && KIND != Kind::kMx8W4 ? 16 : (M_PAD >= 64 ? 8 : 4);
     static constexpr int kThreads = 32 * (4 + kEpiWarps);
     static constexpr int kCols = M_PAD / (kEpiWarps / 4);             // accumulator columns per epilogue thread
     // scale columns of one set (two sets alternate)
@@ -590,6 +594,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                     }
                 }
             }
+            // The start of a tile whose K range goes on in the following CTAs (all resident: the grid is one CTA per SM): their
+            // partials were finished first, so the flags are awaited (each by a thread of its own) and the first partial
+            // is fetched while this segment's MMAs still run.
+            const bool owner = p.split == 0 && from_zero && !to_end;
+            constexpr bool kAhead = kCols <= 32;      // (what the registers hold)
+            float4 ahead[kAhead ? kCols / 4 : 1];
+            int last = blockIdx.x;
+            auto slot_of = [&](int c) {
+                return reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * slot_floats) + col0 / 4 * kTileN + row;
+            };
+            if (owner) {
+                last = cta_of(units, static_cast<long long>(tile + 1) * p.kb - 1, grid);
+                for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
+                    await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
+                epi_sync();
+                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                if (kAhead && alive && col0 < p.M) {     // (the slot of a CTA has room for M_PAD columns)
+#pragma unroll
+                    for (int i = 0; i < kCols / 4; ++i) ahead[i] = __ldcg(slot_of(blockIdx.x + 1) + i * kTileN);
+                }
+            }
             if (alive) alive = mbar_wait_warp_fast(full_tm + buf * 8, (seg / kBuffers) & 1u, abort_flag, p.status, kDevTimeoutGemmTmemFull);
             float acc[kCols];
             if (alive) {
@@ -648,26 +673,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             } else if (!from_zero) {
                 if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
             } else {
-                if (!to_end) {
-                    const long long t_end = static_cast<long long>(tile + 1) * p.kb - 1;
-                    const int last = cta_of(units, t_end, grid);
-                    // every contributor's flag is awaited by a thread of its own, then the partials are added in CTA order
-                    for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
-                        await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
-                    epi_sync();
-                    alive = __all_sync(0xffffffffu, alive && !*abort_flag);
-                    if (alive) {
+                if (owner) {     // add the partials in CTA order
+                    if (alive && col0 < p.M) {
                         for (int c = blockIdx.x + 1; c <= last; ++c) {
-                            const float4* peer = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * slot_floats) + row;
                             // (pieces of 32 columns, eight 16-byte loads in flight each: a condition per load would wait for
-                            // every one by itself; the slot of a CTA has room for M_PAD columns)
+                            // every one by itself)
                             constexpr int kPiece = kCols < 32 ? kCols : 32;
 #pragma unroll
                             for (int c0 = 0; c0 < kCols; c0 += kPiece)
                                 if (col0 + c0 < p.M) {
                                     float4 v[kPiece / 4];
 #pragma unroll
-                                    for (int i = 0; i < kPiece / 4; ++i) v[i] = __ldcg(peer + ((col0 + c0) / 4 + i) * kTileN);
+                                    for (int i = 0; i < kPiece / 4; ++i)
+                                        v[i] = kAhead && c == static_cast<int>(blockIdx.x) + 1 ? ahead[i] : __ldcg(slot_of(c) + (c0 / 4 + i) * kTileN);
 #pragma unroll
                                     for (int i = 0; i < kPiece / 4; ++i) {
                                         acc[c0 + 4 * i] += v[i].x, acc[c0 + 4 * i + 1] += v[i].y;
