@@ -42,7 +42,7 @@
 namespace wuda {
 namespace gemm8 {
 
-using gemmtc::add_acq_rel_gpu;
+using gemmtc::arrive_and_wait;
 using gemmtc::await_word;
 using gemmtc::cta_of;
 using gemmtc::kRowBytes;
@@ -404,17 +404,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 if (p.split > 0) {
                     // every CTA of the tile adds one slice of it over all partials, in K order
                     int32_t* counter = p.flags + tile;
-                    if (et == 0 && alive) {
-                        add_acq_rel_gpu(counter, 1);
-                        await_word(counter, [&](int v) { return (v & 0xffff) == p.split; }, abort_flag, p.status);
-                    }
+                    if (et == 0 && alive) arrive_and_wait(counter, p.split, abort_flag, p.status);
                     epi_bar_sync();
                     alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                     if (alive)
                         gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile, p.split, et, 32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
-                    epi_bar_sync();
-                    // the last to leave puts the counter back to zero
-                    if (et == 0 && alive && (add_acq_rel_gpu(counter, 0x10000) >> 16) == p.split - 1) st_release_gpu(counter, 0);
                 } else if (!from_zero) {
                     if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
                 } else {

@@ -124,9 +124,10 @@ __device__ __forceinline__ int ld_acquire_gpu(const int32_t* p) {
     asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ int add_acq_rel_gpu(int32_t* p, int v) {
+// old >= limit ? 0 : old + 1
+__device__ __forceinline__ int inc_acq_rel_gpu(int32_t* p, int limit) {
     int old;
-    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
+    asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(limit) : "memory");
     return old;
 }
 __device__ __forceinline__ long long range_begin(long long units, int c, int grid) { return units * c / grid; }
@@ -175,6 +176,29 @@ __device__ __forceinline__ void transpose4(uint32_t c01, uint32_t c23, uint32_t 
     rows23 = __byte_perm(even_rows, odd_rows, 0x7632);
 }
 
+// One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter).
+template <typename Pred>
+__device__ __forceinline__ void await_word(const int32_t* word, Pred done, volatile int* abort_flag, int32_t* status) {
+    if (done(ld_acquire_gpu(word))) return;
+    const unsigned long long start = globaltimer_ns();
+    uint32_t spins = 0;
+    while (!done(ld_acquire_gpu(word))) {
+        if ((++spins & 255u) == 0u && (*abort_flag || globaltimer_ns() - start > kWaitLimitNs)) {
+            *abort_flag = 1;
+            if (status) atomicCAS(status, 0, static_cast<int>(kDevTimeoutPeerFlag));
+            break;
+        }
+    }
+}
+
+// One thread's arrival at the counter of a tile that `split` CTAs share, and its wait for the others.  The last arrival wraps
+// the counter back to zero, which is what the others wait for: nobody has to reset it (as a second, departing atomic did,
+// 0.5 us behind the results).  No CTA arrives at a counter twice in a launch, and the next launch's arrive after this one.
+__device__ __forceinline__ void arrive_and_wait(int32_t* counter, int split, volatile int* abort_flag, int32_t* status) {
+    if (inc_acq_rel_gpu(counter, split - 1) != split - 1)
+        await_word(counter, [](int v) { return v == 0; }, abort_flag, status);
+}
+
 // This CTA's slice of a weight tile shared by `split` CTAs: the sum over all partials, in K order, scaled and stored.
 // A thread adds four activation rows of a weight row, eight partials in flight.
 template <Kind KIND>
@@ -204,21 +228,6 @@ __device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_flo
                     if (KIND == Kind::kBf16 && c_is_fp32) static_cast<float*>(c)[at] = o;
                     else static_cast<__nv_bfloat16*>(c)[at] = __float2bfloat16_rn(o);
                 }
-        }
-    }
-}
-
-// One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter).
-template <typename Pred>
-__device__ __forceinline__ void await_word(const int32_t* word, Pred done, volatile int* abort_flag, int32_t* status) {
-    if (done(ld_acquire_gpu(word))) return;
-    const unsigned long long start = globaltimer_ns();
-    uint32_t spins = 0;
-    while (!done(ld_acquire_gpu(word))) {
-        if ((++spins & 255u) == 0u && (*abort_flag || globaltimer_ns() - start > kWaitLimitNs)) {
-            *abort_flag = 1;
-            if (status) atomicCAS(status, 0, static_cast<int>(kDevTimeoutPeerFlag));
-            break;
         }
     }
 }
@@ -659,17 +668,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (p.split > 0) {
                 // every CTA of the tile adds one slice of it over all partials, in K order
                 int32_t* counter = p.flags + tile;
-                if (et == 0 && alive) {
-                    add_acq_rel_gpu(counter, 1);
-                    await_word(counter, [&](int v) { return (v & 0xffff) == p.split; }, abort_flag, p.status);
-                }
+                if (et == 0 && alive) arrive_and_wait(counter, p.split, abort_flag, p.status);
                 epi_sync();
                 alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                 if (alive)
                     add_slice<KIND>(p.scratch, slot_floats, tile, p.split, et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32, p.c);
-                epi_sync();
-                // the last to leave puts the counter back to zero
-                if (et == 0 && alive && (add_acq_rel_gpu(counter, 0x10000) >> 16) == p.split - 1) st_release_gpu(counter, 0);
             } else if (!from_zero) {
                 if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
             } else {
