@@ -23,9 +23,9 @@
 //    two accumulator sets are added when a tile's segment ends.  (Above 64 activation rows a thread cannot hold all
 //    columns; the groups then split the columns and both take every unit.)
 // Measured (CUDA-graph replays, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
-// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 35.9,
-// 43.9 -> 37.9, 62.7 -> 45.7, 122.5 -> 89.5 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.7; 2112 x 7168 at 1 / 64 rows
-// 12.3 -> 10.3, 15.3 -> 12.3.  Where the split is stream-K (more than a third of the SMs hold tiles) the results are
+// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 35.0,
+// 43.9 -> 37.2, 62.7 -> 45.9, 122.5 -> 89.7 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.8; 2112 x 7168 at 1 / 64 rows
+// 12.3 -> 10.3, 15.3 -> 10.3; 4096 x 7168 at 64 rows 17.8 -> 14.4.  Where the split is stream-K (more than a third of the SMs hold tiles) the results are
 // bit-identical to those of the earlier form: the order of the additions is the same.
 // Every wait is bounded and reports through the status word.
 #include <cuda.h>
@@ -52,7 +52,7 @@ using gemmtc::ld_acquire_gpu;
 using gemmtc::range_begin;
 using gemmtc::st_release_gpu;
 
-constexpr int kFirstEpiWarp = 4;     // warp 0 copies, 1 issues MMAs, 2 prepares scales, 3 is idle, 4..11 are two epilogue warpgroups
+constexpr int kFirstEpiWarp = 4;     // warp 0 copies, 1 issues MMAs, 2 prepares scales, 3 awaits partials, 4..11 are two epilogue warpgroups
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 32 * (kFirstEpiWarp + kEpiWarps);
 // (more copies in flight cost DRAM efficiency: 24576 x 7168 at 16 rows 35.9 us with 6 stages, 37.3 with 10)
@@ -99,8 +99,8 @@ struct Smem {
     static __host__ __device__ constexpr int scale_off(int stages, int a_rows) { return stages * stage_bytes(a_rows); }
     static __host__ __device__ constexpr int comb_off(int stages, int a_rows) { return scale_off(stages, a_rows) + kTmemStages * M_PAD * 4; }
     static __host__ __device__ constexpr int bar_off(int stages, int a_rows) { return comb_off(stages, a_rows) + kCombineBytes; }
-    // barriers: full[6] empty[6] full_tm[8] empty_tm[8]
-    static __host__ __device__ constexpr int misc_off(int stages, int a_rows) { return bar_off(stages, a_rows) + (2 * kMaxStages + 16) * 8; }
+    // barriers: full[6] empty[6] full_tm[8] empty_tm[8] partials
+    static __host__ __device__ constexpr int misc_off(int stages, int a_rows) { return bar_off(stages, a_rows) + (2 * kMaxStages + 17) * 8; }
     static __host__ __device__ constexpr int total(int stages, int a_rows) { return misc_off(stages, a_rows) + 32 + 1024; }
 };
 
@@ -133,9 +133,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     const int S = p.stages;
     const uint32_t stage_bytes = L::stage_bytes(p.a_rows);
     const uint32_t bars = base + L::bar_off(S, p.a_rows);
-    const uint32_t full = bars, empty = full + kMaxStages * 8, full_tm = empty + kMaxStages * 8, empty_tm = full_tm + 8 * 8;
+    const uint32_t full = bars, empty = full + kMaxStages * 8, full_tm = empty + kMaxStages * 8, empty_tm = full_tm + 8 * 8, partials = empty_tm + 8 * 8;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, p.a_rows));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 4);
+    volatile int* last_peer_slot = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 8);
     float* products = reinterpret_cast<float*>(base_ptr + L::scale_off(S, p.a_rows));     // [kTS][M_PAD]: a_s * w_s
     float* comb = reinterpret_cast<float*>(base_ptr + L::comb_off(S, p.a_rows));
     constexpr bool kAlt = L::kAlternate;
@@ -153,6 +154,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             mbar_init(full_tm + i * 8, 2);        // the MMAs have retired and the scale products are written
             mbar_init(empty_tm + i * 8, kAlt ? kEpiWarps / 2 : kEpiWarps);   // the warps that read a stage
         }
+        mbar_init(partials, 1);
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -171,7 +173,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         u0 = range_begin(units, blockIdx.x, gridDim.x);
         count = static_cast<int>(range_begin(units, blockIdx.x + 1, gridDim.x) - u0);
     }
-    const int tile0 = static_cast<int>(u0 / p.kb), kb0 = static_cast<int>(u0 % p.kb);
+    const int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
+    // The last tile of a stream-K range may go on in the following CTAs (all resident: the grid is one CTA per SM).  If this
+    // CTA holds its start, it adds their partials, of CTAs blockIdx.x + 1 .. last_peer, in CTA order.
+    const long long last_tile = static_cast<uint32_t>(u0 + count - 1) / static_cast<uint32_t>(p.kb);
+    const bool shares = p.split == 0 && last_tile * p.kb >= u0 && (last_tile + 1) * p.kb > u0 + count;
     if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
@@ -301,6 +307,17 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             if (b.n >= count || !write(b)) break;
             fill(b);
         }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------ the other CTAs' partials, awaited beside the stream
+        // (each by a lane of its own; they are finished first)
+        if (shares) {
+            const int last_peer = cta_of(units, (last_tile + 1) * p.kb - 1, gridDim.x);
+            for (int c = blockIdx.x + 1 + static_cast<int>(lane); c <= last_peer; c += 32)
+                await_word<200>(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
+            if (lane == 0) *last_peer_slot = last_peer;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(partials);
+        }
     } else if (warp >= kFirstEpiWarp) {
         // ------------------------------------------------------------ epilogue
         const int ew = warp - kFirstEpiWarp;
@@ -413,15 +430,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                     if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
                 } else {
                     if (!to_end) {
-                        // This CTA holds the start of the tile's K range and the range continues in
-                        // the following CTAs (all resident: the grid is one CTA per SM).  Add their
-                        // partials in CTA order, so the sum does not depend on timing.
-                        const long long t_end = static_cast<long long>(tile + 1) * p.kb - 1;
-                        const int last = cta_of(units, t_end, gridDim.x);
-                        // every contributor's flag is awaited by a thread of its own
-                        for (int c = blockIdx.x + 1 + et; c <= last && alive; c += 32 * kEpiWarps)
-                            await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
-                        epi_bar_sync();
+                        if (alive) alive = mbar_wait_warp_fast(partials, 0, abort_flag, p.status, kDevTimeoutPeerFlag);
+                        const int last = *last_peer_slot;      // (an aborting CTA does not use it)
                         alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                         if (alive) {
                             for (int c = blockIdx.x + 1; c <= last; ++c) {

@@ -19,7 +19,7 @@
 // reads as 2^-127.
 // Measured (CUDA-graph replays, us; before = scale images built unit by unit by the fetching warps, two accumulators,
 // passes of 128 rows, partials added by one CTA per tile):
-//   24576 x 7168 at 64 rows 41.0 -> 35.1; 7168 x 16384 at 256 rows 69.5 -> 40.3; 73728 x 1536 at 64 rows (the q
+//   24576 x 7168 at 64 rows 41.0 -> 35.1; 7168 x 16384 at 256 rows 69.5 -> 39.3; 73728 x 1536 at 64 rows (the q
 //   projection; before with the activations resident in shared memory) 28.8 -> 25.8; 4096 x 7168 at 64 rows 20.5 -> 14.7;
 //   4-bit weights: 24576 x 7168 at 64 rows 32.0 -> 28.7, 7168 x 16384 at 200 rows 76 -> 39
 #include "gemm_tc.cuh"

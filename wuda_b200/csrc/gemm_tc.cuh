@@ -130,7 +130,12 @@ __device__ __forceinline__ int inc_acq_rel_gpu(int32_t* p, int limit) {
     asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(limit) : "memory");
     return old;
 }
-__device__ __forceinline__ long long range_begin(long long units, int c, int grid) { return units * c / grid; }
+// floor(units * c / grid) for fewer than 2^32 units (16 KB each), in 32-bit divisions: a launch's prologue is on the critical path of a short call, and a 64-bit
+// division takes a few hundred cycles
+__device__ __forceinline__ long long range_begin(long long units, int c, int grid) {
+    const uint32_t u = static_cast<uint32_t>(units), g = static_cast<uint32_t>(grid), q = u / g, rest = u - q * g;
+    return static_cast<long long>(q) * c + rest * static_cast<uint32_t>(c) / g;
+}
 __device__ __forceinline__ int cta_of(long long units, long long u, int grid) {
     int c = static_cast<int>(u * grid / units);
     while (c + 1 < grid && range_begin(units, c + 1, grid) <= u) ++c;
@@ -176,8 +181,9 @@ __device__ __forceinline__ void transpose4(uint32_t c01, uint32_t c23, uint32_t 
     rows23 = __byte_perm(even_rows, odd_rows, 0x7632);
 }
 
-// One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter).
-template <typename Pred>
+// One thread's bounded wait for a word in global memory (another CTA's flag or a tile's counter); SLEEP_NS > 0 where the wait
+// runs beside the stream and must not take its issue slots.
+template <unsigned SLEEP_NS = 0, typename Pred>
 __device__ __forceinline__ void await_word(const int32_t* word, Pred done, volatile int* abort_flag, int32_t* status) {
     if (done(ld_acquire_gpu(word))) return;
     const unsigned long long start = globaltimer_ns();
@@ -188,6 +194,7 @@ __device__ __forceinline__ void await_word(const int32_t* word, Pred done, volat
             if (status) atomicCAS(status, 0, static_cast<int>(kDevTimeoutPeerFlag));
             break;
         }
+        if (SLEEP_NS) __nanosleep(SLEEP_NS);
     }
 }
 
@@ -289,6 +296,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
         }
     }
+    int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
     if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
@@ -297,7 +305,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             prefetch_tmap(&asf_map);
         }
         if constexpr (KIND != Kind::kMx8W4) {
-            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+            int tile = tile0, kb = kb0;
             for (int n = 0; n < count && n < S; ++n) {
                 tma_prefetch_2d(&w_map, kb * (KIND == Kind::kBf16 ? kRowBytes / 2 : kRowBytes), tile * kTileN);
                 if (++kb == p.kb) kb = 0, ++tile;
@@ -320,6 +328,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if (static_cast<int>(blockIdx.x) < grid) {
             u0 = range_begin(units, blockIdx.x, grid);
             count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
+            tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
         }
     }
 
@@ -331,7 +340,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             const uint32_t tx = stage_bytes - (KIND == Kind::kMx8W4 ? kWBytes / 2 : 0);   // packed weights: the padding is not counted
             int s = 0;
             uint32_t phase = 1;
-            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+            int tile = tile0, kb = kb0;
             int seen_tile = -1, grp = grouped ? -1 : 0, expert = 0, wtile = 0;
             for (int n = 0; n < count; ++n) {
                 // grouped: `tile` is the flat index; the weight tile is the expert's, the activations the group's
@@ -374,7 +383,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if (elect_one()) {
             int s = 0;
             uint32_t phase = 0, seg = 0, img = 0, nv_set = 0;   // img: images taken so far
-            int kb = static_cast<int>(u0 % p.kb);
+            int kb = kb0;
             const uint32_t sf_cols = tmem_base + L::kAccCols;
             bool alive = true;
             for (int n = 0; n < count && alive;) {
@@ -461,7 +470,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         if constexpr (kMx) {
             constexpr int kQ = (M_PAD + 31) / 32;      // activation rows of a lane: lane, lane + 32, ..
             const uint32_t me = warp - 2;
-            int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb), n = 0;
+            int tile = tile0, kb = kb0, n = 0;
             auto advance = [&](int times) {
                 for (; times > 0; --times) {
                     const int len = min(4 - (kb & 3), p.kb - kb);
@@ -579,7 +588,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         const int row = et & 127, col0 = (et >> 7) * kCols;      // weight row inside the tile, first column
         const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
         bool alive = true;
-        int tile = static_cast<int>(u0 / p.kb), kb = static_cast<int>(u0 % p.kb);
+        int tile = tile0, kb = kb0;
         uint32_t seg = 0;
         const int64_t slot_floats = static_cast<int64_t>(M_PAD) * kTileN;
         int grp = 0, seen_grp = -1;
@@ -616,7 +625,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (owner) {
                 last = cta_of(units, static_cast<long long>(tile + 1) * p.kb - 1, grid);
                 for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
-                    await_word(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
+                    await_word<200>(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
                 epi_sync();
                 alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                 if (kAhead && alive && col0 < p.M) {     // (the slot of a CTA has room for M_PAD columns)
