@@ -28,9 +28,9 @@
 //               128-byte-swizzled operand layout.
 //               The same bytes serve as the K-major operand of Q K^T and as the MN-major
 //               operand of P V.
-//   warps 12-13 issue Q K^T, of the even and of the odd blocks: a thread gets one MMA out about every hundred
-//               cycles and spends as long again on the commit, the loop and its waits, so one of the two is
-//               already waiting for the score tile when the other's MMAs retire;
+//   warps 12-13 issue Q K^T, of the even and of the odd blocks (an MMA of M 128 x N 64 x K 16 takes the tensor pipe 62
+//               cycles, issuing it about ten): one of the two is already waiting for the score tile when the other's
+//               MMAs retire;
 //   warp 14     issues P V of a block as soon as its probabilities are stored.
 // Every wait is bounded; a wait that runs out leaves a code in the status word and the CTA
 // exits normally.
@@ -355,10 +355,8 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         if (clamped && p.status) atomicCAS(p.status, 0, static_cast<int>(kDevMlaScaleRange));
     } else if (warp == kIssuerWarp || warp == kIssuerWarp + 1) {
         // ------------------------------------------------------------ score issuers
-        // A block's 32 MMAs keep their issuing thread busy for longer than they keep the tensor pipe, and the commit,
-        // the loop and the two waits behind them cost that thread as much again while the other warps of its scheduler
-        // compute; so two threads take the blocks alternately: one is already waiting for the score tile to be read
-        // when the other's MMAs retire.  Each has its own pair of barriers, so that it sees every phase of the ones it
+        // Two threads take the blocks alternately: one is already waiting for the score tile to be read when the other's
+        // MMAs retire.  Each has its own pair of barriers, so that it sees every phase of the ones it
         // waits on.
         const int me = warp - kIssuerWarp;
         constexpr uint32_t idesc_qk = umma_idesc(kRows, kBlock, 0, 0);     // fp16 operands
