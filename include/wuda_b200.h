@@ -725,7 +725,7 @@ int wuda_gemm_fp8_grouped_pow2(const void* a, const float* a_scales, const void*
  *   w_packed e2m1 [n, k/2] bytes, the element of the lower K index in the low nibble (torch.float4_e2m1fn_x2);
  *            32-byte aligned
  *   w_sf     [n, k/32] exponent bytes (torch.float8_e8m0fnu): weight (row, j) = code * 2^(w_sf[row, j/32] - 127)
- *   c_bf16   bf16 [m, n];  0 <= m <= 256 (above 128 rows: two passes), k % 128 == 0
+ *   c_bf16   bf16 [m, n];  0 <= m <= 256, k % 128 == 0
  *   scratch  as for wuda_gemm_fp8_blockscaled (wuda_gemm_fp8_scratch_bytes(m, n))
  *
  * The kernel of wuda_gemm_fp8_blockscaled_pow2 with the weight operand read as e2m1 (the tile is 8 KB of global
@@ -806,7 +806,7 @@ int wuda_front_emit(const void* y8_bf16, const float* y16_f32, const int64_t* po
  * reference has no NVFP4 GEMM: its fp4_gemm (origin/kernel.py:441-536) is FP8-activation x
  * FP4-weight with 1x32 e8m0 scales; this entry is the 16-element-ue4m3 + per-tensor-fp32 form.
  *
- *   a  uint8 [m, k/2];  w  uint8 [n, k/2];  1 <= m <= 256 (above 128 rows: two passes over the weights), k % 256 == 0; 16-byte aligned
+ *   a  uint8 [m, k/2];  w  uint8 [n, k/2];  1 <= m <= 256, k % 256 == 0; 16-byte aligned
  *   a_sf_packed, w_sf_packed: the ue4m3 scale bytes in tensor-core order: per 128 rows x 256 K one
  *      2048-byte block [K/64 step (4)][row % 32 (32)][row / 32 (4)][scale of the step (4)],
  *      blocks ordered [row tile][k / 256]; rows beyond m / n are zero-padded to a multiple of 128

@@ -616,7 +616,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             // partials were finished first, so the flags are awaited (each by a thread of its own) and the first partial
             // is fetched while this segment's MMAs still run.
             const bool owner = p.split == 0 && from_zero && !to_end;
-            constexpr bool kAhead = kCols <= 32;      // (what the registers hold)
+            constexpr bool kAhead = kCols <= 32 || (M_PAD == 128 && !kMx);      // (what the registers hold without spills)
             float4 ahead[kAhead ? kCols / 4 : 1];
             int last = blockIdx.x;
             auto slot_of = [&](int c) {
@@ -697,7 +697,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                                     float4 v[kPiece / 4];
 #pragma unroll
                                     for (int i = 0; i < kPiece / 4; ++i)
-                                        v[i] = kAhead && c == static_cast<int>(blockIdx.x) + 1 ? ahead[i] : __ldcg(slot_of(c) + (c0 / 4 + i) * kTileN);
+                                        v[i] = kAhead && c == static_cast<int>(blockIdx.x) + 1 ? ahead[c0 / 4 + i] : __ldcg(slot_of(c) + (c0 / 4 + i) * kTileN);
 #pragma unroll
                                     for (int i = 0; i < kPiece / 4; ++i) {
                                         acc[c0 + 4 * i] += v[i].x, acc[c0 + 4 * i + 1] += v[i].y;
