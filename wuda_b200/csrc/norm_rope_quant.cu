@@ -56,8 +56,24 @@ __device__ __forceinline__ void quant_store8(const float (&v)[8], int pow2, uint
     for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(group_mask, amax, o));
     const float s = group_scale(amax, pow2);
     float q[8];
+    if (s < INFINITY) {
+        // v / s for eight v and one s: with r = 1/s correctly rounded, q0 = v r and the remainder v - q0 s (exact in an
+        // FMA), q0 + remainder * r is the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990) as long as the
+        // remainder does not underflow; where it does, |v / s| is far below half of the smallest e4m3 value and the code is
+        // a zero of v's sign either way.  Three instructions per value instead of a division: RMSNorm + RoPE quantisation of
+        // 256 tokens (7168 + 24576 values each) 18.1 -> 15.4 us, of one token 7.7 -> 7.0.
+        const float r = __frcp_rn(s);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = fminf(fmaxf(__fdiv_rn(v[i], s), -448.f), 448.f);
+        for (int i = 0; i < 8; ++i) {
+            const float q0 = __fmul_rn(v[i], r);
+            q[i] = copysignf(fmaf(fmaf(-q0, s, v[i]), r, q0), v[i]);     // (the sum of a negative zero and zero is positive)
+        }
+    } else {        // an infinite value in the group: v / inf
+#pragma unroll
+        for (int i = 0; i < 8; ++i) q[i] = __fdiv_rn(v[i], s);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) q[i] = fminf(fmaxf(q[i], -448.f), 448.f);
     uint2 packed;
     packed.x = pack_e4m3x4(q[0], q[1], q[2], q[3]);
     packed.y = pack_e4m3x4(q[4], q[5], q[6], q[7]);
