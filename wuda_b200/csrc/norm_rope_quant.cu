@@ -199,6 +199,11 @@ __global__ void __launch_bounds__(1024) rope_quant_kernel(const RopeParams p) {
     // (blockIdx.y splits a token's chunks over several CTAs when there are few tokens)
     // four 16-byte loads of a thread are in flight before the first is used: the kernel is a few MB of latency
     const int stride = blockDim.x * gridDim.y;
+    const bool table16 = ((reinterpret_cast<uintptr_t>(p.cos_t) | reinterpret_cast<uintptr_t>(p.sin_t)) & 15u) == 0;
+    // a chunk's place inside its head, carried from chunk to chunk instead of a remainder per chunk (with the tables read 16
+    // bytes at a time: norm + RoPE quantisation of 256 tokens 15.4 -> 14.8 us)
+    const int head_step = 8 * stride % p.head_dim;
+    int in_head = 8 * (blockIdx.y * blockDim.x + threadIdx.x) % p.head_dim;
     for (int ch0 = blockIdx.y * blockDim.x + threadIdx.x; ch0 < chunks; ch0 += 4 * stride) {
         uint4 raw[4];
 #pragma unroll
@@ -210,13 +215,21 @@ __global__ void __launch_bounds__(1024) rope_quant_kernel(const RopeParams p) {
             if (ch >= chunks) break;                 // uniform over a 16-thread group
             float v[8];
             unpack8(raw[u], v);
-            const int in_head = (8 * ch) % p.head_dim;
             if (in_head >= nope) {
                 const int pair0 = (in_head - nope) >> 1;
+                float cv[4], sv[4];
+                if (table16) {      // (a row of the tables is a multiple of four pairs)
+                    const float4 c4 = *reinterpret_cast<const float4*>(cs + pair0), s4 = *reinterpret_cast<const float4*>(sn + pair0);
+                    cv[0] = c4.x, cv[1] = c4.y, cv[2] = c4.z, cv[3] = c4.w;
+                    sv[0] = s4.x, sv[1] = s4.y, sv[2] = s4.z, sv[3] = s4.w;
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) cv[i] = cs[pair0 + i], sv[i] = sn[pair0 + i];
+                }
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float c = cs[pair0 + i];
-                    const float s = p.inverse ? -sn[pair0 + i] : sn[pair0 + i];
+                    const float c = cv[i];
+                    const float s = p.inverse ? -sv[i] : sv[i];
                     const float re = v[2 * i], im = v[2 * i + 1];
                     // unfused, as a complex multiply in fp32 (no FMA contraction)
                     v[2 * i] = bf16_round(__fsub_rn(__fmul_rn(re, c), __fmul_rn(im, s)));
@@ -229,6 +242,8 @@ __global__ void __launch_bounds__(1024) rope_quant_kernel(const RopeParams p) {
                 quant_store8(v, p.pow2, p.y_fp8 + o,
                              p.y_scales ? p.y_scales + static_cast<int64_t>(t) * (width >> 7) + (ch >> 4) : nullptr,
                              (ch & 15) == 0);
+            in_head += head_step;
+            if (in_head >= p.head_dim) in_head -= p.head_dim;
         }
     }
 }
