@@ -14,7 +14,7 @@
 //  * swap-AB: the UMMA M dimension (128) is a tile of weight rows, the UMMA N dimension is the activation count rounded
 //    up to 16; the activations (a few MB at most) are re-read from L2 for every weight tile (gemm_tc.cuh says why that
 //    is cheap);
-//  * the work split is gemm_tc.cuh's: stream-K, or for few weight tiles the same number of CTAs per tile;
+//  * the work split is gemm_tc.cuh's: stream-K, for few weight tiles with the partial sums added in slices;
 //  * per unit: an elected thread fetches the weight tile (128 x 128 B) and the activation tile, another issues four
 //    tcgen05.mma kind::f8f6f4 into a fresh TMEM stage, and an epilogue warpgroup adds the stage, times the unit's scales,
 //    to its register accumulators.  The scales of a stage, already multiplied (a_s * w_s), are written beside it by a
@@ -25,8 +25,8 @@
 // Measured (CUDA-graph replays, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
 // activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 35.0,
 // 43.9 -> 37.2, 62.7 -> 45.9, 122.5 -> 89.7 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.8; 2112 x 7168 at 1 / 64 rows
-// 12.3 -> 10.3, 15.3 -> 10.3; 4096 x 7168 at 64 rows 17.8 -> 14.4.  Where the split is stream-K (more than a third of the SMs hold tiles) the results are
-// bit-identical to those of the earlier form: the order of the additions is the same.
+// 12.3 -> 10.3, 15.3 -> 10.3; 4096 x 7168 at 64 rows 17.8 -> 14.4.  The results are bit-identical
+// to those of the earlier form: the order of the additions is the same.
 // Every wait is bounded and reports through the status word.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -42,14 +42,17 @@
 namespace wuda {
 namespace gemm8 {
 
-using gemmtc::arrive_and_wait;
 using gemmtc::await_word;
 using gemmtc::cta_of;
+using gemmtc::holders_of;
+using gemmtc::inc_acq_rel_gpu;
+using gemmtc::unpack_holders;
 using gemmtc::kRowBytes;
 using gemmtc::kTileN;
 using gemmtc::kWBytes;
 using gemmtc::ld_acquire_gpu;
 using gemmtc::range_begin;
+using gemmtc::slot_index;
 using gemmtc::st_release_gpu;
 
 constexpr int kFirstEpiWarp = 4;     // warp 0 copies, 1 issues MMAs, 2 prepares scales, 3 awaits partials, 4..11 are two epilogue warpgroups
@@ -62,14 +65,14 @@ struct Params {
     const float* a_scales;     // [M, a_kb_total]
     const float* w_scales;     // [ceil(N/128), K/128]
     __nv_bfloat16* c;          // [M, N]
-    float* scratch;            // [grid] partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]
-    int32_t* flags;            // stream-K: one flag per CTA; split: one counter per weight tile; zero between calls
+    float* scratch;            // partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]: [grid], sliced also [n_tiles]
+    int32_t* flags;            // one flag per CTA; sliced: one counter per weight tile; zero between calls
     int32_t* status;
     int M, N, K, kb;           // kb = K / 128
     int n_tiles;
     int a_rows;                // M rounded up to 16
     int stages;
-    int split;                 // CTAs per weight tile, 0 = stream-K
+    int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each
     int vec_scales;            // rows of a_scales can be read 16 bytes at a time
     // grouped form: weight tile t belongs to group t / group_tiles and reads the activations'
     // columns [group * K, (group + 1) * K); a_kb_total = K blocks in an activation row
@@ -162,22 +165,13 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         tmem_relinquish();
     }
     const long long units = static_cast<long long>(p.n_tiles) * p.kb;
-    long long u0;
-    int count;
-    if (p.split > 0) {
-        const int tile = static_cast<int>(blockIdx.x) / p.split, j = static_cast<int>(blockIdx.x) - tile * p.split;
-        const int k0 = p.kb * j / p.split;
-        u0 = static_cast<long long>(tile) * p.kb + k0;
-        count = p.kb * (j + 1) / p.split - k0;
-    } else {
-        u0 = range_begin(units, blockIdx.x, gridDim.x);
-        count = static_cast<int>(range_begin(units, blockIdx.x + 1, gridDim.x) - u0);
-    }
+    const long long u0 = range_begin(units, blockIdx.x, gridDim.x);
+    const int count = static_cast<int>(range_begin(units, blockIdx.x + 1, gridDim.x) - u0);
     const int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
     // The last tile of a stream-K range may go on in the following CTAs (all resident: the grid is one CTA per SM).  If this
     // CTA holds its start, it adds their partials, of CTAs blockIdx.x + 1 .. last_peer, in CTA order.
     const long long last_tile = static_cast<uint32_t>(u0 + count - 1) / static_cast<uint32_t>(p.kb);
-    const bool shares = p.split == 0 && last_tile * p.kb >= u0 && (last_tile + 1) * p.kb > u0 + count;
+    const bool shares = !p.sliced && last_tile * p.kb >= u0 && (last_tile + 1) * p.kb > u0 + count;
     if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
@@ -336,6 +330,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         int tile = tile0, kb = kb0;
         int seg_kb0 = kb;                               // first K block of the running segment
         constexpr int64_t kSlotFloats = static_cast<int64_t>(M_PAD) * kTileN;
+        int seg = 0;
+        uint32_t held = 0;                              // sliced: who shares the first and the second tile of this range
+        if (p.sliced) {
+            held = holders_of(units, tile0, p.kb, gridDim.x);
+            if (last_tile != tile0) held |= holders_of(units, tile0 + 1, p.kb, gridDim.x) << 16;
+        }
 
         // An aborting CTA keeps walking the loop (every wait then fails at once) so that all
         // 256 epilogue threads reach every named barrier; it only skips the arithmetic.
@@ -407,9 +407,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 const int c0 = half * kHalf;             // this thread finishes columns c0 .. c0 + kHalf - 1
                 const int nrow = tile * kTileN + row_in_tile;
                 const bool from_zero = (seg_kb0 == 0), to_end = (kb + 1 == p.kb);
-                if (p.split > 0 || !from_zero) {
+                if (p.sliced || !from_zero) {
                     // partial sums to this CTA's slot, 16 bytes = four columns of a row
-                    float4* slot = reinterpret_cast<float4*>(p.scratch + static_cast<int64_t>(blockIdx.x) * kSlotFloats) + row_in_tile;
+                    float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced, from_zero, tile) * kSlotFloats) + row_in_tile;
                     if (alive) {
 #pragma unroll
                         for (int i = 0; i < kHalf; i += 4)
@@ -418,14 +418,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                     __threadfence();
                     epi_bar_sync();
                 }
-                if (p.split > 0) {
-                    // every CTA of the tile adds one slice of it over all partials, in K order
-                    int32_t* counter = p.flags + tile;
-                    if (et == 0 && alive) arrive_and_wait(counter, p.split, abort_flag, p.status);
-                    epi_bar_sync();
-                    alive = __all_sync(0xffffffffu, alive && !*abort_flag);
-                    if (alive)
-                        gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile, p.split, et, 32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
+                if (p.sliced) {
+                    // (the last arrival wraps the tile's counter back to zero: gemm_tc.cuh)
+                    if (et == 0 && alive) inc_acq_rel_gpu(p.flags + tile, unpack_holders(held, seg).count() - 1);
                 } else if (!from_zero) {
                     if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
                 } else {
@@ -517,10 +512,22 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
 #pragma unroll
                 for (int i = 0; i < kCols; ++i) acc[i] = 0.f;
                 seg_kb0 = 0;
+                ++seg;
             }
             if (++kb == p.kb) {
                 kb = 0;
                 ++tile;
+            }
+        }
+        if (p.sliced) {
+#pragma unroll 1
+            for (int i = 0; i < seg; ++i) {
+                if (et == 0 && alive) await_word(p.flags + tile0 + i, [](int v) { return v == 0; }, abort_flag, p.status);
+                epi_bar_sync();
+                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                if (alive)
+                    gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile0 + i, unpack_holders(held, i), et, 32 * kEpiWarps, p.M, p.N, 1.f, 0,
+                                                          p.c);
             }
         }
     }
@@ -557,12 +564,8 @@ static int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, Params& p,
     WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
     const long long units = static_cast<long long>(p.n_tiles) * p.kb;
     const int sms = gemm_sms(dev);
-    // (the two-rank form needs a finished tile in one CTA; the owner of a tile then adds at most kMaxSplit partials)
-    constexpr int kMaxSplit = M_PAD <= 16 ? 16 : (M_PAD == 32 ? 12 : (M_PAD == 64 ? 8 : 6));
-    p.split = p.tp_peer_inbox ? 0 : gemmtc::tile_split(p.n_tiles, p.kb, sms);
-    int grid = units < sms ? static_cast<int>(units) : sms;
-    if (p.split > 0) grid = p.n_tiles * p.split;
-    else if (static_cast<long long>(p.n_tiles) * kMaxSplit < grid) grid = p.n_tiles * kMaxSplit;
+    const int grid = gemmtc::grid_of(units, p.n_tiles, M_PAD, sms);
+    p.sliced = !p.tp_peer_inbox && gemmtc::slice_wise(grid, p.n_tiles);     // (the two-rank form needs a finished tile in one CTA)
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem, stream, w_map, a_map, p));
     return WUDA_OK;
 }
@@ -643,7 +646,7 @@ int gemm_fp8_setup_and_launch(const GemmCall& g) {
     p.a_kb_total = g.groups * (g.k / 128);
     p.a_rows = gemmtc::rows_of(g.m);
     p.vec_scales = p.kb % 4 == 0 && aligned16(g.a_scales);
-    p.split = 0;
+    p.sliced = 0;
     p.scratch = g.slots;
     p.flags = g.flags;
     p.stages = 0;

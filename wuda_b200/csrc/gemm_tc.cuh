@@ -17,12 +17,14 @@
 //   * block scales of the FP8 / 4-bit kinds are exponent bytes in tensor memory.  A 32-bit scale column holds four
 //     consecutive K blocks (the MMA's scale id picks one), so two warps build ONE image per four units, from scales
 //     they requested sixteen units earlier; the fetching and the issuing thread never wait for scale arithmetic.
-//   * work split.  Weight tiles enough for every SM: stream-K, i.e. the flat unit list in equal contiguous ranges; a
-//     range that starts inside a tile leaves its partial sums in its scratch slot and the CTA with the tile's start
-//     adds them in CTA order - it comes to that tile last, the partial was finished first.  Few tiles ("split"): the
-//     same number of CTAs for every tile, each with one K range; all leave their partial sums, and once the tile's
-//     counter is complete each CTA adds one slice of the tile over all partials, in order - instead of one CTA adding
-//     seven or more whole partials one after the other.  Both orders are fixed: results do not depend on timing.
+//   * work split: stream-K, i.e. the flat unit list in equal contiguous ranges, at most max_split() of them to a tile.
+//     Tiles enough for every SM: a range that starts inside a tile leaves its partial sums in its scratch slot and the
+//     CTA with the tile's start adds them in CTA order - it comes to that tile last, the partial was finished first.
+//     Few tiles ("sliced"): every CTA leaves the partial sums of its one or two tiles, and once a tile's counter is
+//     complete each of its CTAs adds one slice of it over all partials - instead of one CTA adding up to fifteen whole
+//     partials one after the other.  The order of the additions is CTA order either way and part of the results (it
+//     moves single roundings of the fp32 sums, and 4-bit quantisation behind them makes 4e-3 of a layer's output of
+//     that): it depends on the shape and the SM count alone, not on timing.
 //   * before it waits for the kernel ahead (programmatic launch) a CTA asks L2 for its first weight tiles, so a chain
 //     of small kernels hides the start of the weight stream.  A prefetch into L2 is a hint: it reads nothing into the
 //     SM, so weights written by an earlier kernel of the chain are still seen.
@@ -52,19 +54,18 @@ constexpr int kImgSlots = 4;
 constexpr int kImgBlock = 512;                // scale bytes of 128 rows, four bytes each: [row % 32][row / 32]
 constexpr int kNvSfBytes = 2048;              // NVFP4: packed scales of 128 rows x 256 K
 constexpr int kMaxGrid = 192;
-constexpr int kMaxTileSplit = 32;
 constexpr int64_t kFlagBytes = 1024;          // the flags lead the scratch, whatever the shape (kernels share scratches)
 
 struct Params {
     void* c;
     int c_is_fp32;
-    float* scratch;            // [grid] partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]
-    int32_t* flags;            // stream-K: one flag per CTA; split: one counter per weight tile
+    float* scratch;            // partial-tile slots, fp32 [M_PAD / 4][128 weight rows][4 activation rows]: [grid], sliced also [n_tiles]
+    int32_t* flags;            // one flag per CTA; sliced: one counter per weight tile
     int32_t* status;
     int M, N, kb, n_tiles;     // kb = units per weight tile
     int a_rows;                // M rounded up to 16
     int stages;
-    int split;                 // CTAs per weight tile, 0 = stream-K
+    int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each
     // power-of-two scaled kinds
     const float* a_scales;     // [M, scale_cols]
     const float* w_scales;     // [n_tiles, kb] (FP8 weights)
@@ -85,10 +86,10 @@ template <Kind KIND, int M_PAD>
 struct Layout {
     static constexpr bool kMx = KIND == Kind::kMx8 || KIND == Kind::kMx8W4;
     static constexpr int kBlocks = (M_PAD + 127) / 128;               // 128-row blocks of activation scales
-    // FP8 x FP8 up to 128 rows keeps two sums, of the even and of the odd units of a range, added at the end.  The order of
-    // the additions is part of the layer's results: another order moves single bf16 roundings of the projections, and the
-    // 4-bit activations of the experts behind them turn those into 1e-2 of the layer's output.
-    static constexpr int kAccs = KIND == Kind::kMx8 && M_PAD <= 128 ? 2 : 1;
+    // FP8 x FP8 and BF16 up to 128 rows keep two sums, of the even and of the odd units of a range, added at the end.  The
+    // order of the additions is part of the layer's results: another order moves single roundings of the projections, and
+    // the 4-bit activations of the experts behind them turn those into 4e-3 of the layer's output.
+    static constexpr int kAccs = (KIND == Kind::kMx8 || KIND == Kind::kBf16) && M_PAD <= 128 ? 2 : 1;
     static constexpr int kBuffers = kAccs * M_PAD <= 128 ? 2 : 1;
     // Epilogue warps: behind the last copy they move partial sums and results with the bytes in flight that they have, so
     // 256 rows take sixteen (7168 x 16384 FP8 43.8 -> 40.4 us; not with 4-bit weights, whose scale images need the
@@ -198,31 +199,43 @@ __device__ __forceinline__ void await_word(const int32_t* word, Pred done, volat
     }
 }
 
-// One thread's arrival at the counter of a tile that `split` CTAs share, and its wait for the others.  The last arrival wraps
-// the counter back to zero, which is what the others wait for: nobody has to reset it (as a second, departing atomic did,
-// 0.5 us behind the results).  No CTA arrives at a counter twice in a launch, and the next launch's arrive after this one.
-__device__ __forceinline__ void arrive_and_wait(int32_t* counter, int split, volatile int* abort_flag, int32_t* status) {
-    if (inc_acq_rel_gpu(counter, split - 1) != split - 1)
-        await_word(counter, [](int v) { return v == 0; }, abort_flag, status);
+// The CTAs that hold units of a sliced tile.  A CTA has at most two tiles: its range is at most a third of one.
+struct Holders {
+    int first, last;
+    __device__ __forceinline__ int count() const { return last - first + 1; }
+};
+// .. as one word (there are fewer than 256 CTAs): two tiles' stay in registers until the end of a range
+__device__ __forceinline__ uint32_t holders_of(long long units, int tile, int kb, int grid) {
+    const long long begin = static_cast<long long>(tile) * kb;
+    return static_cast<uint32_t>(cta_of(units, begin, grid)) | static_cast<uint32_t>(cta_of(units, begin + kb - 1, grid)) << 8;
+}
+__device__ __forceinline__ Holders unpack_holders(uint32_t both, int i) {
+    return {static_cast<int>(both >> (16 * i) & 0xffu), static_cast<int>(both >> (16 * i + 8) & 0xffu)};
+}
+// Slot of this CTA's partial sums: the one that starts a sliced tile goes behind the CTAs' own (its CTA may hold the end
+// of the tile before, too).
+__device__ __forceinline__ int slot_index(int sliced, bool from_zero, int tile) {
+    return sliced && from_zero ? static_cast<int>(gridDim.x) + tile : static_cast<int>(blockIdx.x);
 }
 
-// This CTA's slice of a weight tile shared by `split` CTAs: the sum over all partials, in K order, scaled and stored.
+// This CTA's slice of a weight tile: the sum over all partials, in CTA order, scaled and stored.
 // A thread adds four activation rows of a weight row, eight partials in flight.
 template <Kind KIND>
-__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, int split, int thread, int threads, int M,
+__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, Holders h, int thread, int threads, int M,
                                           int N, float out_scale, int c_is_fp32, void* c) {
-    const int j = static_cast<int>(blockIdx.x) - tile * split, quads = (M + 3) / 4 * kTileN;
-    const float4* part = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(tile) * split * slot_floats);
-    const int end = quads * (j + 1) / split;
-    for (int e = quads * j / split + thread; e < end; e += threads) {
-        float4 v = __ldcg(part + e);
-        for (int q0 = 1; q0 < split; q0 += 8) {
+    const int j = static_cast<int>(blockIdx.x) - h.first, parts = h.count(), quads = (M + 3) / 4 * kTileN;
+    const float4* start = reinterpret_cast<const float4*>(scratch + (static_cast<int64_t>(gridDim.x) + tile) * slot_floats);
+    const float4* part = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(h.first) * slot_floats);   // [1], [2], ..
+    const int end = quads * (j + 1) / parts;
+    for (int e = quads * j / parts + thread; e < end; e += threads) {
+        float4 v = __ldcg(start + e);
+        for (int q0 = 1; q0 < parts; q0 += 8) {
             float4 x[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) x[q] = __ldcg(part + min(q0 + q, split - 1) * (slot_floats / 4) + e);
+            for (int q = 0; q < 8; ++q) x[q] = __ldcg(part + min(q0 + q, parts - 1) * (slot_floats / 4) + e);
 #pragma unroll
             for (int q = 0; q < 8; ++q)
-                if (q0 + q < split) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
+                if (q0 + q < parts) v.x += x[q].x, v.y += x[q].y, v.z += x[q].z, v.w += x[q].w;
         }
         const float out[4] = {v.x, v.y, v.z, v.w};
         const int m = e / kTileN * 4, nr = tile * kTileN + e % kTileN;
@@ -286,15 +299,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     long long units = static_cast<long long>(p.n_tiles) * p.kb, u0 = 0;
     int grid = static_cast<int>(gridDim.x), count = 0;
     if (!grouped) {
-        if (p.split > 0) {
-            const int tile = static_cast<int>(blockIdx.x) / p.split, j = static_cast<int>(blockIdx.x) - tile * p.split;
-            const int k0 = p.kb * j / p.split;
-            u0 = static_cast<long long>(tile) * p.kb + k0;
-            count = p.kb * (j + 1) / p.split - k0;
-        } else {
-            u0 = range_begin(units, blockIdx.x, grid);
-            count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
-        }
+        u0 = range_begin(units, blockIdx.x, grid);
+        count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
     }
     int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
     if (warp == 0 && elect_one()) {
@@ -594,6 +600,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         int grp = 0, seen_grp = -1;
         float scale = p.out_scale;
         uint32_t stored = 0xffffffffu;       // grouped rows without a token are padding: nobody reads them
+        // sliced: who shares the first and the second tile of this range (found out beside the stream, except by the 256-row
+        // form, which has no register left to keep it)
+        constexpr bool kKeep = M_PAD < 256;
+        uint32_t held = 0;
+        auto holders = [&](int i) {
+            return unpack_holders(kKeep ? held : holders_of(units, tile0 + i, p.kb, grid) << (16 * i), i);
+        };
         for (int n = 0; n < count;) {
             // the segment [kb, kb_end) of `tile`
             const int seg_len = min(p.kb - kb, count - n);
@@ -615,13 +628,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             // The start of a tile whose K range goes on in the following CTAs (all resident: the grid is one CTA per SM): their
             // partials were finished first, so the flags are awaited (each by a thread of its own) and the first partial
             // is fetched while this segment's MMAs still run.
-            const bool owner = p.split == 0 && from_zero && !to_end;
-            constexpr bool kAhead = kCols <= 32 || (M_PAD == 128 && !kMx);      // (what the registers hold without spills)
+            const bool owner = !p.sliced && from_zero && !to_end;
+            constexpr bool kAhead = kCols <= 32 || (M_PAD == 128 && KIND == Kind::kNv4);   // (what the registers hold without spills)
             float4 ahead[kAhead ? kCols / 4 : 1];
             int last = blockIdx.x;
             auto slot_of = [&](int c) {
                 return reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * slot_floats) + col0 / 4 * kTileN + row;
             };
+            if (kKeep && p.sliced) held |= holders_of(units, tile, p.kb, grid) << (16 * seg);
             if (owner) {
                 last = cta_of(units, static_cast<long long>(tile + 1) * p.kb - 1, grid);
                 for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
@@ -664,8 +678,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (lane == 0) mbar_arrive(empty_tm + buf * 8);
 
             const int nrow0 = (tile - grp * p.n_tiles) * kTileN;
-            if (!(from_zero && to_end) && (p.split > 0 || !from_zero)) {   // partial sums to this CTA's slot
-                float4* slot = reinterpret_cast<float4*>(p.scratch + static_cast<int64_t>(blockIdx.x) * slot_floats) + row;
+            if (p.sliced || !from_zero) {   // partial sums to this CTA's slot
+                float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced, from_zero, tile) * slot_floats) + row;
                 if (alive) {
 #pragma unroll
                     for (int c = 0; c < kCols; c += 4)
@@ -674,14 +688,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 __threadfence();
                 epi_sync();
             }
-            if (p.split > 0) {
-                // every CTA of the tile adds one slice of it over all partials, in K order
-                int32_t* counter = p.flags + tile;
-                if (et == 0 && alive) arrive_and_wait(counter, p.split, abort_flag, p.status);
-                epi_sync();
-                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
-                if (alive)
-                    add_slice<KIND>(p.scratch, slot_floats, tile, p.split, et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32, p.c);
+            if (p.sliced) {
+                // The last arrival wraps the tile's counter back to zero, which is what the others wait for, once they have
+                // nothing else to do.  No CTA arrives at a counter twice in a launch, the next launch's arrive after this one.
+                if (et == 0 && alive) inc_acq_rel_gpu(p.flags + tile, holders(seg).count() - 1);
             } else if (!from_zero) {
                 if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
             } else {
@@ -747,6 +757,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (kb == p.kb) kb = 0, ++tile;
             ++seg;
         }
+        if (p.sliced) {
+#pragma unroll 1
+            for (uint32_t i = 0; i < seg; ++i) {
+                if (et == 0 && alive) await_word(p.flags + tile0 + i, [](int v) { return v == 0; }, abort_flag, p.status);
+                epi_sync();
+                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                if (alive)
+                    add_slice<KIND>(p.scratch, slot_floats, tile0 + static_cast<int>(i), holders(i), et, kEpi, p.M, p.N, p.out_scale,
+                                    p.c_is_fp32, p.c);
+            }
+        }
     }
 
     __syncthreads();
@@ -758,14 +779,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     }
 }
 
-// CTAs per weight tile: as many as the SMs hold when that is at least three (one CTA adding up to six whole partials at
-// the end costs more than the SMs that the division leaves idle), none (stream-K) otherwise.
-inline int tile_split(int n_tiles, int kb, int sms) {
-    int split = sms / n_tiles;
-    if (split > kb) split = kb;
-    if (split > kMaxTileSplit) split = kMaxTileSplit;
-    return split >= 3 ? split : 0;
+// Ranges that share a weight tile at most (adding partial sums costs as much as streaming M_PAD / 64 units of weights, so wide
+// tiles are cut into fewer).
+constexpr int max_split(int m_pad) { return m_pad <= 16 ? 16 : (m_pad == 32 ? 12 : (m_pad == 64 ? 8 : 6)); }
+inline int grid_of(long long units, int n_tiles, int m_pad, int sms) {
+    int grid = units < sms ? static_cast<int>(units) : sms;
+    if (static_cast<long long>(n_tiles) * max_split(m_pad) < grid) grid = n_tiles * max_split(m_pad);
+    return grid;
 }
+// Added in slices where every tile is cut into three ranges or more (and the slots suffice: one per CTA and one per tile).
+inline bool slice_wise(int grid, int n_tiles) { return grid >= 3 * n_tiles && grid + n_tiles <= kMaxGrid; }
 
 template <Kind KIND, int M_PAD>
 int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap& wsf_map, const CUtensorMap& asf_map, Params& p,
@@ -779,12 +802,9 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap
     auto kernel = gemm_tc_kernel<KIND, M_PAD>;
     WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(stages, p.a_rows)));
     const int sms = gemm_sms(dev);
-    const long long units = static_cast<long long>(p.n_tiles) * p.kb;
     // (grouped: the number of groups is only known on the device; one CTA per SM, idle ones return at once)
-    p.split = p.group_expert ? 0 : tile_split(p.n_tiles, p.kb, sms);
-    int grid = sms;
-    if (p.split > 0) grid = p.n_tiles * p.split;
-    else if (!p.group_expert && units < sms) grid = static_cast<int>(units);
+    const int grid = p.group_expert ? sms : grid_of(static_cast<long long>(p.n_tiles) * p.kb, p.n_tiles, M_PAD, sms);
+    p.sliced = !p.group_expert && slice_wise(grid, p.n_tiles);
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(L::kThreads), L::total(stages, p.a_rows), stream, w_map, a_map, wsf_map, asf_map, p));
     return WUDA_OK;
 }
