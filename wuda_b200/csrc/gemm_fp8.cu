@@ -236,7 +236,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         // ------------------------------------------------------------ scale products
         // In groups of four K blocks of a tile (aligned to four, cut at the ends of the range).  A lane holds the scales of
         // rows lane, lane + 32, ..; two groups are in registers, each refilled when it has been written out.  (One warp: it
-        // sees every phase of the barriers it waits on.)
+        // sees every phase of the barriers it waits on.)  All through L2: gemm_tc.cuh says why.
         constexpr int kQ = (M_PAD + 31) / 32;
         int tile = tile0, kb = kb0, n = 0;
         struct Raw {
@@ -265,10 +265,10 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                     }
                 }
                 const float* src = p.w_scales + static_cast<int64_t>(tile) * p.kb + k0;
-                r.w.x = __ldg(src);
-                r.w.y = k0 + 1 < p.kb ? __ldg(src + 1) : 0.f;
-                r.w.z = k0 + 2 < p.kb ? __ldg(src + 2) : 0.f;
-                r.w.w = k0 + 3 < p.kb ? __ldg(src + 3) : 0.f;
+                r.w.x = __ldcg(src);
+                r.w.y = k0 + 1 < p.kb ? __ldcg(src + 1) : 0.f;
+                r.w.z = k0 + 2 < p.kb ? __ldcg(src + 2) : 0.f;
+                r.w.w = k0 + 3 < p.kb ? __ldcg(src + 3) : 0.f;
                 const int len = group_len();
                 n += len, kb += len;
                 if (kb == p.kb) kb = 0, ++tile;

@@ -489,6 +489,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 float4 w;               // FP8 weights: the four K blocks' scales
                 uint4 wsf[4];           // 4-bit weights: rows lane + 32 q, four words of four exponent bytes
             };
+            // (through L2, the weights' scales too: this kernel may be resident while the one ahead still writes them, and the
+            // read-only path may then serve lines that an earlier kernel of the chain left in L1)
             auto load = [&](Raw& r) {
                 const int k0 = kb & ~3;
                 const int col = (tile / p.tiles_per_group) * p.kb + k0;
@@ -510,10 +512,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 }
                 if constexpr (KIND == Kind::kMx8) {
                     const float* src = p.w_scales + static_cast<int64_t>(tile) * p.kb + k0;
-                    r.w.x = __ldg(src);
-                    r.w.y = k0 + 1 < p.kb ? __ldg(src + 1) : 1.f;
-                    r.w.z = k0 + 2 < p.kb ? __ldg(src + 2) : 1.f;
-                    r.w.w = k0 + 3 < p.kb ? __ldg(src + 3) : 1.f;
+                    r.w.x = __ldcg(src);
+                    r.w.y = k0 + 1 < p.kb ? __ldcg(src + 1) : 1.f;
+                    r.w.z = k0 + 2 < p.kb ? __ldcg(src + 2) : 1.f;
+                    r.w.w = k0 + 3 < p.kb ? __ldcg(src + 3) : 1.f;
                 } else {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -522,13 +524,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                         if (row < p.N) {
                             const uint8_t* src = p.w_sf + static_cast<int64_t>(row) * p.sf_stride + k0 * 4;
                             if (p.vec_scales) {
-                                r.wsf[q] = __ldg(reinterpret_cast<const uint4*>(src));
+                                r.wsf[q] = __ldcg(reinterpret_cast<const uint4*>(src));
                             } else {
                                 const uint32_t* words = reinterpret_cast<const uint32_t*>(src);
-                                r.wsf[q].x = __ldg(words);
-                                if (k0 + 1 < p.kb) r.wsf[q].y = __ldg(words + 1);
-                                if (k0 + 2 < p.kb) r.wsf[q].z = __ldg(words + 2);
-                                if (k0 + 3 < p.kb) r.wsf[q].w = __ldg(words + 3);
+                                r.wsf[q].x = __ldcg(words);
+                                if (k0 + 1 < p.kb) r.wsf[q].y = __ldcg(words + 1);
+                                if (k0 + 2 < p.kb) r.wsf[q].z = __ldcg(words + 2);
+                                if (k0 + 3 < p.kb) r.wsf[q].w = __ldcg(words + 3);
                             }
                         }
                     }
@@ -618,7 +620,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 if (grouped) grp = tile / p.n_tiles;
                 if (grouped && grp != seen_grp) {
                     seen_grp = grp;
-                    scale = p.out_scale * __ldg(p.expert_scale + __ldcg(p.group_expert + grp));
+                    scale = p.out_scale * __ldcg(p.expert_scale + __ldcg(p.group_expert + grp));
                     if (p.row_token) {
                         const int tok = lane < M_PAD ? __ldcg(p.row_token + grp * M_PAD + lane) : -1;
                         stored = __ballot_sync(0xffffffffu, tok >= 0);
