@@ -802,7 +802,8 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap
         return fail(WUDA_ERR_UNSUPPORTED, "device offers %d bytes of shared memory per block; the kernel needs more", dev.smem_optin);
     p.stages = stages;
     auto kernel = gemm_tc_kernel<KIND, M_PAD>;
-    WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total(stages, p.a_rows)));
+    // (the same limit whatever the rows and stages: it is the kernel's, and another thread may set it before this launch)
+    WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
     const int sms = gemm_sms(dev);
     // (grouped: the number of groups is only known on the device; one CTA per SM, idle ones return at once)
     const int grid = p.group_expert ? sms : grid_of(static_cast<long long>(p.n_tiles) * p.kb, p.n_tiles, M_PAD, sms);
