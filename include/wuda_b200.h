@@ -677,6 +677,13 @@ int wuda_swiglu_quant_fp8(const void* h_bf16, void* y_bf16, void* y_fp8, float* 
  * room for anything beside it).  The number of CTAs decides how a weight tile's K range is cut and therefore the
  * order of the fp32 additions: results are reproducible for a given setting, not across settings. */
 int wuda_gemm_sm_limit(int max_sms);
+/* The GEMM launches the CALLING THREAD makes from now on keep their flags in these 1024 bytes (256-byte aligned, zero before
+ * the first call, zero again after each) instead of the first 1024 bytes of their scratch; NULL: in the scratch again.
+ * Returns the previous setting.  For hosts that capture GEMMs into CUDA graphs: the flags are all of a scratch that must
+ * stay as a call left it until the next, so with them elsewhere the scratch itself can be a temporary of the capture. */
+void* wuda_gemm_flags(void* flags);
+/* *id = the number of the capture that `stream` takes part in (unique in the process), 0 if there is none. */
+int wuda_capture_id(void* stream, unsigned long long* id);
 int64_t wuda_gemm_fp8_scratch_bytes(int m, int n);
 int wuda_gemm_fp8_blockscaled(const void* a, const float* a_scales, const void* w, const float* w_scales,
                               void* c_bf16, int m, int n, int k, void* scratch, int64_t scratch_bytes,

@@ -49,7 +49,7 @@ extern "C" int wuda_gemm_bf16(const void* a_bf16, const void* w_bf16, void* c, i
     p.n_tiles = (n + 127) / 128;
     p.a_rows = rows_of(m);
     p.scratch = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
-    p.flags = static_cast<int32_t*>(scratch);
+    p.flags = gemm_flags(scratch);
 
     CUtensorMap w_map, a_map;
     {

@@ -720,7 +720,7 @@ int gemm_fp8_entry(const void* a, const float* a_scales, const void* w, const fl
     GemmCall g;
     g.a = a, g.a_scales = a_scales, g.w = w, g.w_scales = w_scales, g.c = c_bf16;
     g.m = m, g.n = n, g.k = k, g.groups = groups;
-    g.flags = static_cast<int32_t*>(scratch);
+    g.flags = gemm_flags(scratch);
     g.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
     g.status = status_word;
     g.stream = static_cast<cudaStream_t>(stream);
@@ -910,7 +910,7 @@ extern "C" int wuda_gemm_fp8_blockscaled_tp2(const void* a, const float* a_scale
     GemmCall g;
     g.a = a, g.a_scales = a_scales, g.w = w, g.w_scales = w_scales, g.c = c_bf16;
     g.m = m, g.n = n, g.k = k_local;
-    g.flags = static_cast<int32_t*>(scratch);
+    g.flags = gemm_flags(scratch);
     g.slots = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
     g.status = status_word;
     g.stream = static_cast<cudaStream_t>(stream);

@@ -67,7 +67,7 @@ static int run(const void* a, const float* a_scales, const void* w, const float*
     p.scale_cols = groups * p.kb;
     p.vec_scales = p.kb % 4 == 0 && aligned16(a_scales) && (!w4 || aligned16(w_sf));
     p.scratch = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
-    p.flags = static_cast<int32_t*>(scratch);
+    p.flags = gemm_flags(scratch);
 
     CUtensorMap w_map, a_map;
     {

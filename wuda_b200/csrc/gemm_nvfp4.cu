@@ -75,7 +75,7 @@ extern "C" int wuda_gemm_nvfp4(const void* a, const void* a_sf_packed, float a_g
     p.n_tiles = (n + 127) / 128;
     p.a_rows = rows_of(m);
     p.scratch = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
-    p.flags = static_cast<int32_t*>(scratch);
+    p.flags = gemm_flags(scratch);
 
     CUtensorMap w_map, a_map, wsf_map, asf_map;
     const uint64_t row_bytes = static_cast<uint64_t>(k) / 2;
@@ -152,7 +152,7 @@ extern "C" int wuda_gemm_nvfp4_grouped(const void* a, const void* a_sf_packed, f
     p.n_tiles = n / 128;
     p.a_rows = m_pad;
     p.scratch = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + kFlagBytes);
-    p.flags = static_cast<int32_t*>(scratch);
+    p.flags = gemm_flags(scratch);
     p.group_expert = group_expert;
     p.num_groups = num_groups;
     p.row_token = row_token;

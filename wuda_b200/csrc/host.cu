@@ -22,6 +22,9 @@ int gemm_sms(const DeviceInfo& dev) {
     return g_gemm_sm_limit > 0 && g_gemm_sm_limit < dev.num_sms ? g_gemm_sm_limit : dev.num_sms;
 }
 
+static thread_local int32_t* g_gemm_flags = nullptr;
+int32_t* gemm_flags(void* scratch) { return g_gemm_flags ? g_gemm_flags : static_cast<int32_t*>(scratch); }
+
 int current_device_info(DeviceInfo* out) {
     static std::mutex mu;
     static DeviceInfo cache[64];
@@ -106,6 +109,23 @@ int wuda_num_sms(void) {
 }
 
 }  // extern "C"
+
+extern "C" void* wuda_gemm_flags(void* flags) {
+    void* before = wuda::g_gemm_flags;
+    wuda::g_gemm_flags = static_cast<int32_t*>(flags);
+    return before;
+}
+
+extern "C" int wuda_capture_id(void* stream, unsigned long long* id) {
+    using namespace wuda;
+    clear_error();
+    WUDA_REQUIRE(id, "id must not be NULL");
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long got = 0;
+    WUDA_CUDA(cudaStreamGetCaptureInfo_v2(static_cast<cudaStream_t>(stream), &status, &got, nullptr, nullptr, nullptr));
+    *id = status == cudaStreamCaptureStatusActive ? got : 0;
+    return WUDA_OK;
+}
 
 extern "C" int wuda_gemm_sm_limit(int max_sms) {
     const int before = wuda::g_gemm_sm_limit;

@@ -39,6 +39,8 @@ struct DeviceInfo {
 int current_device_info(DeviceInfo* out);
 // SMs the GEMM launches of the calling thread may cover: all of the device's, or fewer after wuda_gemm_sm_limit
 int gemm_sms(const DeviceInfo& dev);
+// Where those launches find their flags: at the front of the scratch, or where wuda_gemm_flags said
+int32_t* gemm_flags(void* scratch);
 
 // rank-`rank` tiled tensor map. dims/box are innermost-first; strides_bytes has rank-1
 // entries (stride of dims 1..rank-1). Returns a wuda_status.

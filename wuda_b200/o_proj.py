@@ -14,7 +14,7 @@ from dataclasses import dataclass
 import torch
 
 from . import ops
-from ._lib import check, lib
+from ._lib import lib
 
 HEAD_DIM, ROPE_DIM, O_LORA_RANK = 512, 64, 1024
 
@@ -65,11 +65,9 @@ def fp8_gemm_grouped(a, a_s, w, w_s, *, out=None, status_word=None, pow2_scales=
     if out is None:
         out = torch.empty(m, groups * n, dtype=torch.bfloat16, device=a.device)
     need = lib.wuda_gemm_fp8_scratch_bytes(m, groups * n)
-    scratch = ops._scratch_for(a.device, need)
-    entry = lib.wuda_gemm_fp8_grouped_pow2 if pow2_scales else lib.wuda_gemm_fp8_grouped
-    check(entry(a.data_ptr(), a_s.data_ptr(), w.data_ptr(), w_s.data_ptr(), out.data_ptr(), m, n, k, groups, scratch.data_ptr(),
-                scratch.numel(), status_word.data_ptr() if status_word is not None else None,
-                torch.cuda.current_stream().cuda_stream))
+    ops._launch_gemm(lib.wuda_gemm_fp8_grouped_pow2 if pow2_scales else lib.wuda_gemm_fp8_grouped, a.device, need,
+                     (a.data_ptr(), a_s.data_ptr(), w.data_ptr(), w_s.data_ptr(), out.data_ptr(), m, n, k, groups),
+                     ops._ptr(status_word))
     return out
 
 

@@ -7,11 +7,13 @@ the reference's TORCH_CHECK blocks do and failures raise RuntimeError before any
 launched.  Work is enqueued on torch's current CUDA stream.
 """
 import ctypes
+import functools
 
 import torch
 
 from . import _lib
 from ._lib import WudaError, check, lib
+from .scratch import Scratch
 
 __all__ = ["mqa_logits_fp4_decode_out", "mqa_logits_fp4_decode", "mqa_logits_fp8_decode_out", "fp8_paged_mqa_logits", "topk_v2", "topk_v2_transform",
            "IndexerHostPlan", "sparse_mla_decode", "flash_mla_with_kvcache", "device_status_word", "num_sms", "rmsnorm_quant", "act_quant", "rope_quant",
@@ -357,7 +359,7 @@ def _ptr(t):
     return t.data_ptr() if t is not None else None
 
 
-_mla_workspace = {}   # per device: partial sums of split requests (grown on demand)
+_mla_scratch = Scratch(zeroed=False)   # partial sums of split requests
 
 
 def _model1_pool(cache, name):
@@ -407,15 +409,14 @@ def sparse_mla_decode(q, swa_cache, swa_indices, swa_lengths, cmp_cache=None, cm
     _require(out.is_cuda and out.is_contiguous() and out.dtype == torch.bfloat16 and out.shape == q.shape,
              "out must be contiguous CUDA bf16 shaped like q")
     a.out = out.data_ptr()
+    stream = _stream()
     if split and batch > 0:   # small batches: several CTAs per request, merged by a second launch
         need = lib.wuda_sparse_mla_workspace_bytes(batch, heads, a.swa_capacity + a.cmp_capacity)
         _require(need >= 0, "wuda_sparse_mla_workspace_bytes rejected the shape")
         if need > 0:
-            ws = _mla_workspace.get(q.device)
-            if ws is None or ws.numel() < need:
-                ws = _mla_workspace[q.device] = torch.empty(need, dtype=torch.uint8, device=q.device)
-            a.workspace, a.workspace_bytes = ws.data_ptr(), need
-    check(lib.wuda_sparse_mla_decode(ctypes.byref(a), _ptr(status_word), _stream()))
+            a.workspace, _, _, ws = _mla_scratch.get(q.device, stream, need)
+            a.workspace_bytes = need
+    check(lib.wuda_sparse_mla_decode(ctypes.byref(a), _ptr(status_word), stream))
     return out
 
 
@@ -734,25 +735,34 @@ def fp4_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
     a_sf = _scales_as_fp32(a_s, "a_s")
     if out is None:
         out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-    need = lib.wuda_gemm_fp8_scratch_bytes(m, n)
+    need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
     _require(need >= 0, "m must be in [1, 256]")
-    scratch = _scratch_for(a.device, need)
-    check(lib.wuda_gemm_fp8_fp4_pow2(a.data_ptr(), a_sf.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k,
-                                     scratch.data_ptr(), scratch.numel(),
-                                     status_word.data_ptr() if status_word is not None else None, _stream()))
+    _launch_gemm(lib.wuda_gemm_fp8_fp4_pow2, a.device, need,
+                 (a.data_ptr(), a_sf.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k), _ptr(status_word))
     return out
 
 
-_gemm_scratch = {}
+_gemm_scratch = Scratch(zeroed=True)
 
 
-def _scratch_for(device, nbytes):
-    """A zeroed scratch buffer per device, grown on demand (the GEMM leaves it zero)."""
-    buf = _gemm_scratch.get(device)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _gemm_scratch[device] = buf
-    return buf
+@functools.lru_cache(maxsize=1024)
+def _scratch_bytes(entry, m, n):
+    """What the library asks for these sizes (asking takes longer than finding out whether the stream is being captured)."""
+    return entry(m, n)
+
+
+def _launch_gemm(entry, device, need, operands, *rest):
+    """entry(*operands, scratch, its size, *rest, stream) with a scratch of at least `need` bytes."""
+    stream = _stream()
+    at, nbytes, flags, _hold = _gemm_scratch.get(device, stream, need)
+    if flags is None:
+        check(entry(*operands, at, nbytes, *rest, stream))
+        return
+    before = lib.wuda_gemm_flags(flags)
+    try:
+        check(entry(*operands, at, nbytes, *rest, stream))
+    finally:
+        lib.wuda_gemm_flags(before)
 
 
 def fp8_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word=None, pow2_scales=False):
@@ -776,12 +786,10 @@ def fp8_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
              and tuple(b_s.shape) == ((n + 127) // 128, k // 128), "b_s must be contiguous CUDA fp32 [ceil(N/128), K/128]")
     if out is None:
         out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-    need = lib.wuda_gemm_fp8_scratch_bytes(m, n)
+    need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
     _require(need >= 0, "m must be in [1, 256]")
-    scratch = _scratch_for(a.device, need)
-    entry = lib.wuda_gemm_fp8_blockscaled_pow2 if pow2_scales else lib.wuda_gemm_fp8_blockscaled
-    check(entry(a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k, scratch.data_ptr(),
-                scratch.numel(), status_word.data_ptr() if status_word is not None else None, _stream()))
+    _launch_gemm(lib.wuda_gemm_fp8_blockscaled_pow2 if pow2_scales else lib.wuda_gemm_fp8_blockscaled, a.device, need,
+                 (a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k), _ptr(status_word))
     return out
 
 
@@ -798,11 +806,10 @@ def bf16_gemm(a, w, *, out=None, out_dtype=torch.bfloat16, status_word=None):
         out = a.new_empty((*a.shape[:-1], n), dtype=out_dtype)
     _require(out.is_contiguous() and out.dtype in (torch.bfloat16, torch.float32) and out.numel() == m * n,
              "out must be contiguous bf16 or fp32 [M, N]")
-    need = lib.wuda_gemm_bf16_scratch_bytes(m, n)
+    need = _scratch_bytes(lib.wuda_gemm_bf16_scratch_bytes, m, n)
     _require(need >= 0, "m must be in [1, 128]")
-    scratch = _scratch_for(a.device, need)
-    check(lib.wuda_gemm_bf16(a.data_ptr(), w.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), m, n, k,
-                             scratch.data_ptr(), scratch.numel(), _ptr(status_word), _stream()))
+    _launch_gemm(lib.wuda_gemm_bf16, a.device, need,
+                 (a.data_ptr(), w.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), m, n, k), _ptr(status_word))
     return out
 
 
@@ -935,15 +942,11 @@ class TP2Link:
         _require(m <= self.m and n == self.n, "shape outside what the link was created for")
         if out is None:
             out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-        need = lib.wuda_gemm_fp8_scratch_bytes(m, n)
-        scratch = _scratch_for(a.device, need)
+        need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
         self.epoch += 1
-        check(lib.wuda_gemm_fp8_blockscaled_tp2(a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(),
-                                                out.data_ptr(), m, n, k, scratch.data_ptr(), scratch.numel(),
-                                                self._local, self._peer, 0 if self.device_sequence else self.epoch,
-                                                int(peer_wait_ms),
-                                                status_word.data_ptr() if status_word is not None else None,
-                                                _stream()))
+        _launch_gemm(lib.wuda_gemm_fp8_blockscaled_tp2, a.device, need,
+                     (a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k),
+                     self._local, self._peer, 0 if self.device_sequence else self.epoch, int(peer_wait_ms), _ptr(status_word))
         return out
 
     def close(self):
@@ -979,11 +982,9 @@ def nvfp4_gemm(a, a_sf_packed, a_global_scale, w, w_sf_packed, w_global_scale, *
              and w_sf_packed.numel() == ((n + 127) // 128) * 128 * (k // 16), "w_sf_packed has the wrong size")
     if out is None:
         out = a.new_empty((m, n), dtype=torch.bfloat16)
-    need = lib.wuda_gemm_nvfp4_scratch_bytes(m, n)
+    need = _scratch_bytes(lib.wuda_gemm_nvfp4_scratch_bytes, m, n)
     _require(need >= 0, "m must be in [1, 256]")
-    scratch = _scratch_for(a.device, need)
-    check(lib.wuda_gemm_nvfp4(a.data_ptr(), a_sf_packed.data_ptr(), float(a_global_scale), w.data_ptr(),
-                              w_sf_packed.data_ptr(), float(w_global_scale), out.data_ptr(), m, n, k,
-                              scratch.data_ptr(), scratch.numel(),
-                              status_word.data_ptr() if status_word is not None else None, _stream()))
+    _launch_gemm(lib.wuda_gemm_nvfp4, a.device, need,
+                 (a.data_ptr(), a_sf_packed.data_ptr(), float(a_global_scale), w.data_ptr(), w_sf_packed.data_ptr(),
+                  float(w_global_scale), out.data_ptr(), m, n, k), _ptr(status_word))
     return out
