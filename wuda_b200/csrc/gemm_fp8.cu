@@ -27,7 +27,7 @@
 // 43.9 -> 37.2, 62.7 -> 45.9, 122.5 -> 89.7 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.8; 2112 x 7168 at 1 / 64 rows
 // 12.3 -> 10.3, 15.3 -> 10.3; 4096 x 7168 at 64 rows 17.8 -> 14.4.  The results are bit-identical
 // to those of the earlier form: the order of the additions is the same.
-// Every wait is bounded and reports through the status word.
+// Every wait is bounded and reports through the status word; flags and counters end at zero all the same (gemm_tc.cuh).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -51,6 +51,8 @@ using gemmtc::kRowBytes;
 using gemmtc::kTileN;
 using gemmtc::kWBytes;
 using gemmtc::ld_acquire_gpu;
+using gemmtc::lower_flag;
+using gemmtc::raise_flag;
 using gemmtc::range_begin;
 using gemmtc::slot_index;
 using gemmtc::st_release_gpu;
@@ -382,6 +384,11 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
             // ---- end of a segment: the tile's K range ended, or this CTA's range did
             const bool seg_end = (kb + 1 == p.kb) || (n + 1 == count);
             if (seg_end) {
+                auto poison = [&] {      // after a wait that ran out: whoever adds this to anything gets NaN
+#pragma unroll
+                    for (int i = 0; i < kCols; ++i) acc[i] = __int_as_float(0x7fffffff);
+                };
+                if (!alive) poison();
                 if constexpr (kAlt) {
                     // Each group hands the other the columns that one finishes and adds what it gets
                     // to its own half; the sums land in acc[0, kHalf).  x + y == y + x, so the result
@@ -410,24 +417,22 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 if (p.sliced || !from_zero) {
                     // partial sums to this CTA's slot, 16 bytes = four columns of a row
                     float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced, from_zero, tile) * kSlotFloats) + row_in_tile;
-                    if (alive) {
 #pragma unroll
-                        for (int i = 0; i < kHalf; i += 4)
-                            if (c0 + i < p.M) __stcg(slot + (c0 + i) / 4 * kTileN, make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]));
-                    }
+                    for (int i = 0; i < kHalf; i += 4)
+                        if (c0 + i < p.M) __stcg(slot + (c0 + i) / 4 * kTileN, make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]));
                     __threadfence();
                     epi_bar_sync();
                 }
                 if (p.sliced) {
                     // (the last arrival wraps the tile's counter back to zero: gemm_tc.cuh)
-                    if (et == 0 && alive) inc_acq_rel_gpu(p.flags + tile, unpack_holders(held, seg).count() - 1);
+                    if (et == 0) inc_acq_rel_gpu(p.flags + tile, unpack_holders(held, seg).count() - 1);
                 } else if (!from_zero) {
-                    if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
+                    if (et == 0) raise_flag(p.flags + blockIdx.x);
                 } else {
                     if (!to_end) {
                         if (alive) alive = mbar_wait_warp_fast(partials, 0, abort_flag, p.status, kDevTimeoutPeerFlag);
-                        const int last = *last_peer_slot;      // (an aborting CTA does not use it)
                         alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+                        const int last = alive ? *last_peer_slot : cta_of(units, (last_tile + 1) * p.kb - 1, gridDim.x);
                         if (alive) {
                             for (int c = blockIdx.x + 1; c <= last; ++c) {
                                 const float4* peer = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * kSlotFloats) + row_in_tile;
@@ -446,9 +451,9 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                                     }
                             }
                         }
+                        if (!alive) poison();
                         epi_bar_sync();
-                        if (alive)
-                            for (int c = blockIdx.x + 1 + et; c <= last; c += 32 * kEpiWarps) p.flags[c] = 0;   // free again
+                        for (int c = blockIdx.x + 1 + et; c <= last; c += 32 * kEpiWarps) lower_flag(p.flags + c);   // free again
                     }
                     if (p.tp_peer_inbox) {
                         // Two-rank all-reduce fused into the epilogue: the finished fp32 tile goes
@@ -460,14 +465,12 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                         // peer's reads, never two.
                         const int64_t set = static_cast<int64_t>(tp_epoch & 1) * p.n_tiles;
                         const int64_t tile_off = (set + tile) * (M_PAD * kTileN) + row_in_tile;
-                        if (alive) {
 #pragma unroll
-                            for (int i = 0; i < kHalf; ++i)
-                                p.tp_peer_inbox[tile_off + (c0 + i) * kTileN] = acc[i];
-                        }
+                        for (int i = 0; i < kHalf; ++i)
+                            p.tp_peer_inbox[tile_off + (c0 + i) * kTileN] = acc[i];
                         __threadfence_system();
                         epi_bar_sync();
-                        if (et == 0 && alive) {
+                        if (et == 0 && !*abort_flag) {
                             st_release_sys(p.tp_peer_flags + set + tile, tp_epoch);
                             const unsigned long long start = globaltimer_ns();
                             uint32_t spins = 0;

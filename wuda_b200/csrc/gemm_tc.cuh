@@ -28,7 +28,9 @@
 //   * before it waits for the kernel ahead (programmatic launch) a CTA asks L2 for its first weight tiles, so a chain
 //     of small kernels hides the start of the weight stream.  A prefetch into L2 is a hint: it reads nothing into the
 //     SM, so weights written by an earlier kernel of the chain are still seen.
-// Every wait is bounded.
+// Every wait is bounded.  A CTA whose wait ran out records it, fills its partial sums with NaN and takes every step that
+// other CTAs count on all the same, so that all flags and counters are zero again when the launch ends: the next launch
+// must not take what an aborted one left behind for an arrival of its own.
 #pragma once
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -117,6 +119,16 @@ struct Layout {
     static __host__ __device__ constexpr int total(int stages, int a_rows) { return misc_off(stages, a_rows) + 16 + 1024; }
 };
 
+// A CTA's flag goes up when its partial sums are complete and down when the CTA that adds them has done so.  Both flip it,
+// and both always do: in whichever order (the one that adds may have given up waiting), the flag ends at zero.
+__device__ __forceinline__ void raise_flag(int32_t* flag) {
+    asm volatile("red.release.gpu.global.inc.u32 [%0], %1;" ::"l"(flag), "r"(1) : "memory");
+}
+// (nobody reads it any more in this launch, so nothing has to be ordered: a release would hold up the results behind it, the
+// layer at batch 1 by 3 us)
+__device__ __forceinline__ void lower_flag(int32_t* flag) {
+    asm volatile("red.relaxed.gpu.global.inc.u32 [%0], %1;" ::"l"(flag), "r"(1) : "memory");
+}
 __device__ __forceinline__ void st_release_gpu(int32_t* p, int v) {
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -674,7 +686,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 tc_fence_before();
             } else {
 #pragma unroll
-                for (int i = 0; i < kCols; ++i) acc[i] = 0.f;
+                for (int i = 0; i < kCols; ++i) acc[i] = __int_as_float(0x7fffffff);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(empty_tm + buf * 8);
@@ -682,20 +694,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             const int nrow0 = (tile - grp * p.n_tiles) * kTileN;
             if (p.sliced || !from_zero) {   // partial sums to this CTA's slot
                 float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced, from_zero, tile) * slot_floats) + row;
-                if (alive) {
 #pragma unroll
-                    for (int c = 0; c < kCols; c += 4)
-                        if (col0 + c < p.M) __stcg(slot + (col0 + c) / 4 * kTileN, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
-                }
+                for (int c = 0; c < kCols; c += 4)
+                    if (col0 + c < p.M) __stcg(slot + (col0 + c) / 4 * kTileN, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
                 __threadfence();
                 epi_sync();
             }
             if (p.sliced) {
                 // The last arrival wraps the tile's counter back to zero, which is what the others wait for, once they have
                 // nothing else to do.  No CTA arrives at a counter twice in a launch, the next launch's arrive after this one.
-                if (et == 0 && alive) inc_acq_rel_gpu(p.flags + tile, holders(seg).count() - 1);
+                if (et == 0) inc_acq_rel_gpu(p.flags + tile, holders(seg).count() - 1);
             } else if (!from_zero) {
-                if (et == 0 && alive) st_release_gpu(p.flags + blockIdx.x, 1);
+                if (et == 0) raise_flag(p.flags + blockIdx.x);
             } else {
                 if (owner) {     // add the partials in CTA order
                     if (alive && col0 < p.M) {
@@ -719,8 +729,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                         }
                     }
                     epi_sync();
-                    if (alive)
-                        for (int c = blockIdx.x + 1 + et; c <= last; c += kEpi) p.flags[c] = 0;
+                    for (int c = blockIdx.x + 1 + et; c <= last; c += kEpi) lower_flag(p.flags + c);
                 }
                 const int nrow = nrow0 + row;
                 // Rows of C that take 8-byte stores: the four lanes that hold four neighbouring weight rows exchange their
