@@ -397,7 +397,7 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         auto on_enter = [&](const TileCursor& c) {
             if (me == 0 && alive) {
                 const int qs = qc & 1;
-                alive = mbar_wait_lane0(empty_q + qs * 8, ((qc >> 1) & 1) ^ 1, abort_flag, p.status, kDevTimeoutEmptyQ);
+                alive = mbar_wait_warp(empty_q + qs * 8, ((qc >> 1) & 1) ^ 1, abort_flag, p.status, kDevTimeoutEmptyQ);
                 if (alive && elect_one()) {
                     mbar_arrive_expect_tx(full_q + qs * 8, kQBytes + kWBytes);
                     tma_load_2d(q_smem + qs * kQBytes, &q_map, full_q + qs * 8, 0, c.b * kHeads);
@@ -439,7 +439,7 @@ mqa_logits_fp4_paged_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 phys = 0;
             }
             const int s = ring.idx;
-            alive = mbar_wait_lane0(empty_kv + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutEmptyKv);
+            alive = mbar_wait_warp(empty_kv + s * 8, ring.phase ^ 1u, abort_flag, p.status, kDevTimeoutEmptyKv);
             if (!alive) break;
             int page[kMaxPages];
 #pragma unroll

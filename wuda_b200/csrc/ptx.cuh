@@ -140,7 +140,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 // Warp-uniform forms, so that all 32 lanes take the same branch afterwards (callers use
 // full-mask shuffles and __syncwarp).  `_warp`: every lane polls (each lane that later
 // reads data written by the async proxy must observe the barrier itself), then votes.
-// `_lane0`: only lane 0 polls and the result is broadcast.
+// `_lane0`: only lane 0 polls and the result is broadcast; the other lanes' later accesses are ordered behind it by a
+// warp barrier (the shuffle alone orders nothing).  Not before copies or MMAs that an elected lane issues: that lane need not
+// be lane 0.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity,
                                                volatile int* abort_flag, int* status_word,
                                                int code) {
@@ -152,6 +154,7 @@ __device__ __forceinline__ bool mbar_wait_lane0(uint32_t bar, uint32_t parity,
                                                 int code) {
     int ok = 1;
     if (lane_id() == 0) ok = mbar_wait(bar, parity, abort_flag, status_word, code) ? 1 : 0;
+    __syncwarp();
     return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 

@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         for (int j = me; j < blocks && alive; j += 2) {
             {
                 const int s = j % kOwnStages, t = j % kOthStages;
-                alive = mbar_wait_lane0(k_full + s * 8, (j / kOwnStages) & 1u, abort_flag, p.status, kDevTimeoutMlaKeys);
+                alive = mbar_wait_warp(k_full + s * 8, (j / kOwnStages) & 1u, abort_flag, p.status, kDevTimeoutMlaKeys);
                 if (alive && j >= 1)
-                    alive = mbar_wait_lane0(s_empty + (me ^ 1) * 8, ((j - 1) >> 1) & 1u, abort_flag, p.status,
-                                            kDevTimeoutMlaScoresRead);   // the block before, the other issuer's
+                    alive = mbar_wait_warp(s_empty + (me ^ 1) * 8, ((j - 1) >> 1) & 1u, abort_flag, p.status,
+                                           kDevTimeoutMlaScoresRead);   // the block before, the other issuer's
                 if (!alive) break;
                 tc_fence_after();
                 if (elect_one()) {
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         bool alive = true;
         for (int j = 0; j < blocks && alive; ++j) {
             const int t = j & 1, s = j % kOwnStages;
-            alive = mbar_wait_lane0(p_full + t * 8, (j >> 1) & 1u, abort_flag, p.status, kDevTimeoutMlaProbs);
+            alive = mbar_wait_warp(p_full + t * 8, (j >> 1) & 1u, abort_flag, p.status, kDevTimeoutMlaProbs);
             if (!alive) break;
             tc_fence_after();
             if (elect_one()) {
