@@ -576,18 +576,16 @@ static int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, Params& p,
 }  // namespace gemm8
 }  // namespace wuda
 
-// Scratch = one flag per CTA (the first kFlagBytes bytes), then one fp32 partial tile [M_PAD][128] per CTA.
-// The grid never exceeds kMaxGrid CTAs (one per SM).  The flags come first so that calls with different row
-// counts, which size their slots differently, find them in the same place: one scratch buffer can then serve
-// every GEMM of a stream without a slot of one call ever covering the flags of another.
-constexpr int kMaxGrid = 192;
-constexpr int64_t kFlagBytes = 1024;
+// Scratch = flags or counters (the first kFlagBytes bytes), then kMaxGrid slots of one fp32 partial tile [M_PAD][128].
+// The flags come first so that calls with different row counts, which size their slots differently, find them in the same
+// place: one scratch buffer can then serve every GEMM of a stream without a slot of one call ever covering the flags of
+// another.  All kinds share one layout.
+using wuda::gemmtc::kFlagBytes;
+using wuda::gemmtc::kMaxGrid;
 
 extern "C" int64_t wuda_gemm_fp8_scratch_bytes(int m, int n) {
     if (m < 1 || n < 1 || m > 256) return -1;
-    int m_pad = 16;
-    while (m_pad < m) m_pad *= 2;
-    return kFlagBytes + static_cast<int64_t>(kMaxGrid) * m_pad * 128 * 4;
+    return wuda::gemmtc::scratch_bytes(m);
 }
 
 namespace {

@@ -833,7 +833,7 @@ int launch_for(int m, const CUtensorMap& w_map, const CUtensorMap& a_map, const 
     return launch<KIND, 128>(w_map, a_map, wsf_map, asf_map, p, dev, stream);
 }
 
-// Bytes of scratch a call with m rows wants: the flags and a partial-tile slot per CTA.
+// Bytes of scratch a call with m rows wants: the flags and kMaxGrid partial-tile slots.
 inline int64_t scratch_bytes(int m) {
     int m_pad = 16;
     while (m_pad < m) m_pad *= 2;
