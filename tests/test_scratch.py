@@ -96,3 +96,11 @@ def test_a_scratch_that_needs_no_zeros_keeps_no_flags(captures):
     call(kept, captures, 1, 1 << 10)
     captures.of_stream = {1: 7}
     assert call(kept, captures, 1, 1 << 10)[1] is None and not kept._flags
+
+
+@pytest.mark.parametrize("kind", ["fp8", "nvfp4", "bf16"])
+def test_operators_ask_the_library_for_the_size(kind):
+    from wuda_b200 import ops
+    name = "wuda_gemm_%s_scratch_bytes" % kind
+    for m in (1, 16, 17, 128, 128, 129, 257):
+        assert ops._scratch_bytes(name, m, 300) == getattr(ops.lib, name)(m, 300)

@@ -735,7 +735,7 @@ def fp4_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
     a_sf = _scales_as_fp32(a_s, "a_s")
     if out is None:
         out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-    need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
+    need = _scratch_bytes("wuda_gemm_fp8_scratch_bytes", m, n)
     _require(need >= 0, "m must be in [1, 256]")
     _launch_gemm(lib.wuda_gemm_fp8_fp4_pow2, a.device, need,
                  (a.data_ptr(), a_sf.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k), _ptr(status_word))
@@ -748,7 +748,7 @@ _gemm_scratch = Scratch(zeroed=True)
 @functools.lru_cache(maxsize=1024)
 def _scratch_bytes(entry, m, n):
     """What the library asks for these sizes (asking takes longer than finding out whether the stream is being captured)."""
-    return entry(m, n)
+    return getattr(lib, entry)(m, n)
 
 
 def _launch_gemm(entry, device, need, operands, *rest):
@@ -786,7 +786,7 @@ def fp8_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
              and tuple(b_s.shape) == ((n + 127) // 128, k // 128), "b_s must be contiguous CUDA fp32 [ceil(N/128), K/128]")
     if out is None:
         out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-    need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
+    need = _scratch_bytes("wuda_gemm_fp8_scratch_bytes", m, n)
     _require(need >= 0, "m must be in [1, 256]")
     _launch_gemm(lib.wuda_gemm_fp8_blockscaled_pow2 if pow2_scales else lib.wuda_gemm_fp8_blockscaled, a.device, need,
                  (a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k), _ptr(status_word))
@@ -806,7 +806,7 @@ def bf16_gemm(a, w, *, out=None, out_dtype=torch.bfloat16, status_word=None):
         out = a.new_empty((*a.shape[:-1], n), dtype=out_dtype)
     _require(out.is_contiguous() and out.dtype in (torch.bfloat16, torch.float32) and out.numel() == m * n,
              "out must be contiguous bf16 or fp32 [M, N]")
-    need = _scratch_bytes(lib.wuda_gemm_bf16_scratch_bytes, m, n)
+    need = _scratch_bytes("wuda_gemm_bf16_scratch_bytes", m, n)
     _require(need >= 0, "m must be in [1, 128]")
     _launch_gemm(lib.wuda_gemm_bf16, a.device, need,
                  (a.data_ptr(), w.data_ptr(), out.data_ptr(), int(out.dtype == torch.float32), m, n, k), _ptr(status_word))
@@ -942,7 +942,7 @@ class TP2Link:
         _require(m <= self.m and n == self.n, "shape outside what the link was created for")
         if out is None:
             out = a.new_empty((*a.shape[:-1], n), dtype=torch.bfloat16)
-        need = _scratch_bytes(lib.wuda_gemm_fp8_scratch_bytes, m, n)
+        need = _scratch_bytes("wuda_gemm_fp8_scratch_bytes", m, n)
         self.epoch += 1
         _launch_gemm(lib.wuda_gemm_fp8_blockscaled_tp2, a.device, need,
                      (a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), out.data_ptr(), m, n, k),
@@ -982,7 +982,7 @@ def nvfp4_gemm(a, a_sf_packed, a_global_scale, w, w_sf_packed, w_global_scale, *
              and w_sf_packed.numel() == ((n + 127) // 128) * 128 * (k // 16), "w_sf_packed has the wrong size")
     if out is None:
         out = a.new_empty((m, n), dtype=torch.bfloat16)
-    need = _scratch_bytes(lib.wuda_gemm_nvfp4_scratch_bytes, m, n)
+    need = _scratch_bytes("wuda_gemm_nvfp4_scratch_bytes", m, n)
     _require(need >= 0, "m must be in [1, 256]")
     _launch_gemm(lib.wuda_gemm_nvfp4, a.device, need,
                  (a.data_ptr(), a_sf_packed.data_ptr(), float(a_global_scale), w.data_ptr(), w_sf_packed.data_ptr(),
