@@ -665,8 +665,8 @@ int wuda_swiglu_quant_fp8(const void* h_bf16, void* y_bf16, void* y_fp8, float* 
  *   w         e4m3 [n, k], 16-byte aligned;   w_scales fp32 [ceil(n/128), k/128]
  *   c_bf16    bf16 [m, n];   1 <= m <= 256, k % 128 == 0
  *   scratch   device memory of at least wuda_gemm_fp8_scratch_bytes(m, n) bytes, 256-byte
- *             aligned, ZERO before the first call; the kernel leaves it zero again, so the
- *             same scratch can serve call after call (calls that share it must not overlap
+ *             aligned, ZERO before the first call; the kernel leaves its flags zero again (also
+ *             when a wait ran out), so the same scratch can serve call after call (calls that share it must not overlap
  *             on the GPU).  It holds the fp32 partial tiles of weight tiles whose K range is
  *             split across SMs.
  */

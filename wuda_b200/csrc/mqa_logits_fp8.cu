@@ -171,7 +171,7 @@ mqa_logits_fp8_kernel(const __grid_constant__ CUtensorMap q_map,
         // All copies of a tile (key bytes and scales of every page) go out as ONE
         // tensor-copy instruction with one lane per copy.  (Four producers have the time for it; the pages by shuffles
         // to one elected lane took 92.6 us instead of 88.4 for the indexer step of 64 requests x 2 rows.  The MMA issuers
-        // are elected lanes: 88.4 -> 87.4 us, 64 x 32768 tokens 69.6 -> 68.2 us, both with the top-k.)
+        // are elected lanes, which changed nothing that stands out of the noise.)
         const int me = warp;
         const uint64_t stream_policy = policy_evict_first();
         const int ppt = kTile / p.epb;                   // pages per tile: 4, 2 or 1
