@@ -166,14 +166,14 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         tmem_alloc(smem_u32(tmem_slot), L::kTmemCols);
         tmem_relinquish();
     }
-    const long long units = static_cast<long long>(p.n_tiles) * p.kb;
-    const long long u0 = range_begin(units, blockIdx.x, gridDim.x);
+    const uint32_t units = static_cast<uint32_t>(p.n_tiles) * static_cast<uint32_t>(p.kb);
+    const uint32_t u0 = range_begin(units, blockIdx.x, gridDim.x);
     const int count = static_cast<int>(range_begin(units, blockIdx.x + 1, gridDim.x) - u0);
-    const int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
+    const int tile0 = static_cast<int>(u0 / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
     // The last tile of a stream-K range may go on in the following CTAs (all resident: the grid is one CTA per SM).  If this
     // CTA holds its start, it adds their partials, of CTAs blockIdx.x + 1 .. last_peer, in CTA order.
-    const long long last_tile = static_cast<uint32_t>(u0 + count - 1) / static_cast<uint32_t>(p.kb);
-    const bool shares = !p.sliced && last_tile * p.kb >= u0 && (last_tile + 1) * p.kb > u0 + count;
+    const uint32_t last_tile = (u0 + count - 1u) / static_cast<uint32_t>(p.kb);
+    const bool shares = !p.sliced && last_tile * p.kb >= u0 && (last_tile + 1u) * p.kb > u0 + count;
     if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
@@ -336,7 +336,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
         uint32_t held = 0;                              // sliced: who shares the first and the second tile of this range
         if (p.sliced) {
             held = holders_of(units, tile0, p.kb, gridDim.x);
-            if (last_tile != tile0) held |= holders_of(units, tile0 + 1, p.kb, gridDim.x) << 16;
+            if (last_tile != static_cast<uint32_t>(tile0)) held |= holders_of(units, tile0 + 1, p.kb, gridDim.x) << 16;
         }
 
         // An aborting CTA keeps walking the loop (every wait then fails at once) so that all
@@ -529,8 +529,8 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 epi_bar_sync();
                 alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                 if (alive)
-                    gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile0 + i, unpack_holders(held, i), et, 32 * kEpiWarps, p.M, p.N, 1.f, 0,
-                                                          p.c);
+                    gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile0 + i, unpack_holders(held, i), gemmtc::start_slot(tile0 + i), et,
+                                                          32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
             }
         }
     }

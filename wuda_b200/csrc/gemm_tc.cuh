@@ -56,6 +56,7 @@ constexpr int kImgSlots = 4;
 constexpr int kImgBlock = 512;                // scale bytes of 128 rows, four bytes each: [row % 32][row / 32]
 constexpr int kNvSfBytes = 2048;              // NVFP4: packed scales of 128 rows x 256 K
 constexpr int kMaxGrid = 192;
+constexpr int kMaxEvenSplit = 32;
 constexpr int64_t kFlagBytes = 1024;          // the flags lead the scratch, whatever the shape (kernels share scratches)
 
 struct Params {
@@ -67,7 +68,7 @@ struct Params {
     int M, N, kb, n_tiles;     // kb = units per weight tile
     int a_rows;                // M rounded up to 16
     int stages;
-    int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each
+    int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each (even slices: how many CTAs)
     // power-of-two scaled kinds
     const float* a_scales;     // [M, scale_cols]
     const float* w_scales;     // [n_tiles, kb] (FP8 weights)
@@ -92,11 +93,13 @@ struct Layout {
     // order of the additions is part of the layer's results: another order moves single roundings of the projections, and
     // the 4-bit activations of the experts behind them turn those into 4e-3 of the layer's output.
     static constexpr int kAccs = (KIND == Kind::kMx8 || KIND == Kind::kBf16) && M_PAD <= 128 ? 2 : 1;
+    // Beyond 128 rows there is no earlier order to keep (those were two passes), and a CTA's partial sums are 128 KB per tile, so
+    // few tiles are cut evenly and no CTA holds parts of two (4096 x 7168 FP8 at 200 rows 29.8 -> 20.5 us).
+    static constexpr bool kEvenSlices = M_PAD > 128;
     static constexpr int kBuffers = kAccs * M_PAD <= 128 ? 2 : 1;
     // Epilogue warps: behind the last copy they move partial sums and results with the bytes in flight that they have, so
     // 256 rows take sixteen (7168 x 16384 FP8 43.8 -> 40.4 us; not with 4-bit weights, whose scale images need the
-    // registers).  At 128 rows sixteen gain 0.4 us of 24.8 alone but leave no registers for the next kernel of a chain to
-    // set itself up beside this one: the layer at batch 128 takes 1452 instead of 1438 us.
+    // registers).  At 128 rows sixteen are slower: NVFP4 24576 x 7168 28.8 -> 31.4 us, the layer at batch 128 1498 -> 1519.
     static constexpr int kEpiWarps = M_PAD == 256 && KIND != Kind::kMx8W4 ? 16 : (M_PAD >= 64 ? 8 : 4);
     static constexpr int kThreads = 32 * (4 + kEpiWarps);
     static constexpr int kCols = M_PAD / (kEpiWarps / 4);             // accumulator columns per epilogue thread
@@ -143,14 +146,14 @@ __device__ __forceinline__ int inc_acq_rel_gpu(int32_t* p, int limit) {
     asm volatile("atom.acq_rel.gpu.global.inc.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(limit) : "memory");
     return old;
 }
-// floor(units * c / grid) for fewer than 2^32 units (16 KB each), in 32-bit divisions: a launch's prologue is on the critical path of a short call, and a 64-bit
-// division takes a few hundred cycles
-__device__ __forceinline__ long long range_begin(long long units, int c, int grid) {
-    const uint32_t u = static_cast<uint32_t>(units), g = static_cast<uint32_t>(grid), q = u / g, rest = u - q * g;
-    return static_cast<long long>(q) * c + rest * static_cast<uint32_t>(c) / g;
+// floor(units * c / grid) for fewer than 2^32 units (16 KB each), in 32-bit divisions: a launch's prologue is on the critical
+// path of a short call, and a 64-bit division takes a few hundred cycles
+__device__ __forceinline__ uint32_t range_begin(uint32_t units, uint32_t c, uint32_t grid) {
+    const uint32_t q = units / grid, rest = units - q * grid;
+    return q * c + rest * c / grid;
 }
-__device__ __forceinline__ int cta_of(long long units, long long u, int grid) {
-    int c = static_cast<int>(u * grid / units);
+__device__ __forceinline__ int cta_of(uint32_t units, uint32_t u, int grid) {
+    int c = static_cast<int>(static_cast<uint64_t>(u) * static_cast<uint32_t>(grid) / units);
     while (c + 1 < grid && range_begin(units, c + 1, grid) <= u) ++c;
     while (c > 0 && range_begin(units, c, grid) > u) --c;
     return c;
@@ -217,26 +220,27 @@ struct Holders {
     __device__ __forceinline__ int count() const { return last - first + 1; }
 };
 // .. as one word (there are fewer than 256 CTAs): two tiles' stay in registers until the end of a range
-__device__ __forceinline__ uint32_t holders_of(long long units, int tile, int kb, int grid) {
-    const long long begin = static_cast<long long>(tile) * kb;
+__device__ __forceinline__ uint32_t holders_of(uint32_t units, int tile, int kb, int grid) {
+    const uint32_t begin = static_cast<uint32_t>(tile) * static_cast<uint32_t>(kb);
     return static_cast<uint32_t>(cta_of(units, begin, grid)) | static_cast<uint32_t>(cta_of(units, begin + kb - 1, grid)) << 8;
 }
 __device__ __forceinline__ Holders unpack_holders(uint32_t both, int i) {
     return {static_cast<int>(both >> (16 * i) & 0xffu), static_cast<int>(both >> (16 * i + 8) & 0xffu)};
 }
-// Slot of this CTA's partial sums: the one that starts a sliced tile goes behind the CTAs' own (its CTA may hold the end
-// of the tile before, too).
+// Slot of this CTA's partial sums.  Those that start a sliced tile go behind the CTAs' own (their CTA may hold the end of the
+// tile before, too).
+__device__ __forceinline__ int start_slot(int tile) { return static_cast<int>(gridDim.x) + tile; }
 __device__ __forceinline__ int slot_index(int sliced, bool from_zero, int tile) {
-    return sliced && from_zero ? static_cast<int>(gridDim.x) + tile : static_cast<int>(blockIdx.x);
+    return sliced && from_zero ? start_slot(tile) : static_cast<int>(blockIdx.x);
 }
 
 // This CTA's slice of a weight tile: the sum over all partials, in CTA order, scaled and stored.
 // A thread adds four activation rows of a weight row, eight partials in flight.
 template <Kind KIND>
-__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, Holders h, int thread, int threads, int M,
-                                          int N, float out_scale, int c_is_fp32, void* c) {
+__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, Holders h, int first_slot, int thread,
+                                          int threads, int M, int N, float out_scale, int c_is_fp32, void* c) {
     const int j = static_cast<int>(blockIdx.x) - h.first, parts = h.count(), quads = (M + 3) / 4 * kTileN;
-    const float4* start = reinterpret_cast<const float4*>(scratch + (static_cast<int64_t>(gridDim.x) + tile) * slot_floats);
+    const float4* start = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(first_slot) * slot_floats);
     const float4* part = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(h.first) * slot_floats);   // [1], [2], ..
     const int end = quads * (j + 1) / parts;
     for (int e = quads * j / parts + thread; e < end; e += threads) {
@@ -308,13 +312,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     }
     const bool grouped = KIND == Kind::kNv4 && p.group_expert != nullptr;
     // the unit range of this CTA (the grouped form learns its number of units from the kernel ahead)
-    long long units = static_cast<long long>(p.n_tiles) * p.kb, u0 = 0;
+    uint32_t units = static_cast<uint32_t>(p.n_tiles) * static_cast<uint32_t>(p.kb), u0 = 0;
     int grid = static_cast<int>(gridDim.x), count = 0;
     if (!grouped) {
         u0 = range_begin(units, blockIdx.x, grid);
         count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
     }
-    int tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
+    int tile0 = static_cast<int>(u0 / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
     if (warp == 0 && elect_one()) {
         prefetch_tmap(&w_map);
         prefetch_tmap(&a_map);
@@ -342,11 +346,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         // Only the first min(grid, units) CTAs take part: every participating CTA then owns at least one unit, which
         // the fix-up relies on when it waits for the CTAs that share a tile.
         units *= *p.num_groups;
-        if (units < grid) grid = static_cast<int>(units);
+        if (units < static_cast<uint32_t>(grid)) grid = static_cast<int>(units);
         if (static_cast<int>(blockIdx.x) < grid) {
             u0 = range_begin(units, blockIdx.x, grid);
             count = static_cast<int>(range_begin(units, blockIdx.x + 1, grid) - u0);
-            tile0 = static_cast<int>(static_cast<uint32_t>(u0) / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
+            tile0 = static_cast<int>(u0 / static_cast<uint32_t>(p.kb)), kb0 = static_cast<int>(u0) - tile0 * p.kb;
         }
     }
 
@@ -603,6 +607,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     } else {
         // ------------------------------------------------------------ epilogue
         constexpr int kEpi = 32 * L::kEpiWarps, kCols = L::kCols;
+        constexpr bool kEven = L::kEvenSlices;
         auto epi_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(kEpi) : "memory"); };
         const int et = static_cast<int>(threadIdx.x) - 128;
         const int row = et & 127, col0 = (et >> 7) * kCols;      // weight row inside the tile, first column
@@ -610,16 +615,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
         bool alive = true;
         int tile = tile0, kb = kb0;
         uint32_t seg = 0;
-        const int64_t slot_floats = static_cast<int64_t>(M_PAD) * kTileN;
+        constexpr int64_t slot_floats = static_cast<int64_t>(M_PAD) * kTileN;
         int grp = 0, seen_grp = -1;
         float scale = p.out_scale;
         uint32_t stored = 0xffffffffu;       // grouped rows without a token are padding: nobody reads them
-        // sliced: who shares the first and the second tile of this range (found out beside the stream, except by the 256-row
-        // form, which has no register left to keep it)
-        constexpr bool kKeep = M_PAD < 256;
+        // sliced: who shares the first and the second tile of this range
         uint32_t held = 0;
-        auto holders = [&](int i) {
-            return unpack_holders(kKeep ? held : holders_of(units, tile0 + i, p.kb, grid) << (16 * i), i);
+        auto holders = [&](int i) -> Holders {
+            if (!kEven) return unpack_holders(held, i);
+            const int first = static_cast<int>(blockIdx.x) / p.sliced * p.sliced;
+            return {first, first + p.sliced - 1};
+        };
+        // this CTA's slice of its first or second tile, once the partial sums of all are there
+        auto slice = [&](int i) {
+            const int of = kEven ? static_cast<int>(blockIdx.x) / p.sliced : tile0 + i;   // (not from tile0: it would take a register)
+            if (et == 0 && alive) await_word(p.flags + of, [](int v) { return v == 0; }, abort_flag, p.status);
+            epi_sync();
+            alive = __all_sync(0xffffffffu, alive && !*abort_flag);
+            if (alive) {
+                const Holders h = holders(i);
+                add_slice<KIND>(p.scratch, slot_floats, of, h, kEven ? h.first : start_slot(of), et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32,
+                                p.c);
+            }
         };
         for (int n = 0; n < count;) {
             // the segment [kb, kb_end) of `tile`
@@ -649,9 +666,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             auto slot_of = [&](int c) {
                 return reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * slot_floats) + col0 / 4 * kTileN + row;
             };
-            if (kKeep && p.sliced) held |= holders_of(units, tile, p.kb, grid) << (16 * seg);
+            if (!kEven && p.sliced) held |= holders_of(units, tile, p.kb, grid) << (16 * seg);
             if (owner) {
-                last = cta_of(units, static_cast<long long>(tile + 1) * p.kb - 1, grid);
+                last = cta_of(units, static_cast<uint32_t>(tile + 1) * static_cast<uint32_t>(p.kb) - 1u, grid);
                 for (int c = blockIdx.x + 1 + et; c <= last && alive; c += kEpi)
                     await_word<200>(p.flags + c, [](int v) { return v != 0; }, abort_flag, p.status);
                 epi_sync();
@@ -693,7 +710,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
 
             const int nrow0 = (tile - grp * p.n_tiles) * kTileN;
             if (p.sliced || !from_zero) {   // partial sums to this CTA's slot
-                float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced, from_zero, tile) * slot_floats) + row;
+                float4* slot = reinterpret_cast<float4*>(p.scratch + slot_index(p.sliced && !kEven, from_zero, tile) * slot_floats) + row;
 #pragma unroll
                 for (int c = 0; c < kCols; c += 4)
                     if (col0 + c < p.M) __stcg(slot + (col0 + c) / 4 * kTileN, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
@@ -704,6 +721,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 // The last arrival wraps the tile's counter back to zero, which is what the others wait for, once they have
                 // nothing else to do.  No CTA arrives at a counter twice in a launch, the next launch's arrive after this one.
                 if (et == 0) inc_acq_rel_gpu(p.flags + tile, holders(seg).count() - 1);
+                if (kEven) slice(0);
             } else if (!from_zero) {
                 if (et == 0) raise_flag(p.flags + blockIdx.x);
             } else {
@@ -768,16 +786,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (kb == p.kb) kb = 0, ++tile;
             ++seg;
         }
-        if (p.sliced) {
+        if (!kEven && p.sliced) {
 #pragma unroll 1
-            for (uint32_t i = 0; i < seg; ++i) {
-                if (et == 0 && alive) await_word(p.flags + tile0 + i, [](int v) { return v == 0; }, abort_flag, p.status);
-                epi_sync();
-                alive = __all_sync(0xffffffffu, alive && !*abort_flag);
-                if (alive)
-                    add_slice<KIND>(p.scratch, slot_floats, tile0 + static_cast<int>(i), holders(i), et, kEpi, p.M, p.N, p.out_scale,
-                                    p.c_is_fp32, p.c);
-            }
+            for (uint32_t i = 0; i < seg; ++i) slice(i);
         }
     }
 
@@ -800,6 +811,13 @@ inline int grid_of(long long units, int n_tiles, int m_pad, int sms) {
 }
 // Added in slices where every tile is cut into three ranges or more (and the slots suffice: one per CTA and one per tile).
 inline bool slice_wise(int grid, int n_tiles) { return grid >= 3 * n_tiles && grid + n_tiles <= kMaxGrid; }
+// Even slices: CTAs per tile, as many as the SMs hold when that is at least three (and every one gets a unit), else none.
+inline int even_split(int n_tiles, int kb, int sms) {
+    int split = sms / n_tiles;
+    if (split > kb) split = kb;
+    if (split > kMaxEvenSplit) split = kMaxEvenSplit;
+    return split >= 3 ? split : 0;
+}
 
 template <Kind KIND, int M_PAD>
 int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap& wsf_map, const CUtensorMap& asf_map, Params& p,
@@ -815,8 +833,13 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap
     WUDA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
     const int sms = gemm_sms(dev);
     // (grouped: the number of groups is only known on the device; one CTA per SM, idle ones return at once)
-    const int grid = p.group_expert ? sms : grid_of(static_cast<long long>(p.n_tiles) * p.kb, p.n_tiles, M_PAD, sms);
-    p.sliced = !p.group_expert && slice_wise(grid, p.n_tiles);
+    int grid = p.group_expert ? sms : grid_of(static_cast<long long>(p.n_tiles) * p.kb, p.n_tiles, M_PAD, sms);
+    if (L::kEvenSlices) {
+        p.sliced = even_split(p.n_tiles, p.kb, sms);
+        if (p.sliced) grid = p.n_tiles * p.sliced;
+    } else {
+        p.sliced = !p.group_expert && slice_wise(grid, p.n_tiles);
+    }
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(L::kThreads), L::total(stages, p.a_rows), stream, w_map, a_map, wsf_map, asf_map, p));
     return WUDA_OK;
 }
