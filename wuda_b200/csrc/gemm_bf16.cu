@@ -9,8 +9,8 @@
 //
 // The kernel is gemm_tc.cuh's: a unit is 128 weight rows x 64 K-elements, four tcgen05.mma kind::f16 (K = 16); nothing is
 // rescaled between K blocks.
-// Measured (CUDA-graph replays, us; before = four fetching and two issuing warps, partials added by one CTA per tile):
-// 7168 x 16384 at 64 rows 46.9 -> 43.0, 4096 x 7168 at 100 rows 28.5 -> 20.5, 256 x 7168 at 64 rows (the router) 17.8 -> 10.3.
+// Measured (as in gemm_tc.cuh, us; before = four fetching and two issuing warps, partials added by one CTA per tile):
+// 7168 x 16384 at 64 rows 50.3 -> 46.7, 4096 x 7168 at 100 rows 27.7 -> 23.0, 256 x 7168 at 64 rows (the router) 16.4 -> 10.3.
 #include "gemm_tc.cuh"
 
 extern "C" int64_t wuda_gemm_bf16_scratch_bytes(int m, int n) {

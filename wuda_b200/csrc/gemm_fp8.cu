@@ -22,11 +22,11 @@
 //    epilogue thread waits once per unit.  The two epilogue warpgroups take units alternately and their chains overlap; the
 //    two accumulator sets are added when a tile's segment ends.  (Above 64 activation rows a thread cannot hold all
 //    columns; the groups then split the columns and both take every unit.)
-// Measured (CUDA-graph replays, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
-// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 39.0 -> 35.0,
-// 43.9 -> 37.2, 62.7 -> 45.9, 122.5 -> 89.7 (two passes); 7168 x 16384 at 64 rows 32.5 -> 28.8; 2112 x 7168 at 1 / 64 rows
-// 12.3 -> 10.3, 15.3 -> 10.3; 4096 x 7168 at 64 rows 17.8 -> 14.4.  The results are bit-identical
-// to those of the earlier form: the order of the additions is the same.
+// Measured (as in gemm_tc.cuh, us; before = scales fetched by the epilogue threads behind two barriers per unit, resident
+// activations for short K, partials added by one CTA per tile): 24576 x 7168 at 16 / 64 / 128 / 256 rows 38.3 -> 34.7,
+// 47.1 -> 40.6, 66.1 -> 54.7, 131 -> 109 (two passes); 7168 x 16384 at 64 rows 32.9 -> 29.5; 2112 x 7168 at 1 / 64 rows
+// 13.3 -> 12.3, 16.4 -> 11.0; 4096 x 7168 at 64 rows 17.6 -> 16.7.  The results are bit-identical to those of the earlier
+// form: the order of the additions is the same.
 // Every wait is bounded and reports through the status word; flags and counters end at zero all the same (gemm_tc.cuh).
 #include <cuda.h>
 #include <cuda_bf16.h>

@@ -17,11 +17,11 @@
 // are the four 32-wide scales of one K block, so every unit has its own weight image).
 // A scale that is not a power of two is truncated to one and reported (WUDA_DEV_SCALE_NOT_POW2); a zero scale
 // reads as 2^-127.
-// Measured (CUDA-graph replays, us; before = scale images built unit by unit by the fetching warps, two accumulators,
+// Measured (as in gemm_tc.cuh, us; before = scale images built unit by unit by the fetching warps, two accumulators,
 // passes of 128 rows, partials added by one CTA per tile):
-//   24576 x 7168 at 64 rows 41.0 -> 35.1; 7168 x 16384 at 256 rows 69.5 -> 39.3; 73728 x 1536 at 64 rows (the q
-//   projection; before with the activations resident in shared memory) 28.8 -> 25.8; 4096 x 7168 at 64 rows 20.5 -> 14.7;
-//   4-bit weights: 24576 x 7168 at 64 rows 32.0 -> 28.7, 7168 x 16384 at 200 rows 76 -> 39
+//   24576 x 7168 at 64 rows 44.4 -> 38.6; 7168 x 16384 at 256 rows 78.6 -> 51.0; 73728 x 1536 at 64 rows (the q
+//   projection; before with the activations resident in shared memory) 29.6 -> 28.7; 4096 x 7168 at 64 rows 20.5 -> 18.4;
+//   4-bit weights: 24576 x 7168 at 64 rows 37.6 -> 30.7, 7168 x 16384 at 200 rows 75.9 -> 44.4
 #include "gemm_tc.cuh"
 
 namespace wuda {

@@ -15,8 +15,8 @@
 // Scale layout in global memory ("packed"): per 128 rows x 256 K one 2 KB block
 // [4 K/64 steps][32 = row % 32][4 = row / 32][4 scales of the step], blocks ordered [row tile][K/256].
 // It is the image tcgen05.cp.32x128b.warpx4 expects, so a unit's scales are one contiguous copy.
-// Measured (CUDA-graph replays, us; before = four fetching and two issuing warps, passes of 128 rows): 24576 x 7168 at
-// 8 rows 23.2 -> 21.7, at 128 rows 33.1 -> 24.9, at 200 rows 64.4 -> 29.3; 7168 x 16384 at 64 rows 22.6 -> 19.2; routed
+// Measured (as in gemm_tc.cuh, us; before = four fetching and two issuing warps, passes of 128 rows): 24576 x 7168 at
+// 8 rows 24.1 -> 21.3, at 128 rows 34.9 -> 28.7, at 200 rows 66.8 -> 36.9; 7168 x 16384 at 64 rows 23.6 -> 19.3; routed
 // experts of 64 tokens (grouped) 884 -> 877 per block
 //
 // Grouped form (routed experts): row group g (16 activation rows) belongs to expert group_expert[g]; flat tile
