@@ -42,6 +42,13 @@ int gemm_sms(const DeviceInfo& dev);
 // Where those launches find their flags: at the front of the scratch, or where wuda_gemm_flags said
 int32_t* gemm_flags(void* scratch);
 
+// wuda_mhc_pre; with act_quant its FP8 output is what wuda_rmsnorm_quant_fp8 makes of `normed` with power-of-two scales (the two
+// differ in where the smallest scale lies, and for infinities and NaN).
+int mhc_pre_as(bool act_quant, const void* hidden_states, const float* weight, const float* base, const float* scale,
+               const void* attn_norm_gamma, float hc_eps, float rms_eps, float norm_eps, float* pre, float* post, float* comb,
+               void* collapsed_bf16, void* normed_bf16, void* x_fp8, float* x_scales, void* workspace, int64_t workspace_bytes, int m,
+               int hidden, void* stream);
+
 // rank-`rank` tiled tensor map. dims/box are innermost-first; strides_bytes has rank-1
 // entries (stride of dims 1..rank-1). Returns a wuda_status.
 int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const void* base,
@@ -71,6 +78,8 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Asks L2 for the line at p: a hint that reads nothing into the SM, so it may go out before pdl_wait().
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 #endif
 

@@ -11,7 +11,7 @@
 //   inverse RoPE + quantisation, grouped wo_a, quantisation, wo_b (on a pair: K-split with the all-reduce
 //       fused into the epilogue over peer memory), mHC post
 //   mHC pre (ffn weights) + ffn RMSNorm, router projection + routing
-//   shared expert (quantise, w1|w3, SwiGLU + quantise, w2), routed NVFP4 experts (dispatch, gather +
+//   shared expert (its input quantised by the mHC pre; w1|w3, SwiGLU + quantise, w2), routed NVFP4 experts (dispatch, gather +
 //       quantise, grouped w1|w3, SwiGLU + quantise, grouped w2), combine (on a pair: with the exchange of
 //       partial rows over peer memory), mHC post
 //
@@ -334,9 +334,9 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
     WUDA_STAGE(wuda_mhc_post(b.projected, t->hidden_in, b.a_post, b.a_comb, b.attn_out, m, hidden, stream));
 
     // ---------------------------------------------------------------- feed-forward half
-    WUDA_STAGE(wuda_mhc_pre(b.attn_out, w->ffn_hc_weight, w->ffn_hc_base, w->ffn_hc_scale, w->ffn_norm, w->hc_eps, w->rms_eps,
-                            w->norm_eps, b.f_pre, b.f_post, b.f_comb, nullptr, b.f_normed, nullptr, nullptr, b.pre_ws,
-                            wuda_mhc_pre_workspace_bytes(s->m_max, hidden), m, hidden, stream));
+    WUDA_STAGE(mhc_pre_as(true, b.attn_out, w->ffn_hc_weight, w->ffn_hc_base, w->ffn_hc_scale, w->ffn_norm, w->hc_eps, w->rms_eps,
+                          w->norm_eps, b.f_pre, b.f_post, b.f_comb, nullptr, b.f_normed, w->shared_w13 ? b.s_x8 : nullptr,
+                          w->shared_w13 ? b.s_xs : nullptr, b.pre_ws, wuda_mhc_pre_workspace_bytes(s->m_max, hidden), m, hidden, stream));
     // the shared expert on the side stream, beside router projection, routing, dispatch and gather
     const void* shared_rows = nullptr;
     if (w->shared_w13) {
@@ -344,9 +344,7 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
         WUDA_CUDA(cudaEventRecord(side->fork[1], main_stream));
         WUDA_CUDA(cudaStreamWaitEvent(side->stream, side->fork[1], 0));
         wuda_gemm_sm_limit(shared_sms(sms));
-        int st = wuda_rmsnorm_quant_fp8(b.f_normed, hidden, nullptr, 0, 0.0f, nullptr, b.s_x8, b.s_xs, m, hidden, 1, side->stream);
-        if (st == WUDA_OK)
-            st = wuda_gemm_fp8_blockscaled(b.s_x8, b.s_xs, w->shared_w13, w->shared_w13_scales, b.s_h, m, 2 * si, hidden,
+        int st = wuda_gemm_fp8_blockscaled(b.s_x8, b.s_xs, w->shared_w13, w->shared_w13_scales, b.s_h, m, 2 * si, hidden,
                                            b.side_scratch, b.gemm_scratch_bytes, status, side->stream);
         if (st == WUDA_OK) st = wuda_swiglu_quant_fp8(b.s_h, nullptr, b.s_a8, b.s_as, m, si, w->swiglu_limit, 1, side->stream);
         if (st == WUDA_OK)

@@ -35,7 +35,8 @@ constexpr int kStreams = 4;
 constexpr int kMix = 24;                 // pre 4 | post 4 | comb 16
 constexpr int kPart = kMix + 1;          // + sum of squares
 constexpr int kSlice = 512;              // K elements per slice
-constexpr int kMixThreads = 128;         // thread = token row of the tile = tensor-memory lane
+constexpr int kMixRows = 128;            // thread = token row of the tile = tensor-memory lane
+constexpr int kMixThreads = 256;         // the other four warps help to split the weights
 constexpr int kMixTile = 128;            // tokens per CTA (UMMA M)
 constexpr int kMixN = 80;                // 3 x 24 operand rows, padded to a multiple of 16 (UMMA N)
 constexpr int kKBlocks = kSlice / 64;    // 128-byte K blocks per slice
@@ -63,6 +64,7 @@ struct Params {
     float* x_scales;               // [m, hidden / 128]
     int m, hidden, slices;
     float hc_eps, rms_eps, norm_eps;
+    int act_quant;                 // x_fp8 by the rule of act_quant (amax clamped at 1e-4, times 1/448) instead of the fused kernel's
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) mhc_pre_mix_kernel(const __gri
         tmem_relinquish();
     }
     // the 24 x 512 weights of the slice (constants: they may be read before the kernel ahead has finished):
-    // item = (row j, 8 consecutive K) -> two 16-byte loads, twelve items per thread
+    // item = (row j, 8 consecutive K) -> two 16-byte loads, six items per thread
     constexpr int kItems = kMix * (kSlice / 8) / kMixThreads;
     float4 wraw[kItems][2];
 #pragma unroll
@@ -181,8 +183,9 @@ __global__ void __launch_bounds__(kMixThreads, 1) mhc_pre_mix_kernel(const __gri
         umma_commit(mma_done);
     }
     // sum of squares of this thread's token row, from the tile in shared memory, while the MMAs run
+    const bool has_row = threadIdx.x < kMixRows;
     float ss = 0.f;
-    if (alive) {
+    if (alive && has_row) {
         const int r = threadIdx.x;
 #pragma unroll 2
         for (int kb = 0; kb < kKBlocks; ++kb)
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kMixThreads, 1) mhc_pre_mix_kernel(const __gri
                 }
             }
     }
-    alive = alive && mbar_wait(mma_done, 0, abort_flag, nullptr, 0);
+    alive = alive && has_row && mbar_wait(mma_done, 0, abort_flag, nullptr, 0);
     const int t = tile * kMixTile + threadIdx.x;
     if (alive) {
         tc_fence_after();
@@ -290,9 +293,11 @@ __global__ void __launch_bounds__(128) mhc_tail_kernel(const float* mix, const f
 // barrier of the eight row warps alone (the ninth warp is busy with the Sinkhorn iterations or gone)
 __device__ __forceinline__ void row_warps_sync() { asm volatile("bar.sync 1, %0;" ::"n"(kFinishThreads) : "memory"); }
 
+// A chain of latencies (7 us for a few hundred KB): all its loads (the slices of a thread, the rows, gamma, the gates' scales and
+// bases) are one round, and the first of it is on its way to L2 before the wait.  With the weights of the mix split by eight
+// warps instead of four and the shared expert's input quantised here: the layer at batch 1 / 64 241.3 -> 236.4 / 1160 -> 1154 us.
 __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p) {
     pdl_launch_dependents();
-    pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
     __shared__ float mix[kPart];
     __shared__ float pre_s[kStreams];
     __shared__ float warp_ss[kFinishThreads / 32];
@@ -301,6 +306,8 @@ __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p)
     constexpr int kMaxVec = 4;                       // hidden <= 4 * 256 * 8 = 8192
     const bool row_warp = threadIdx.x < kFinishThreads;
     const int vectors = (row_warp && (p.collapsed || p.normed || p.x_fp8)) ? p.hidden / 8 : 0;
+    if (p.gamma && threadIdx.x * 64 < p.hidden) prefetch_l2(p.gamma + threadIdx.x * 64);   // (a hint: nothing is read before the wait)
+    pdl_wait();   // nothing of global memory is read before the kernel ahead has finished
     // the token's four rows are requested first: their latency hides behind the slice sums, the gates and the
     // Sinkhorn iterations, none of which needs them
     uint4 raw[kMaxVec][kStreams];
@@ -313,13 +320,31 @@ __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p)
                                      : make_uint4(0u, 0u, 0u, 0u);
     }
 
+    uint4 gamma[kMaxVec];
+#pragma unroll
+    for (int k = 0; k < kMaxVec; ++k) {
+        const int vi = threadIdx.x + k * kFinishThreads;
+        gamma[k] = vi < vectors && p.gamma ? __ldcg(reinterpret_cast<const uint4*>(p.gamma) + vi) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    const float pre_scale = __ldcg(p.scale), pre_base = __ldcg(p.base + (lane & (kStreams - 1)));
+
     // 25 sums over the slices: 8 groups of threads take every eighth slice each (independent loads), then
     // the 8 group sums are added in order - a fixed tree, so the result does not depend on timing
     __shared__ float group_sum[8][kPart];
     if (threadIdx.x < 8 * kPart) {
         const int j = threadIdx.x % kPart, grp = threadIdx.x / kPart;
         float s = 0.f;
-        for (int sl = grp; sl < p.slices; sl += 8) s += p.ws[(static_cast<int64_t>(sl) * p.m + t) * kPart + j];
+        for (int s0 = grp; s0 < p.slices; s0 += 64) {
+            float v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int sl = s0 + 8 * i;
+                v[i] = sl < p.slices ? p.ws[(static_cast<int64_t>(sl) * p.m + t) * kPart + j] : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if (s0 + 8 * i < p.slices) s += v[i];
+        }
         group_sum[grp][j] = s;
     }
     __syncthreads();
@@ -336,7 +361,7 @@ __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p)
         const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fdiv_rn(mix[kMix], static_cast<float>(kStreams * p.hidden)) + p.rms_eps));
         if (row_warp) {
             if (lane < kStreams) {
-                const float v = sigmoid(mix[lane] * r * p.scale[0] + p.base[lane]) + p.hc_eps;
+                const float v = sigmoid(mix[lane] * r * pre_scale + pre_base) + p.hc_eps;
                 pre_s[lane] = v;
                 if (p.pre) p.pre[t * kStreams + lane] = v;
             }
@@ -404,8 +429,7 @@ __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p)
         float amax = 0.f;
         uint4 o = make_uint4(0, 0, 0, 0);
         if (on) {
-            const uint4 graw = __ldg(reinterpret_cast<const uint4*>(p.gamma) + vi);
-            const uint32_t gw[4] = {graw.x, graw.y, graw.z, graw.w};
+            const uint32_t gw[4] = {gamma[k].x, gamma[k].y, gamma[k].z, gamma[k].w};
             uint32_t* ow = &o.x;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -422,7 +446,19 @@ __global__ void __launch_bounds__(kFinishLaunch) mhc_pre_finish_kernel(Params p)
         if (p.x_fp8) {
 #pragma unroll
             for (int s = 8; s > 0; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
-            if (on) {
+            if (on && p.act_quant) {
+                // as rmsnorm_quant_kernel quantises a row with power-of-two scales: v / s, one product with the exact
+                // reciprocal unless a value is infinite
+                const uint32_t bits = __float_as_uint(__fmul_rn(fmaxf(amax, 1e-4f), 1.0f / 448.0f));
+                const uint32_t exponent = ((bits >> 23) & 0xffu) + ((bits & 0x7fffffu) ? 1u : 0u);
+                const float s = __uint_as_float(exponent << 23), inv = __uint_as_float((254u - exponent) << 23);
+                float q[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q[i] = fminf(fmaxf(exponent < 255u ? __fmul_rn(v[i], inv) : __fdiv_rn(v[i], s), -448.f), 448.f);
+                *(reinterpret_cast<uint2*>(p.x_fp8 + static_cast<int64_t>(t) * p.hidden) + vi) =
+                    make_uint2(pack_e4m3x4(q[0], q[1], q[2], q[3]), pack_e4m3x4(q[4], q[5], q[6], q[7]));
+                if ((threadIdx.x & 15) == 0) p.x_scales[static_cast<int64_t>(t) * (p.hidden / 128) + vi / 16] = s;
+            } else if (on) {
                 const uint32_t bits = __float_as_uint(fmaxf(__fdiv_rn(amax, 448.f), 1e-4f));
                 const int e = static_cast<int>((bits >> 23) & 0xff) - 127 + ((bits & 0x7fffffu) ? 1 : 0);
                 const float inv = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
@@ -483,6 +519,7 @@ int fill_params(wuda::mhcpre::Params& p, const void* hidden_states, const float*
     p.hc_eps = hc_eps;
     p.rms_eps = rms_eps;
     p.norm_eps = norm_eps;
+    p.act_quant = 0;
     return WUDA_OK;
 }
 
@@ -508,12 +545,12 @@ int launch_mix(const wuda::mhcpre::Params& p, cudaStream_t stream) {
 
 }  // namespace
 
-extern "C" int wuda_mhc_pre(const void* hidden_states, const float* weight, const float* base, const float* scale,
-                            const void* attn_norm_gamma, float hc_eps, float rms_eps, float norm_eps, float* pre,
-                            float* post, float* comb, void* collapsed_bf16, void* normed_bf16, void* x_fp8,
-                            float* x_scales, void* workspace, int64_t workspace_bytes, int m, int hidden,
-                            void* stream) {
-    using namespace wuda;
+namespace wuda {
+
+int mhc_pre_as(bool act_quant, const void* hidden_states, const float* weight, const float* base, const float* scale,
+               const void* attn_norm_gamma, float hc_eps, float rms_eps, float norm_eps, float* pre, float* post, float* comb,
+               void* collapsed_bf16, void* normed_bf16, void* x_fp8, float* x_scales, void* workspace, int64_t workspace_bytes, int m,
+               int hidden, void* stream) {
     using namespace wuda::mhcpre;
     clear_error();
     WUDA_REQUIRE(weight && base && scale, "weight, base and scale are required");
@@ -521,6 +558,7 @@ extern "C" int wuda_mhc_pre(const void* hidden_states, const float* weight, cons
     int st = fill_params(p, hidden_states, weight, base, scale, attn_norm_gamma, hc_eps, rms_eps, norm_eps, pre, post, comb,
                          nullptr, collapsed_bf16, normed_bf16, x_fp8, x_scales, workspace, m, hidden);
     if (st != WUDA_OK) return st;
+    p.act_quant = act_quant;
     const int64_t need = wuda_mhc_pre_workspace_bytes(m, hidden);
     WUDA_REQUIRE(workspace_bytes >= need, "workspace holds %lld bytes; %lld are needed (wuda_mhc_pre_workspace_bytes)",
                  static_cast<long long>(workspace_bytes), static_cast<long long>(need));
@@ -528,6 +566,17 @@ extern "C" int wuda_mhc_pre(const void* hidden_states, const float* weight, cons
     if (st != WUDA_OK) return st;
     WUDA_CUDA(launch_pdl(mhc_pre_finish_kernel, dim3(m), dim3(kFinishLaunch), 0, static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
+}
+
+}  // namespace wuda
+
+extern "C" int wuda_mhc_pre(const void* hidden_states, const float* weight, const float* base, const float* scale,
+                            const void* attn_norm_gamma, float hc_eps, float rms_eps, float norm_eps, float* pre,
+                            float* post, float* comb, void* collapsed_bf16, void* normed_bf16, void* x_fp8,
+                            float* x_scales, void* workspace, int64_t workspace_bytes, int m, int hidden,
+                            void* stream) {
+    return wuda::mhc_pre_as(false, hidden_states, weight, base, scale, attn_norm_gamma, hc_eps, rms_eps, norm_eps, pre, post, comb,
+                            collapsed_bf16, normed_bf16, x_fp8, x_scales, workspace, workspace_bytes, m, hidden, stream);
 }
 
 extern "C" int wuda_mhc_pre_mix(const void* hidden_states, const float* weight, void* workspace, int64_t workspace_bytes,
