@@ -209,3 +209,32 @@ def test_bad_arguments(wuda):
     with pytest.raises(RuntimeError):
         wuda.rope_quant(x3, torch.zeros(2, dtype=torch.int32, device="cuda"), torch.zeros(8, 32, device="cuda"),
                         torch.zeros(8, 32, device="cuda"), 64)
+
+
+@pytest.mark.parametrize("tokens,heads,head_dim,rope_dim", [(1, 128, 512, 64), (2, 128, 192, 64), (25, 128, 192, 64), (37, 1, 128, 64),
+                                                            (149, 128, 192, 64), (297, 3, 128, 128), (5, 11, 384, 8), (3, 128, 640, 64)])
+@pytest.mark.parametrize("scale_fmt", [None, "ue8m0"])
+def test_rope_rows_cut_over_ctas(wuda, tokens, heads, head_dim, rope_dim, scale_fmt):
+    """A row is cut by its length and the number of tokens; every cut gives the bytes of the row computed in one piece, i.e. those
+    of torch's fp32 arithmetic with the same roundings."""
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn(tokens, heads, head_dim, generator=g, device="cuda").bfloat16()
+    x[0, 0, :128] = -0.0
+    pos = torch.randint(0, 512, (tokens,), generator=g, device="cuda")
+    ang = torch.randn(512, rope_dim // 2, generator=g, device="cuda") * 3
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    y16, y8, s = wuda.rope_quant(x, pos, cos, sin, rope_dim, scale_fmt=scale_fmt, return_bf16=True)
+    want = x.float()
+    tail = want[..., head_dim - rope_dim:]
+    re, im = tail[..., 0::2].clone(), tail[..., 1::2].clone()
+    c, d = cos[pos][:, None, :], sin[pos][:, None, :]
+    tail[..., 0::2], tail[..., 1::2] = re * c - im * d, re * d + im * c
+    want = want.bfloat16()
+    assert torch.equal(y16.view(torch.int16), want.view(torch.int16))
+    v = want.float().view(tokens, -1, 128)
+    scale = v.abs().amax(-1).clamp_min(1e-4) * torch.tensor(1.0 / 448, device="cuda")
+    if scale_fmt:
+        scale = torch.exp2(torch.ceil(torch.log2(scale.double()))).float()
+    assert torch.equal(s, scale)
+    codes = (v / scale[..., None]).clamp(-448, 448).view(tokens, -1).to(torch.float8_e4m3fn)
+    assert torch.equal(y8.view(torch.uint8), codes.view(torch.uint8))

@@ -57,23 +57,27 @@ __device__ __forceinline__ void quant_store8(const float (&v)[8], int pow2, uint
     const float s = group_scale(amax, pow2);
     float q[8];
     if (s < INFINITY) {
-        // v / s for eight v and one s: with r = 1/s correctly rounded, q0 = v r and the remainder v - q0 s (exact in an
-        // FMA), q0 + remainder * r is the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990) as long as the
+        // v / s for eight v and one s: with r = 1/s correctly rounded, q0 = v r and the remainder q0 s - v (exact in an
+        // FMA), q0 - remainder * r is the correctly rounded quotient (Markstein, IBM J. Res. Dev. 34, 1990) as long as the
         // remainder does not underflow; where it does, |v / s| is far below half of the smallest e4m3 value and the code is
-        // a zero of v's sign either way.  Three instructions per value instead of a division: RMSNorm + RoPE quantisation of
-        // 256 tokens (7168 + 24576 values each) 18.1 -> 15.4 us, of one token 7.7 -> 7.0.
+        // a zero of v's sign either way.  (With the remainder this way round a zero keeps its sign: of v = -0 it is +0, and
+        // -0 + -0 is -0.)  Three instructions per value instead of a division: RMSNorm + RoPE quantisation of
+        // 256 tokens (7168 + 24576 values each) 18.1 -> 15.4 us, of one token 7.7 -> 7.0.  A power of two has an exact
+        // reciprocal and needs the product alone.
         const float r = __frcp_rn(s);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const float q0 = __fmul_rn(v[i], r);
-            q[i] = copysignf(fmaf(fmaf(-q0, s, v[i]), r, q0), v[i]);     // (the sum of a negative zero and zero is positive)
+        for (int i = 0; i < 8; ++i) q[i] = __fmul_rn(v[i], r);
+        if (!pow2) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) q[i] = fmaf(-fmaf(q[i], s, -v[i]), r, q[i]);
         }
     } else {        // an infinite value in the group: v / inf
 #pragma unroll
         for (int i = 0; i < 8; ++i) q[i] = __fdiv_rn(v[i], s);
     }
+    // NaN becomes -448; the upper bound is the conversion's own (it saturates)
 #pragma unroll
-    for (int i = 0; i < 8; ++i) q[i] = fminf(fmaxf(q[i], -448.f), 448.f);
+    for (int i = 0; i < 8; ++i) q[i] = fmaxf(q[i], -448.f);
     uint2 packed;
     packed.x = pack_e4m3x4(q[0], q[1], q[2], q[3]);
     packed.y = pack_e4m3x4(q[4], q[5], q[6], q[7]);
@@ -112,19 +116,40 @@ struct NormParams {
 
 __global__ void __launch_bounds__(1024, 1) rmsnorm_quant_kernel(const NormParams p) {
     pdl_launch_dependents();
-    pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
     __shared__ float warp_part[32];
-    __shared__ float total;
     const int row = blockIdx.x;
     const int chunks = p.dim >> 3;                     // 16-byte chunks in the row
     const __nv_bfloat16* x = p.x + static_cast<int64_t>(row) * p.x_stride;
+    // The weights' way to L2 starts before the wait (a hint: nothing is read yet), and row and weights are one round of loads:
+    // 1 to 100 rows of 7168 4.6 -> 3.6 us, 256 rows 6.1 -> 5.2
+    const uint4* gamma = static_cast<const uint4*>(p.gamma);
+    if (p.gamma) {
+#pragma unroll
+        for (int c = 0; c < kMaxChunks; ++c) {
+            const int ch = c * blockDim.x + threadIdx.x;
+            if (ch < chunks) prefetch_l2(gamma + (p.gamma_is_bf16 ? ch : 2 * ch));
+        }
+    }
+    pdl_wait();   // nothing of global memory is read before the kernel ahead has finished
+    uint4 raw[kMaxChunks], g0[kMaxChunks], g1[kMaxChunks];
+#pragma unroll
+    for (int c = 0; c < kMaxChunks; ++c) {
+        const int ch = c * blockDim.x + threadIdx.x;
+        raw[c] = g0[c] = g1[c] = make_uint4(0u, 0u, 0u, 0u);
+        if (ch < chunks) {
+            raw[c] = *reinterpret_cast<const uint4*>(x + 8 * ch);
+            if (p.gamma) {
+                g0[c] = gamma[p.gamma_is_bf16 ? ch : 2 * ch];
+                if (!p.gamma_is_bf16) g1[c] = gamma[2 * ch + 1];
+            }
+        }
+    }
     float v[kMaxChunks][8];
     float ss = 0.f;
 #pragma unroll
     for (int c = 0; c < kMaxChunks; ++c) {
-        const int ch = c * blockDim.x + threadIdx.x;
-        if (ch < chunks) {
-            unpack8(*reinterpret_cast<const uint4*>(x + 8 * ch), v[c]);
+        unpack8(raw[c], v[c]);
+        if (c * blockDim.x + threadIdx.x < chunks) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) ss = fmaf(v[c][i], v[c][i], ss);
         }
@@ -135,13 +160,11 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_quant_kernel(const NormParams
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if ((threadIdx.x & 31) == 0) warp_part[threadIdx.x >> 5] = ss;
         __syncthreads();
-        if (threadIdx.x < 32) {
-            float t = threadIdx.x < (blockDim.x >> 5) ? warp_part[threadIdx.x] : 0.f;
+        // (every warp adds the warps' sums itself, all in the same order)
+        const int lane = threadIdx.x & 31;
+        float total = lane < (blockDim.x >> 5) ? warp_part[lane] : 0.f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-            if (threadIdx.x == 0) total = t;
-        }
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         rs = __fdiv_rn(1.0f, __fsqrt_rn(total / static_cast<float>(p.dim) + p.eps));
     }
 #pragma unroll
@@ -151,12 +174,11 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_quant_kernel(const NormParams
             if (p.gamma) {
                 float g[8];
                 if (p.gamma_is_bf16) {
-                    unpack8(*reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(p.gamma) + 8 * ch), g);
+                    unpack8(g0[c], g);
                 } else {
-                    const float4* g4 = reinterpret_cast<const float4*>(static_cast<const float*>(p.gamma) + 8 * ch);
-                    const float4 a = g4[0], b = g4[1];
-                    g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
-                    g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
+                    const uint32_t w[8] = {g0[c].x, g0[c].y, g0[c].z, g0[c].w, g1[c].x, g1[c].y, g1[c].z, g1[c].w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) g[i] = __uint_as_float(w[i]);
                 }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[c][i] = bf16_round(__fmul_rn(g[i], __fmul_rn(v[c][i], rs)));
@@ -171,6 +193,12 @@ __global__ void __launch_bounds__(1024, 1) rmsnorm_quant_kernel(const NormParams
     }
 }
 
+// A CTA of 256 threads takes one round of two chunks per thread and is gone: five fit on an SM, and the loads of the next overlap the
+// arithmetic of the ones there.  (Four chunks per thread in one wave of CTAs loaded in step and computed in step: 64 / 256 tokens of
+// 128 heads x 192 4.6 -> 4.3 / 10.2 -> 9.2 us, x 512 6.7 -> 5.6 / 21.0 -> 17.4; with four or six CTAs per SM 4.1 / 9.2, 5.7 / 18.5 and
+// 4.3 / 9.6, 6.6 / 18.0.)
+constexpr int kRopeThreads = 256, kRopeDepth = 2;
+
 struct RopeParams {
     const __nv_bfloat16* x;
     const int64_t* positions;
@@ -182,7 +210,7 @@ struct RopeParams {
     int tokens, heads, head_dim, rope_dim, max_pos, inverse, pow2;
 };
 
-__global__ void __launch_bounds__(1024) rope_quant_kernel(const RopeParams p) {
+__global__ void __launch_bounds__(kRopeThreads, 5) rope_quant_kernel(const RopeParams p) {
     pdl_launch_dependents();
     pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
     const int t = blockIdx.x;
@@ -197,20 +225,20 @@ __global__ void __launch_bounds__(1024) rope_quant_kernel(const RopeParams p) {
     // every thread of a 16-thread quantisation group runs the same number of iterations
     // (width is a multiple of 128), so the shuffles inside quant_store8 are convergent
     // (blockIdx.y splits a token's chunks over several CTAs when there are few tokens)
-    // four 16-byte loads of a thread are in flight before the first is used: the kernel is a few MB of latency
+    // (the 16-byte loads of a thread's chunks are in flight before the first is used)
     const int stride = blockDim.x * gridDim.y;
     const bool table16 = ((reinterpret_cast<uintptr_t>(p.cos_t) | reinterpret_cast<uintptr_t>(p.sin_t)) & 15u) == 0;
     // a chunk's place inside its head, carried from chunk to chunk instead of a remainder per chunk (with the tables read 16
     // bytes at a time: norm + RoPE quantisation of 256 tokens 15.4 -> 14.8 us)
     const int head_step = 8 * stride % p.head_dim;
     int in_head = 8 * (blockIdx.y * blockDim.x + threadIdx.x) % p.head_dim;
-    for (int ch0 = blockIdx.y * blockDim.x + threadIdx.x; ch0 < chunks; ch0 += 4 * stride) {
-        uint4 raw[4];
+    for (int ch0 = blockIdx.y * blockDim.x + threadIdx.x; ch0 < chunks; ch0 += kRopeDepth * stride) {
+        uint4 raw[kRopeDepth];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < kRopeDepth; ++u)
             raw[u] = ch0 + u * stride < chunks ? *reinterpret_cast<const uint4*>(x + 8 * (ch0 + u * stride)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < kRopeDepth; ++u) {
             const int ch = ch0 + u * stride;
             if (ch >= chunks) break;                 // uniform over a 16-thread group
             float v[8];
@@ -360,13 +388,15 @@ extern "C" int wuda_rope_quant_fp8(const void* x_bf16, const int64_t* positions,
     p.inverse = inverse;
     p.pow2 = scale_mode;
     const int chunks = heads * head_dim / 8;
-    // CTAs of 256 threads, each thread four 16-byte chunks per round; a token's row is cut over as many CTAs as keep
-    // the whole launch within one resident wave (a quantisation group is 16 consecutive threads, so any multiple of
-    // the block size is a valid cut, and whole 16-thread groups stay in step)
-    const int threads = chunks < 256 ? (chunks + 31) / 32 * 32 : 256;
-    int splits = 1;
-    const int rounds = (chunks + 4 * threads - 1) / (4 * threads);
-    while (splits < rounds && tokens * splits * 2 <= 5 * 148) splits *= 2;
+    // A row is cut over as many CTAs as it has rounds of kRopeDepth 16-byte chunks per thread (a quantisation group is 16
+    // consecutive threads, so any multiple of the block size is a valid cut, and whole 16-thread groups stay in step).  With
+    // few tokens it is cut further, down to a chunk per thread, up to two CTAs per SM: one token of 128 heads x 192 / x 512
+    // 3.6 -> 2.6 / 4.0 -> 2.6 us.
+    const int threads = chunks < kRopeThreads ? (chunks + 31) / 32 * 32 : kRopeThreads;
+    const int rounds = (chunks + kRopeDepth * threads - 1) / (kRopeDepth * threads), most = (chunks + threads - 1) / threads;
+    const int few = 2 * 148 / tokens < most ? 2 * 148 / tokens : most;
+    int splits = rounds > few ? rounds : few;
+    if (splits > 65535) splits = 65535;      // (the loop takes what is left)
     WUDA_CUDA(launch_pdl(rope_quant_kernel, dim3(dim3(tokens, splits)), dim3(threads), 0, static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
 }
