@@ -3,6 +3,9 @@
 nvcc cross-compiles without a GPU, so this runs anywhere the CUDA toolkit is present.
 The library links the static CUDA runtime and resolves the one driver function it needs
 (cuTensorMapEncodeTiled) at run time, so it also loads where no driver is installed.
+
+wuda_b200/_fast.so (csrc/fast_ops.cpp, g++) is the operators' native call path from Python; it is built against the installed
+torch and loads the library's entry points by name.
 """
 import os
 import subprocess
@@ -11,6 +14,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libwuda_b200.so")
+FAST = os.path.join(HERE, "_fast.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -29,6 +33,24 @@ def headers():
     hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
     hs.append(os.path.join(HERE, "..", "include", "wuda_b200.h"))
     return hs
+
+
+def build_fast(force=False):
+    src = os.path.join(CSRC, "fast_ops.cpp")
+    newest = max(os.path.getmtime(p) for p in (src, os.path.join(HERE, "..", "include", "wuda_b200.h")))
+    if not force and os.path.exists(FAST) and os.path.getmtime(FAST) >= newest:
+        return FAST
+    import sysconfig
+    import torch
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    cmd = ([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+            "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI] +
+           ["-I" + p for p in (root + "/include", root + "/include/torch/csrc/api/include", cuda + "/include",
+                               sysconfig.get_paths()["include"])] +
+           [src, "-o", FAST, "-L" + root + "/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+    subprocess.check_call(cmd)
+    return FAST
 
 
 def build(force=False, verbose=False):
@@ -51,6 +73,7 @@ def build(force=False, verbose=False):
     if procs or not os.path.exists(LIB):
         cmd = [nvcc, "-shared", "-o", LIB] + objs + ["-Xcompiler", "-fPIC", "-gencode", "arch=compute_100a,code=sm_100a"]
         subprocess.check_call(cmd)
+    build_fast(force)
     return LIB
 
 

@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from . import _lib
+from . import _fast, _lib
 from ._lib import WudaError, check, lib
 from .scratch import Scratch
 
@@ -21,13 +21,16 @@ __all__ = ["mqa_logits_fp4_decode_out", "mqa_logits_fp4_decode", "mqa_logits_fp8
            "fp4_gemm", "fp4_act_quant", "hc_split_sinkhorn", "head_ssq_standalone", "idx_postprocess_standalone",
            "idx_postprocess_fp8_standalone", "mqa_compressor_standalone", "mqa_compressor_paged", "topk_v2_plan"]
 
+# The operators that a server calls by themselves try csrc/fast_ops.cpp first: checks, outputs and launch in one native call,
+# which does nothing and returns None for whatever it does not know or would have to refuse.
+_fast.bind(lib._handle)
+
 NUM_INDEX_HEADS = 64
 INDEX_HEAD_DIM = 128
 
 
 def _stream():
-    # the handle of torch.cuda.current_stream() without the Stream object around it: 0.2 us instead of 3.2 us per call, of
-    # the 14-18 us that an operator called directly costs the host (allocations and checks included)
+    # the handle of torch.cuda.current_stream() without the Stream object around it: 0.2 us instead of 3.2 us per call
     return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
@@ -63,6 +66,10 @@ def mqa_logits_fp8_decode_out(q, kv_cache, weights, context_lens, block_table, s
     rows per request; rows b*next_n .. b*next_n+next_n-1 share block_table[b].
     Positions t >= context are not written.
     """
+    done = _fast.mqa_logits_fp8(q, kv_cache, weights, context_lens, block_table, logits, kv_entries_per_block,
+                                kv_block_stride_bytes, next_n, status_word)
+    if done is not None:
+        return done
     _require(q.is_cuda and q.is_contiguous() and q.dtype == torch.float8_e4m3fn and q.dim() == 3
              and q.size(1) == NUM_INDEX_HEADS and q.size(2) == INDEX_HEAD_DIM,
              "q must be contiguous CUDA FP8 [R,64,128]")
@@ -115,6 +122,10 @@ def mqa_logits_fp4_decode_out(q, sf_q, kv_cache, weights, context_lens, block_ta
     [B, 64, 64] packed e2m1, sf_q int32 [B, 64] (four ue8m0 bytes), kv_cache uint8 [num_blocks, stride] of fused
     pages (keys, then scale words), weights fp32 [B, 64], context_lens int32 [B], block_table int32 [B, pages],
     logits fp32 [B, >= max_context_len]; only t < context is written."""
+    done = _fast.mqa_logits_fp4(q, sf_q, kv_cache, weights, context_lens, block_table, logits, max_context_len,
+                                kv_entries_per_block, kv_block_stride_bytes, status_word)
+    if done is not None:
+        return done
     _require(q.is_cuda and q.is_contiguous() and q.element_size() == 1 and q.dim() == 3 and q.shape[1:] == (64, 64),
              "q must be contiguous CUDA int8 [B, 64, 64]")
     b = q.size(0)
@@ -159,6 +170,9 @@ def topk_v2_transform(scores, seq_lens, page_table, page_indices, page_size=64, 
     reference's plan tensor) is accepted and ignored.  Never allocates.
     `rows_per_table_row` (keyword, default 1 as in the reference) lets the next_n score
     rows of one request share that request's page-table row."""
+    done = _fast.topk(scores, seq_lens, page_table, page_indices, page_size, raw_indices, rows_per_table_row)
+    if done is not None:
+        return done
     _require(scores.is_cuda and scores.dtype == torch.float32 and scores.dim() == 2 and scores.stride(1) == 1,
              "scores must be CUDA FP32 [rows, L] with unit inner stride")
     rows = scores.size(0)
@@ -250,6 +264,9 @@ def rmsnorm_quant(x, gamma, eps=1e-6, *, quant=True, scale_fmt=None, return_bf16
     FP8 quantisation.  Returns (y_bf16 or None, y_fp8 or None, scales or None).
     scale_fmt: None = fp32 amax/448 scales, anything else = power-of-two scales, as the
     origin's act_quant (origin/kernel.py:105-125).  gamma None = no normalisation."""
+    done = _fast.rmsnorm_quant(x, gamma, eps, quant, scale_fmt, return_bf16)
+    if done is not None:
+        return done
     _require(x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.stride(1) == 1,
              "x must be CUDA bf16 [rows, dim] with unit inner stride")
     rows, dim = x.shape
@@ -272,6 +289,9 @@ def act_quant(x, block_size=128, scale_fmt=None):
     """Block-wise FP8 quantisation with the origin's signature (origin/kernel.py:105):
     returns (y float8_e4m3fn, scales fp32 [..., N/128])."""
     _require(block_size == 128, "block_size must be 128")
+    done = _fast.act_quant(x, scale_fmt)
+    if done is not None:
+        return done
     shape = x.shape
     _, y8, sc = rmsnorm_quant(x.reshape(-1, shape[-1]), None, quant=True, scale_fmt=scale_fmt, return_bf16=False)
     return y8.view(shape), sc.view(*shape[:-1], shape[-1] // 128)
@@ -282,6 +302,9 @@ def rope_quant(x, positions, cos_table, sin_table, rope_dim, *, inverse=False, q
     """Partial RoPE of bf16 [tokens, heads, head_dim] (last rope_dim dims of each head) and,
     in the same pass, 1x128 FP8 quantisation of the flat row.  Returns (y_bf16 or None,
     y_fp8 [tokens, heads*head_dim] or None, scales or None)."""
+    done = _fast.rope_quant(x, positions, cos_table, sin_table, rope_dim, inverse, quant, scale_fmt, return_bf16)
+    if done is not None:
+        return done
     _require(x.is_cuda and x.is_contiguous() and x.dtype == torch.bfloat16 and x.dim() == 3,
              "x must be contiguous CUDA bf16 [tokens, heads, head_dim]")
     tokens, heads, head_dim = x.shape
@@ -378,6 +401,10 @@ def sparse_mla_decode(q, swa_cache, swa_indices, swa_lengths, cmp_cache=None, cm
     swa_indices[b] in swa_cache, then cmp_lengths[b] entries of cmp_indices[b] in cmp_cache (pool entry
     indices, negative = skipped), with the attention sink in the denominator.  Returns bf16
     [batch, heads, 512]."""
+    done = _fast.sparse_mla_decode(q, swa_cache, swa_indices, swa_lengths, cmp_cache, cmp_indices, cmp_lengths, attn_sink,
+                                   softmax_scale, out, status_word, split, _mla_scratch._streams)
+    if done is not None:
+        return done
     _require(q.is_cuda and q.is_contiguous() and q.dtype == torch.bfloat16 and q.dim() == 3 and q.size(2) == 512,
              "q must be contiguous CUDA bf16 [batch, heads, 512]")
     batch, heads = q.size(0), q.size(1)
@@ -722,6 +749,9 @@ def fp4_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
     """C[M,N] = A_fp8[M,K] @ B_fp4[N,K]^T with the origin's signature (origin/kernel.py:518-536): a e4m3, a_s one
     POWER-OF-TWO scale per row and 128 K-elements (fp32 or float8_e8m0fnu: act_quant with scale_fmt "ue8m0"), b
     float4_e2m1fn_x2 [N, K/2], b_s float8_e8m0fnu [N, K/32].  bf16 output."""
+    done = _fast.fp4_gemm(a, a_s, b, b_s, out, status_word, _gemm_scratch._streams)
+    if done is not None:
+        return done
     _require(a.is_cuda and a.is_contiguous() and a.dtype == torch.float8_e4m3fn, "a must be contiguous CUDA e4m3")
     _require(b.is_cuda and b.is_contiguous() and b.element_size() == 1 and b.dim() == 2,
              "b must be contiguous CUDA float4_e2m1fn_x2 (or bytes) [N, K/2]")
@@ -770,6 +800,9 @@ def fp8_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
     output: the origin's fp8_gemm(a, a_s, b, b_s) (origin/kernel.py:257-273).  pow2_scales=True promises that
     every scale is a power of two (the reference's UE8M0 scales) and takes the kernel that applies them inside
     the tensor core."""
+    done = _fast.fp8_gemm(a, a_s, b, b_s, out, status_word, pow2_scales, _gemm_scratch._streams)
+    if done is not None:
+        return done
     if a_s.dtype != torch.float32 and b_s.dtype != torch.float32:    # float8_e8m0fnu scales: powers of two by type
         pow2_scales = True
     a_s, b_s = _scales_as_fp32(a_s, "a_s"), _scales_as_fp32(b_s, "b_s")
@@ -796,6 +829,9 @@ def fp8_gemm(a, a_s, b, b_s, scale_dtype=torch.float32, *, out=None, status_word
 def bf16_gemm(a, w, *, out=None, out_dtype=torch.bfloat16, status_word=None):
     """C[M,N] = A[M,K] @ W[N,K]^T on bf16 operands with fp32 accumulation; bf16 or fp32 output
     (the origin's `linear` on bf16 weights, origin/model.py:108-120)."""
+    done = _fast.bf16_gemm(a, w, out, out_dtype, status_word, _gemm_scratch._streams)
+    if done is not None:
+        return done
     _require(a.is_cuda and a.is_contiguous() and a.dtype == torch.bfloat16, "a must be contiguous CUDA bf16")
     _require(w.is_cuda and w.is_contiguous() and w.dtype == torch.bfloat16 and w.dim() == 2,
              "w must be contiguous CUDA bf16 [N, K]")
@@ -971,6 +1007,10 @@ def nvfp4_gemm(a, a_sf_packed, a_global_scale, w, w_sf_packed, w_global_scale, *
     """bf16 C[M,N] = NVFP4 A[M,K] @ W[N,K]^T: a, w packed e2m1 uint8 [rows, K/2]; *_sf_packed the
     ue4m3 block scales in tensor-core order (wuda_b200.workloads.pack_nvfp4_scales); one fp32
     scale per tensor."""
+    done = _fast.nvfp4_gemm(a, a_sf_packed, a_global_scale, w, w_sf_packed, w_global_scale, out, status_word,
+                            _gemm_scratch._streams)
+    if done is not None:
+        return done
     _require(a.is_cuda and a.is_contiguous() and a.dtype == torch.uint8 and a.dim() == 2, "a must be CUDA uint8 [M, K/2]")
     _require(w.is_cuda and w.is_contiguous() and w.dtype == torch.uint8 and w.dim() == 2 and w.size(1) == a.size(1),
              "w must be CUDA uint8 [N, K/2]")
