@@ -150,6 +150,21 @@ __device__ __forceinline__ uint4 bf16x8_to_f16x8(uint4 v) {
     return make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
 }
 
+// 16 bytes global -> shared, or zeros where there is nothing to read
+__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, bool valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+// Where 16-byte piece i of a row of kRowBytes lies in a staging area: consecutive rows' equal pieces in different banks.
+template <uint32_t kRowBytes>
+__device__ __forceinline__ uint32_t staged(uint32_t base, int row, int piece) {
+    return base + row * kRowBytes + ((piece ^ (row & 7)) << 4);
+}
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                  : "memory");
@@ -267,57 +282,74 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
     const int first = static_cast<int>(blockIdx.z) * per_split;
     const int blocks = min(max(all_blocks - first, 0), per_split);
 
+    // Records are requested kAhead passes before they are converted: a gather from random pages takes far longer than a pass's
+    // turn through the pipeline.  The first ones are on their way while the query is laid out.
+    const bool producer = warp >= kSoftmaxWarps && warp < kIssuerWarp;
+    const int pw = warp - kSoftmaxWarps, row = pw * 4 + (lane >> 3), piece = lane & 7, first_key = first * kBlock;
+    int idx[kAhead + 1];
+    if (producer) {
+#pragma unroll
+        for (int u = 0; u <= kAhead; ++u) idx[u] = fetch_index(p, b, first_key + u * kPass + row, n_swa, n_total);
+    }
+    // The query rows, zero-padded to 128, come in as they lie, 16 bytes per lane and whole lines per warp: rotary dims to their
+    // place in the swizzled K-major operand layout, where the lane that brought a piece converts it, scaled dims to the (still
+    // unused) key stages, from where a row's thread takes them to tensor memory (row = lane, column = a pair of dims).  (A row
+    // per thread straight from global memory touches 32 lines with every load: one request of 1152 keys, the first block's
+    // scores 14.7 -> 9.5 us after the CTA's start, with the records asked for ahead of it.)
+    const uint8_t* q_bytes = reinterpret_cast<const uint8_t*>(p.q + static_cast<int64_t>(b) * p.heads * kDim);
+    for (int i = threadIdx.x; i < kRows * (kDim / 8); i += kThreads) {
+        const int r = i / (kDim / 8), at = i % (kDim / 8), c = at >> 3;
+        const uint32_t dst = c < kQTmemChunks ? base + kOffOwn + c * kQChunk : base + kOffQ + (c - kQTmemChunks) * kQChunk;
+        cp_async_16(staged<128>(dst, r, at & 7), r < p.heads ? q_bytes + static_cast<int64_t>(i) * 16 : q_bytes, r < p.heads);
+    }
+    KeyRegs ring[kAhead + 1];
+    bool bad = false;
+    int next_idx = -1;
+    if (producer) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) fetch_key(p, first_key + u * kPass + row, n_swa, idx[u], piece, ring[u], &bad);
+        next_idx = idx[kAhead];
+    }
+    cp_async_wait_all();
+    for (int i = threadIdx.x; i < kRows * (kDim / 8); i += kThreads) {
+        const int r = i / (kDim / 8), at = i % (kDim / 8), c = at >> 3;
+        if (c < kQTmemChunks) continue;
+        const uint32_t mine = staged<128>(base + kOffQ + (c - kQTmemChunks) * kQChunk, r, at & 7);
+        st_shared_v4(mine, bf16x8_to_f16x8(ld_shared_v4(mine)));
+    }
     tc_fence_before();
-    __syncthreads();   // the tensor-memory base address is published
+    __syncthreads();   // the tensor-memory base address is published, the query has arrived
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    // the query rows, zero-padded to 128: rotary dims to shared memory in the swizzled K-major operand
-    // layout, scaled dims to tensor memory (row = lane, column = a pair of dims)
-    constexpr int kQSmemPieces = (8 - kQTmemChunks) * 8;
-    for (int i = threadIdx.x; i < kRows * kQSmemPieces; i += kThreads) {
-        const int row = i / kQSmemPieces, piece = i % kQSmemPieces;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row < p.heads)
-            v = __ldg(reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(b) * p.heads + row) * kDim +
-                                                     kQTmemChunks * 64) + piece);
-        st_shared_v4(base + kOffQ + (piece >> 3) * kQChunk + row * 128 + (((piece & 7) ^ (row & 7)) << 4), bf16x8_to_f16x8(v));
-    }
-    if (warp < kSoftmaxWarps) {
-        const int row = warp * 32 + lane;
-        const uint4* src = reinterpret_cast<const uint4*>(p.q + (static_cast<int64_t>(b) * p.heads + row) * kDim);
+    {   // three warps per quarter of the lanes, two chunks each
+        static_assert(kQTmemChunks == 6 && kIssuerWarp == 12, "chunks per warp");
+        if (warp < kIssuerWarp) {
+            const int quarter = warp & 3;
 #pragma unroll 1
-        for (int c = 0; c < kQTmemChunks; ++c) {
-            uint32_t w[32];
+            for (int c2 = 0; c2 < 4; ++c2) {
+                const int c = (warp >> 2) * 2 + (c2 >> 1);
+                uint32_t w[16];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const uint4 v = bf16x8_to_f16x8(row < p.heads ? __ldg(src + c * 8 + i) : make_uint4(0, 0, 0, 0));
-                w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+                for (int i = 0; i < 4; ++i) {
+                    const uint4 v = bf16x8_to_f16x8(
+                        ld_shared_v4(staged<128>(base + kOffOwn + c * kQChunk, quarter * 32 + lane, (c2 & 1) * 4 + i)));
+                    w[4 * i] = v.x, w[4 * i + 1] = v.y, w[4 * i + 2] = v.z, w[4 * i + 3] = v.w;
+                }
+                tmem_st_32x16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + kColQ + c * 32 + (c2 & 1) * 16, w);
             }
-            tmem_st_32x32(tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + kColQ + c * 32, w);
+            tmem_st_wait();
         }
-        tmem_st_wait();
     }
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
 
-    if (warp >= kSoftmaxWarps && warp < kIssuerWarp) {
+    if (producer) {
         // ------------------------------------------------------------ key producers
-        const int pw = warp - kSoftmaxWarps;
-        const int row = pw * 4 + (lane >> 3), piece = lane & 7;
-        bool bad = false, clamped = false;
-        // a block's records are requested kAhead blocks before they are converted: a gather from
-        // random pages takes far longer than one block's turn through the pipeline
-        KeyRegs ring[kAhead + 1];
+        bool clamped = false;
         constexpr int kPasses = kBlock / kPass;
-        const int passes = blocks * kPasses, first_key = first * kBlock;
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-            const int g = first_key + u * kPass + row;
-            fetch_key(p, g, n_swa, fetch_index(p, b, g, n_swa, n_total), piece, ring[u], &bad);
-        }
-        int next_idx = fetch_index(p, b, first_key + kAhead * kPass + row, n_swa, n_total);
+        const int passes = blocks * kPasses;
         bool alive = true;
         for (int q0 = 0; q0 < passes && alive; q0 += kAhead + 1) {
 #pragma unroll
@@ -521,6 +553,10 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         if (alive && blocks > 0)
             alive = mbar_wait_warp(pv_done + ((blocks - 1) & 1) * 8, ((blocks - 1) >> 1) & 1u, abort_flag, p.status,
                                    kDevTimeoutMlaOutput);
+        // The output rows wait in shared memory (nothing reads the key stages any more), from where all warps store them whole
+        // lines at a time: a row per thread straight to global memory touches 32 lines with every instruction (128 KB of partial
+        // sums 5.4 -> 2.4 us).
+        const uint32_t out_addr = base + kOffOwn;
         if (alive && gridDim.z > 1) {
             // partial result of this run of blocks: the unnormalised sums with their reference maximum
             tc_fence_after();
@@ -530,17 +566,14 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
                 p.part_ml[slot * 2 + 1] = blocks > 0 ? l : 0.0f;
             }
             if (blocks > 0) {   // the combine step skips partials whose maximum is -inf
-                float* dst = p.part_o + slot * kDim + half * kHalf;
 #pragma unroll 1
                 for (int c = 0; c < kHalf; c += 32) {
                     uint32_t o[32];
                     tmem_ld_32x32(lane_addr + kColO + c, o);
                     tmem_ld_wait();
-                    if (row < p.heads) {
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4)
-                            *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
-                    }
+                    for (int i = 0; i < 32; i += 4)
+                        st_shared_v4(staged<kHalf * 4>(out_addr, row, (c + i) / 4), make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]));
                 }
             }
             tc_fence_before();
@@ -552,7 +585,6 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
                 const float sink = (p.sink && row < p.heads) ? ex2(__ldg(p.sink + row) * kLog2e - m_ref) : 0.0f;
                 inv = 1.0f / (l + sink);   // an overwhelming sink gives 1 / inf = 0
             }
-            __nv_bfloat16* dst = p.out + (static_cast<int64_t>(b) * p.heads + row) * kDim + half * kHalf;
 #pragma unroll 1
             for (int c = 0; c < kHalf; c += 32) {
                 uint32_t o[32];
@@ -560,19 +592,17 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
                     tmem_ld_32x32(lane_addr + kColO + c, o);
                     tmem_ld_wait();
                 }
-                if (row < p.heads) {
 #pragma unroll
-                    for (int i = 0; i < 32; i += 8) {
-                        uint32_t w[4];
+                for (int i = 0; i < 32; i += 8) {
+                    uint32_t w[4];
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            const float lo = any ? __uint_as_float(o[i + 2 * k]) * inv : 0.0f;
-                            const float hi = any ? __uint_as_float(o[i + 2 * k + 1]) * inv : 0.0f;
-                            const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                            w[k] = *reinterpret_cast<const uint32_t*>(&h);
-                        }
-                        *reinterpret_cast<uint4*>(dst + c + i) = make_uint4(w[0], w[1], w[2], w[3]);
+                    for (int k = 0; k < 4; ++k) {
+                        const float lo = any ? __uint_as_float(o[i + 2 * k]) * inv : 0.0f;
+                        const float hi = any ? __uint_as_float(o[i + 2 * k + 1]) * inv : 0.0f;
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                        w[k] = *reinterpret_cast<const uint32_t*>(&h);
                     }
+                    st_shared_v4(staged<kHalf * 2>(out_addr, row, (c + i) / 8), make_uint4(w[0], w[1], w[2], w[3]));
                 }
             }
             tc_fence_before();
@@ -580,6 +610,24 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
     }
 
     __syncthreads();
+    if (!*abort_flag) {
+        const int heads = p.heads;
+        if (gridDim.z > 1) {
+            float* dst = p.part_o + (static_cast<int64_t>(b) * gridDim.z + blockIdx.z) * heads * kDim + half * kHalf;
+            constexpr int kPieces = kHalf / 4;
+#pragma unroll 6
+            for (int i = threadIdx.x; blocks > 0 && i < heads * kPieces; i += kThreads)
+                *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(i / kPieces) * kDim + i % kPieces * 4) =
+                    ld_shared_v4(staged<kHalf * 4>(base + kOffOwn, i / kPieces, i % kPieces));
+        } else {
+            __nv_bfloat16* dst = p.out + static_cast<int64_t>(b) * heads * kDim + half * kHalf;
+            constexpr int kPieces = kHalf / 8;
+#pragma unroll 6
+            for (int i = threadIdx.x; i < heads * kPieces; i += kThreads)
+                *reinterpret_cast<uint4*>(dst + static_cast<int64_t>(i / kPieces) * kDim + i % kPieces * 8) =
+                    ld_shared_v4(staged<kHalf * 2>(base + kOffOwn, i / kPieces, i % kPieces));
+        }
+    }
     if (*abort_flag) abort_drain_sleep();
     __syncthreads();
     if (warp == kIssuerWarp) {
@@ -594,19 +642,34 @@ __global__ void __launch_bounds__(128) sparse_mla_combine_kernel(const Params p,
     pdl_wait();
     const int h = blockIdx.x, b = blockIdx.y;
     const int64_t first = (static_cast<int64_t>(b) * splits) * p.heads + h;
-    float m = -INFINITY;
-    for (int z = 0; z < splits; ++z) m = fmaxf(m, p.part_ml[(first + static_cast<int64_t>(z) * p.heads) * 2]);
+    // lane z holds the reference maximum and the sum of partial z (at most 32 of them); the rows come four at a time
+    const int lane = threadIdx.x & 31;
+    float mine_m = -INFINITY, mine_l = 0.0f;
+    if (lane < splits) {
+        const float2 ml = *reinterpret_cast<const float2*>(p.part_ml + (first + static_cast<int64_t>(lane) * p.heads) * 2);
+        mine_m = ml.x, mine_l = ml.y;
+    }
+    float m = mine_m;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     float den = 0.0f;
     if (m != -INFINITY) {
-        for (int z = 0; z < splits; ++z) {
-            const int64_t slot = first + static_cast<int64_t>(z) * p.heads;
-            const float mz = p.part_ml[slot * 2];
-            if (mz == -INFINITY) continue;
-            const float w = ex2(mz - m);
-            den += w * p.part_ml[slot * 2 + 1];
-            const float4 o = *reinterpret_cast<const float4*>(p.part_o + slot * kDim + threadIdx.x * 4);
-            acc.x += w * o.x, acc.y += w * o.y, acc.z += w * o.z, acc.w += w * o.w;
+        const uint32_t live = __ballot_sync(0xffffffffu, mine_m != -INFINITY);
+        for (int z0 = 0; z0 < splits; z0 += 4) {
+            float4 o[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if ((live >> (z0 + i)) & 1u)
+                    o[i] = *reinterpret_cast<const float4*>(p.part_o + (first + static_cast<int64_t>(z0 + i) * p.heads) * kDim + threadIdx.x * 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float mz = __shfl_sync(0xffffffffu, mine_m, z0 + i), lz = __shfl_sync(0xffffffffu, mine_l, z0 + i);
+                if (!((live >> (z0 + i)) & 1u)) continue;
+                const float w = ex2(mz - m);
+                den += w * lz;
+                acc.x += w * o[i].x, acc.y += w * o[i].y, acc.z += w * o[i].z, acc.w += w * o[i].w;
+            }
         }
         if (p.sink) den += ex2(__ldg(p.sink + h) * kLog2e - m);
     }
