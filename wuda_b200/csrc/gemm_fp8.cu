@@ -420,8 +420,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < kHalf; i += 4)
                         if (c0 + i < p.M) __stcg(slot + (c0 + i) / 4 * kTileN, make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]));
-                    __threadfence();
-                    epi_bar_sync();
+                    epi_bar_sync();     // (the flag's release covers what the barrier orders before it: gemm_tc.cuh)
                 }
                 if (p.sliced) {
                     // (the last arrival wraps the tile's counter back to zero: gemm_tc.cuh)
@@ -434,22 +433,33 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                         alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                         const int last = alive ? *last_peer_slot : cta_of(units, (last_tile + 1) * p.kb - 1, gridDim.x);
                         if (alive) {
-                            for (int c = blockIdx.x + 1; c <= last; ++c) {
+                            // (the next partial's loads are in flight while one is added, where the registers hold two)
+                            constexpr bool kTwo = kHalf <= 32;
+                            constexpr int kPiece = kHalf < 32 ? kHalf : 32;
+                            auto fetch = [&](int c, int i0, float4 (&v)[kPiece / 4]) {
                                 const float4* peer = reinterpret_cast<const float4*>(p.scratch + static_cast<int64_t>(c) * kSlotFloats) + row_in_tile;
-                                constexpr int kPiece = kHalf < 32 ? kHalf : 32;
 #pragma unroll
-                                for (int i0 = 0; i0 < kHalf; i0 += kPiece)
-                                    if (c0 + i0 < p.M) {
-                                        float4 v[kPiece / 4];
+                                for (int i = 0; i < kPiece / 4; ++i) v[i] = __ldcg(peer + ((c0 + i0) / 4 + i) * kTileN);
+                            };
 #pragma unroll
-                                        for (int i = 0; i < kPiece / 4; ++i) v[i] = __ldcg(peer + ((c0 + i0) / 4 + i) * kTileN);
+                            for (int i0 = 0; i0 < kHalf; i0 += kPiece)
+                                if (c0 + i0 < p.M) {
+                                    float4 v[2][kPiece / 4];
+                                    if (kTwo) fetch(blockIdx.x + 1, i0, v[0]);
+                                    for (int c = blockIdx.x + 1; c <= last; c += 2) {
 #pragma unroll
-                                        for (int i = 0; i < kPiece / 4; ++i) {
-                                            acc[i0 + 4 * i] += v[i].x, acc[i0 + 4 * i + 1] += v[i].y;
-                                            acc[i0 + 4 * i + 2] += v[i].z, acc[i0 + 4 * i + 3] += v[i].w;
+                                        for (int h = 0; h < 2; ++h) {
+                                            if (c + h > last) break;
+                                            if (!kTwo) fetch(c + h, i0, v[h]);
+                                            else if (c + h < last) fetch(c + h + 1, i0, v[h ^ 1]);
+#pragma unroll
+                                            for (int i = 0; i < kPiece / 4; ++i) {
+                                                acc[i0 + 4 * i] += v[h][i].x, acc[i0 + 4 * i + 1] += v[h][i].y;
+                                                acc[i0 + 4 * i + 2] += v[h][i].z, acc[i0 + 4 * i + 3] += v[h][i].w;
+                                            }
                                         }
                                     }
-                            }
+                                }
                         }
                         if (!alive) poison();
                         epi_bar_sync();

@@ -717,7 +717,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
 #pragma unroll
                 for (int c = 0; c < kCols; c += 4)
                     if (col0 + c < p.M) __stcg(slot + (col0 + c) / 4 * kTileN, make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]));
-                __threadfence();
+                // The barrier orders all threads' stores before the one thread's release of the flag or counter behind it, which
+                // covers them all: a fence of every thread's own in between held up the tail of short calls by 0.7 us.
                 epi_sync();
             }
             if (p.sliced) {
