@@ -142,6 +142,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, p.a_rows));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 4);
     volatile int* last_peer_slot = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 8);
+    volatile int* arrived_last = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 12);
     float* products = reinterpret_cast<float*>(base_ptr + L::scale_off(S, p.a_rows));     // [kTS][M_PAD]: a_s * w_s
     float* comb = reinterpret_cast<float*>(base_ptr + L::comb_off(S, p.a_rows));
     constexpr bool kAlt = L::kAlternate;
@@ -424,7 +425,17 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 }
                 if (p.sliced) {
                     // (the last arrival wraps the tile's counter back to zero: gemm_tc.cuh)
-                    if (et == 0) inc_acq_rel_gpu(p.flags + tile, unpack_holders(held, seg).count() - 1);
+                    const gemmtc::Holders h = unpack_holders(held, seg);
+                    if (M_PAD == 16 && gemmtc::last_adds(p.M, 32 * kEpiWarps)) {
+                        if (et == 0) *arrived_last = inc_acq_rel_gpu(p.flags + tile, h.count() - 1) == h.count() - 1;
+                        epi_bar_sync();
+                        if (*arrived_last)
+                            gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile, h, gemmtc::start_slot(tile), 0, 1, et, 32 * kEpiWarps,
+                                                                  p.M, p.N, 1.f, 0, p.c);
+                        epi_bar_sync();     // (before the word is written again)
+                    } else if (et == 0) {
+                        inc_acq_rel_gpu(p.flags + tile, h.count() - 1);
+                    }
                 } else if (!from_zero) {
                     if (et == 0) raise_flag(p.flags + blockIdx.x);
                 } else {
@@ -532,15 +543,16 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 ++tile;
             }
         }
-        if (p.sliced) {
+        if (p.sliced && !(M_PAD == 16 && gemmtc::last_adds(p.M, 32 * kEpiWarps))) {
 #pragma unroll 1
             for (int i = 0; i < seg; ++i) {
                 if (et == 0 && alive) await_word(p.flags + tile0 + i, [](int v) { return v == 0; }, abort_flag, p.status);
                 epi_bar_sync();
                 alive = __all_sync(0xffffffffu, alive && !*abort_flag);
                 if (alive)
-                    gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile0 + i, unpack_holders(held, i), gemmtc::start_slot(tile0 + i), et,
-                                                          32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
+                    gemmtc::add_slice<gemmtc::Kind::kMx8>(p.scratch, kSlotFloats, tile0 + i, unpack_holders(held, i), gemmtc::start_slot(tile0 + i),
+                                                          static_cast<int>(blockIdx.x) - unpack_holders(held, i).first, unpack_holders(held, i).count(),
+                                                          et, 32 * kEpiWarps, p.M, p.N, 1.f, 0, p.c);
             }
         }
     }

@@ -22,7 +22,7 @@
 //     CTA with the tile's start adds them in CTA order - it comes to that tile last, the partial was finished first.
 //     Few tiles ("sliced"): every CTA leaves the partial sums of its one or two tiles, and once a tile's counter is
 //     complete each of its CTAs adds one slice of it over all partials - instead of one CTA adding up to fifteen whole
-//     partials one after the other.  The order of the additions is CTA order either way and part of the results (it
+//     partials one after the other (with few rows the CTA that completes the counter adds the tile, last_adds()).  The order of the additions is CTA order either way and part of the results (it
 //     moves single roundings of the fp32 sums, and 4-bit quantisation behind them makes 4e-3 of a layer's output of
 //     that): it depends on the shape and the SM count alone, not on timing.
 //   * before it waits for the kernel ahead (programmatic launch) a CTA asks L2 for its first weight tiles, so a chain
@@ -237,16 +237,16 @@ __device__ __forceinline__ int slot_index(int sliced, bool from_zero, int tile) 
     return sliced && from_zero ? start_slot(tile) : static_cast<int>(blockIdx.x);
 }
 
-// This CTA's slice of a weight tile: the sum over all partials, in CTA order, scaled and stored.
+// Slice j of `slices` of a weight tile: the sum over all partials, in CTA order, scaled and stored.
 // A thread adds four activation rows of a weight row, eight partials in flight.
 template <Kind KIND>
-__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, Holders h, int first_slot, int thread,
-                                          int threads, int M, int N, float out_scale, int c_is_fp32, void* c) {
-    const int j = static_cast<int>(blockIdx.x) - h.first, parts = h.count(), quads = (M + 3) / 4 * kTileN;
+__device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_floats, int tile, Holders h, int first_slot, int j, int slices,
+                                          int thread, int threads, int M, int N, float out_scale, int c_is_fp32, void* c) {
+    const int parts = h.count(), quads = (M + 3) / 4 * kTileN;
     const float4* start = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(first_slot) * slot_floats);
     const float4* part = reinterpret_cast<const float4*>(scratch + static_cast<int64_t>(h.first) * slot_floats);   // [1], [2], ..
-    const int end = quads * (j + 1) / parts;
-    for (int e = quads * j / parts + thread; e < end; e += threads) {
+    const int end = quads * (j + 1) / slices;
+    for (int e = quads * j / slices + thread; e < end; e += threads) {
         float4 v = __ldcg(start + e);
         for (int q0 = 1; q0 < parts; q0 += 8) {
             float4 x[8];
@@ -271,6 +271,11 @@ __device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_flo
     }
 }
 
+// Few activation rows: a sliced tile has no more than two quads of sums per epilogue thread, which then are one round of loads
+// however few CTAs share them.  The CTA that arrives last at the tile's counter adds the whole tile, right there, and nobody
+// has to wait for the others: FP8 2112 x 7168 at one row, plain calls, 9.0 -> 8.0 us.
+__device__ __forceinline__ bool last_adds(int M, int threads) { return (M + 3) / 4 * kTileN <= 2 * threads; }
+
 template <Kind KIND, int M_PAD>
 __global__ void __launch_bounds__(Layout<KIND, M_PAD>::kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
@@ -289,6 +294,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                    full_tm = img_empty + kImgSlots * 8, empty_tm = full_tm + 16;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + L::misc_off(S, p.a_rows));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 4);
+    volatile int* arrived_last = reinterpret_cast<volatile int*>(base_ptr + L::misc_off(S, p.a_rows) + 8);
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
     const uint32_t lane = lane_id();
@@ -637,8 +643,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             alive = __all_sync(0xffffffffu, alive && !*abort_flag);
             if (alive) {
                 const Holders h = holders(i);
-                add_slice<KIND>(p.scratch, slot_floats, of, h, kEven ? h.first : start_slot(of), et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32,
-                                p.c);
+                add_slice<KIND>(p.scratch, slot_floats, of, h, kEven ? h.first : start_slot(of), static_cast<int>(blockIdx.x) - h.first,
+                                h.count(), et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32, p.c);
             }
         };
         for (int n = 0; n < count;) {
@@ -724,7 +730,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (p.sliced) {
                 // The last arrival wraps the tile's counter back to zero, which is what the others wait for, once they have
                 // nothing else to do.  No CTA arrives at a counter twice in a launch, the next launch's arrive after this one.
-                if (et == 0) inc_acq_rel_gpu(p.flags + tile, holders(seg).count() - 1);
+                const Holders h = holders(seg);
+                if (M_PAD == 16 && last_adds(p.M, kEpi)) {
+                    if (et == 0) *arrived_last = inc_acq_rel_gpu(p.flags + tile, h.count() - 1) == h.count() - 1;
+                    epi_sync();
+                    if (*arrived_last)
+                        add_slice<KIND>(p.scratch, slot_floats, tile, h, start_slot(tile), 0, 1, et, kEpi, p.M, p.N, p.out_scale, p.c_is_fp32, p.c);
+                    epi_sync();     // (before the word is written again)
+                } else if (et == 0) {
+                    inc_acq_rel_gpu(p.flags + tile, h.count() - 1);
+                }
                 if (kEven) slice(0);
             } else if (!from_zero) {
                 if (et == 0) raise_flag(p.flags + blockIdx.x);
@@ -790,7 +805,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (kb == p.kb) kb = 0, ++tile;
             ++seg;
         }
-        if (!kEven && p.sliced) {
+        if (!kEven && p.sliced && !(M_PAD == 16 && last_adds(p.M, kEpi))) {
 #pragma unroll 1
             for (uint32_t i = 0; i < seg; ++i) slice(i);
         }
