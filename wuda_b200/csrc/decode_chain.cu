@@ -16,7 +16,8 @@
 //   7 top-k + page transform
 // Only 1 -> 2 -> 4 -> 6 -> 7 is a chain.  5 needs nothing from 1-4 and 3 feeds nothing in 4-7, so
 // they run on two side streams forked from and joined back into the caller's stream with events
-// (5 joins before 6, 3 at the end).  Under stream capture the forks become parallel branches of the
+// (5 joins before 6, 3 at the end).  A layer's scatter of the front projection, which 5 and the folded head weights of 4 need,
+// goes ahead of 5 on its stream: in front of 1, where it was, it cost the layer at batch 1 / 64 / 128 4.1 / 5 / 5 us.  Under stream capture the forks become parallel branches of the
 // graph.  The side streams and events are created once per device and never destroyed.
 #include "host.h"
 
@@ -26,7 +27,7 @@ namespace chain {
 struct Side {
     bool ready = false;
     cudaStream_t writers = nullptr, query = nullptr;
-    cudaEvent_t fork = nullptr, forked_gemm = nullptr, writers_done = nullptr, query_done = nullptr;
+    cudaEvent_t fork = nullptr, forked_gemm = nullptr, writers_done = nullptr, query_done = nullptr, produced = nullptr;
 };
 
 int side_of_current_device(Side** out) {
@@ -38,7 +39,7 @@ int side_of_current_device(Side** out) {
     if (!s.ready) {
         WUDA_CUDA(cudaStreamCreateWithFlags(&s.writers, cudaStreamNonBlocking));
         WUDA_CUDA(cudaStreamCreateWithFlags(&s.query, cudaStreamNonBlocking));
-        for (cudaEvent_t* e : {&s.fork, &s.forked_gemm, &s.writers_done, &s.query_done})
+        for (cudaEvent_t* e : {&s.fork, &s.forked_gemm, &s.writers_done, &s.query_done, &s.produced})
             WUDA_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         s.ready = true;
     }
@@ -51,7 +52,11 @@ int side_of_current_device(Side** out) {
 
 extern "C" int wuda_csa_decode_step(const wuda_csa_weights* w, const wuda_csa_caches* c, const wuda_csa_step* s,
                                     const wuda_csa_workspace* ws, int m, void* stream) {
-    using namespace wuda;
+    return wuda::csa_decode_step(w, c, s, ws, m, stream, nullptr, nullptr);
+}
+
+int wuda::csa_decode_step(const wuda_csa_weights* w, const wuda_csa_caches* c, const wuda_csa_step* s, const wuda_csa_workspace* ws,
+                          int m, void* stream, int (*produce)(void* context, void* stream), void* context) {
     clear_error();
     WUDA_REQUIRE(w && c && s && ws, "weights, caches, step and workspace must not be NULL");
     WUDA_REQUIRE(m >= 1 && m <= 128, "m must be in [1, 128] (got %d)", m);
@@ -106,7 +111,9 @@ extern "C" int wuda_csa_decode_step(const wuda_csa_weights* w, const wuda_csa_ca
     cw.window.pool = c->swa_pool;
     cw.window.dst = s->swa_dst;
     const bool fp4 = c->idx_fp4 != 0;   // the indexer's FP4 form: Hadamard + MXFP4 query and keys, block-scaled logits
-    int status = (fp4 ? wuda_cache_writers_fp4 : wuda_cache_writers_fp8)(&cw, m, ws->status_word, side->writers);
+    int status = produce ? produce(context, side->writers) : WUDA_OK;
+    if (produce) WUDA_CUDA(cudaEventRecord(side->produced, side->writers));
+    if (status == WUDA_OK) status = (fp4 ? wuda_cache_writers_fp4 : wuda_cache_writers_fp8)(&cw, m, ws->status_word, side->writers);
     WUDA_CUDA(cudaEventRecord(side->writers_done, side->writers));
 
     // ---- the chain on the caller's stream.  Every fork is joined on every path out of this function,
@@ -128,6 +135,7 @@ extern "C" int wuda_csa_decode_step(const wuda_csa_weights* w, const wuda_csa_ca
                                      w->max_pos, s->q_main_out, m, w->main_heads, w->out_heads, w->eps, side->query);
         WUDA_CUDA(cudaEventRecord(side->query_done, side->query));
     }
+    if (produce) WUDA_CUDA(cudaStreamWaitEvent(main_stream, side->produced, 0));     // the heads' weights (w64)
     if (status == WUDA_OK)
         status = fp4 ? wuda_index_q_post_fp4(y, n_total, s->q_pos, w->cos_table, w->sin_table, w->max_pos, ws->iq_fp8,
                                              ws->w_folded, m, w->index_heads, stream)

@@ -42,6 +42,11 @@ int gemm_sms(const DeviceInfo& dev);
 // Where those launches find their flags: at the front of the scratch, or where wuda_gemm_flags said
 int32_t* gemm_flags(void* scratch);
 
+// wuda_csa_decode_step whose w64, window rows and state rings a launch of the caller's produces: `produce` enqueues it on the
+// stream it is given, beside the q norm and projection, which do not need them.
+int csa_decode_step(const wuda_csa_weights* w, const wuda_csa_caches* c, const wuda_csa_step* s, const wuda_csa_workspace* ws, int m,
+                    void* stream, int (*produce)(void* context, void* stream), void* context);
+
 // wuda_mhc_pre; with act_quant its FP8 output is what wuda_rmsnorm_quant_fp8 makes of `normed` with power-of-two scales (the two
 // differ in where the smallest scale lies, and for infinities and NaN).
 int mhc_pre_as(bool act_quant, const void* hidden_states, const float* weight, const float* base, const float* scale,

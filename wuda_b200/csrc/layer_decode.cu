@@ -266,8 +266,11 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
         WUDA_CUDA(cudaStreamWaitEvent(main_stream, side->done[0], 0));
         if (st != WUDA_OK) return st;
     }
-    WUDA_STAGE(wuda_front_emit(b.front_out, b.y16, t->pos, c.main_state, w->ape, t->main_state_row, c.idx_state, w->idx_ape,
-                               t->idx_state_row, b.win_y2, b.w64, c.state_rows_total, m, status, stream));
+    // the scatter of the BF16 segment runs beside the q norm and projection, ahead of the cache writers that read it
+    const auto emit = [&](void* on) {
+        return wuda_front_emit(b.front_out, b.y16, t->pos, c.main_state, w->ape, t->main_state_row, c.idx_state, w->idx_ape,
+                               t->idx_state_row, b.win_y2, b.w64, c.state_rows_total, m, status, on);
+    };
     wuda_csa_step step = {};
     step.q_raw = b.front_out;                 // the q_lora columns of the front projection, read in place
     step.q_raw_stride = kFront8;
@@ -299,7 +302,9 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
     ws.gemm_scratch = b.gemm_scratch;
     ws.gemm_scratch_bytes = b.gemm_scratch_bytes;
     ws.status_word = status;
-    WUDA_STAGE(wuda_csa_decode_step(&w->csa, &c, &step, &ws, m, stream));
+    WUDA_STAGE(csa_decode_step(
+        &w->csa, &c, &step, &ws, m, stream,
+        [](void* context, void* on) { return (*static_cast<decltype(emit)*>(context))(on); }, const_cast<void*>(static_cast<const void*>(&emit))));
 
     wuda_sparse_mla_args a = {};
     a.q = b.q_main;
