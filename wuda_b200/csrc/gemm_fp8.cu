@@ -590,7 +590,7 @@ static int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, Params& p,
     const long long units = static_cast<long long>(p.n_tiles) * p.kb;
     const int sms = gemm_sms(dev);
     const int grid = gemmtc::grid_of(units, p.n_tiles, M_PAD, sms);
-    p.sliced = !p.tp_peer_inbox && gemmtc::slice_wise(grid, p.n_tiles);     // (the two-rank form needs a finished tile in one CTA)
+    p.sliced = !p.tp_peer_inbox && gemmtc::slice_wise(grid, p.n_tiles, M_PAD);     // (the two-rank form needs a finished tile in one CTA)
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem, stream, w_map, a_map, p));
     return WUDA_OK;
 }
