@@ -73,3 +73,9 @@ def test_gather_and_nvfp4_codes(wuda, tokens, topk, k, gs, values):
     image = sf.cpu().numpy().reshape(n // 16, k // 256, 4, 32, 16)[:, :, :, :16, :4]     # [group, kb, step, row, byte]
     image = image.reshape(n // 16, k // 256, 4, 16, 4).transpose(0, 3, 1, 2, 4).reshape(n, k // 16)
     assert np.array_equal(image[rows[live]], s)
+
+
+# CTAs of 128 threads and of 768, either side of the line between them, more tokens than one walk takes, more rows than one look-up
+@pytest.mark.parametrize("tokens,topk,k", [(26, 4, 7168), (27, 9, 7168), (160, 2, 7168), (46, 1, 4096), (170, 13, 7168)])
+def test_gather_stores_a_token_to_all_its_rows(wuda, tokens, topk, k):
+    test_gather_and_nvfp4_codes(wuda, tokens, topk, k, 1.0 / 448, "normal")

@@ -120,11 +120,25 @@ int side_of_current_device(Side** out) {
     return WUDA_OK;
 }
 
-// SM shares (of the device's n): FP8 front segment 5/16 (its weights are 14.7 MB against the BF16 segment's
-// 37.6 MB), BF16 segment the rest; the shared expert all but 32, which the router's small kernels keep.
+// SM shares (of the device's n): FP8 front segment 5/16 (its weights are 14.7 MB against the BF16 segment's 37.6 MB), BF16 segment
+// the rest.  (16 + 21 tiles, cut into four ranges each by 64 + 84 SMs, would end together and sooner, but the order of these sums
+// moves the experts' 4-bit activations: 1.4e-2 of the output at batch 1.)
 int front8_sms(int n) { return n * 5 / 16 > 8 ? n * 5 / 16 : n; }
 int front16_sms(int n) { return n * 5 / 16 > 8 ? n - n * 5 / 16 : n; }
-int shared_sms(int n) { return n > 64 ? n - 32 : n; }
+// Shared expert, w1|w3: what the router projection (tiles of 128 experts, cut into at most 16 / 12 / 8 / 6 ranges) leaves, as whole
+// ranges per tile: a range that holds parts of two tiles takes part in two exchanges of partial sums.  4096 x 7168 at 1 / 64 / 128
+// rows by itself: 116 SMs 10.0 / 14.4 / 18.7 us, 96 SMs 10.0 / 13.1 / 17.4, 128 SMs 8.7 / 11.2 / 14.2.
+int shared_sms(int n, int m, int inter, int experts) {
+    const int split = m <= 16 ? 16 : (m <= 32 ? 12 : (m <= 64 ? 8 : 6));
+    const int left = n - (experts + 127) / 128 * split, tiles = (2 * inter + 127) / 128;
+    return left >= tiles ? left / tiles * tiles : (n > 64 ? n - 32 : n);
+}
+// w2: a range per tile and no exchange while a tile is no more than 16 units (7168 x 2048 at 1 / 64 / 128 rows: 116 SMs 7.3 / 9.8 / 13.4 us,
+// 56 SMs 7.5 / 9.2 / 11.3), so that the gather beside it finds free SMs.
+int shared_down_sms(int limit, int hidden, int inter) {
+    const int tiles = (hidden + 127) / 128;
+    return inter <= 16 * 128 && tiles <= limit ? tiles : limit;
+}
 
 // Lays the buffers out for up to m rows; returns the bytes used, or -1 for a geometry an entry point refuses.
 int64_t carve(const wuda_layer_weights* w, int m, int topk, int64_t logits_stride, int window, void* base, Buffers* b) {
@@ -348,10 +362,12 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
         const int si = w->shared_inter;
         WUDA_CUDA(cudaEventRecord(side->fork[1], main_stream));
         WUDA_CUDA(cudaStreamWaitEvent(side->stream, side->fork[1], 0));
-        wuda_gemm_sm_limit(shared_sms(sms));
+        const int up_sms = shared_sms(sms, m, si, w->experts_total);
+        wuda_gemm_sm_limit(up_sms);
         int st = wuda_gemm_fp8_blockscaled(b.s_x8, b.s_xs, w->shared_w13, w->shared_w13_scales, b.s_h, m, 2 * si, hidden,
                                            b.side_scratch, b.gemm_scratch_bytes, status, side->stream);
         if (st == WUDA_OK) st = wuda_swiglu_quant_fp8(b.s_h, nullptr, b.s_a8, b.s_as, m, si, w->swiglu_limit, 1, side->stream);
+        wuda_gemm_sm_limit(shared_down_sms(up_sms, hidden, si));
         if (st == WUDA_OK)
             st = wuda_gemm_fp8_blockscaled(b.s_a8, b.s_as, w->shared_w2, w->shared_w2_scales, b.s_out, m, hidden, si, b.side_scratch,
                                            b.gemm_scratch_bytes, status, side->stream);

@@ -226,8 +226,8 @@ __device__ __forceinline__ int64_t sf_offset(int row, int k16, int kb_per_row) {
     return (static_cast<int64_t>(group) * kb_per_row + kb) * 2048 + (within >> 2) * 512 + r * 16 + (within & 3);
 }
 
-// A thread of the two quantisation kernels owns one block of 16 values of one (token, expert) pair's row; the
-// four scale bytes of a 64-value step are collected by the first of its four lanes and stored as one word.
+// A thread of the two quantisation kernels owns one block of 16 values; the four scale bytes of a 64-value step are collected by
+// the first of its four lanes and stored as one word.
 // Rows without a token are not touched at all: the grouped GEMM, given row_token, does not store their
 // outputs, and nothing else reads them.
 __device__ __forceinline__ void unpack_bf16x8(const uint4& raw, float* v) {
@@ -239,15 +239,17 @@ __device__ __forceinline__ void unpack_bf16x8(const uint4& raw, float* v) {
     }
 }
 
-__device__ __forceinline__ void store_block(uint8_t* a4, uint8_t* a_sf, int row, int b, int row_blocks, const uint32_t (&packed)[2],
-                                            uint32_t sf, bool live) {
-    // (every lane of the warp takes part in the shuffles; blocks of a row never straddle a group of four lanes
-    // because row_blocks is a multiple of 16)
+// (every lane of the warp takes part in the shuffles; blocks of a row never straddle a group of four lanes
+// because a row has a multiple of 16 of them)
+__device__ __forceinline__ uint32_t sf_word(uint32_t sf) {
     uint32_t word = sf;
     word |= __shfl_down_sync(0xffffffffu, sf, 1) << 8;
     word |= __shfl_down_sync(0xffffffffu, sf, 2) << 16;
     word |= __shfl_down_sync(0xffffffffu, sf, 3) << 24;
-    if (!live) return;
+    return word;
+}
+__device__ __forceinline__ void store_block(uint8_t* a4, uint8_t* a_sf, int row, int b, int row_blocks, const uint32_t (&packed)[2],
+                                            uint32_t word) {
     *reinterpret_cast<uint2*>(a4 + static_cast<int64_t>(row) * (row_blocks * 8) + b * 8) = make_uint2(packed[0], packed[1]);
     if ((b & 3) == 0) *reinterpret_cast<uint32_t*>(a_sf + sf_offset(row, b, row_blocks / 16)) = word;
 }
@@ -261,48 +263,49 @@ struct GatherParams {
     uint8_t* a4;                 // [rows, K / 2]
     uint8_t* a_sf;               // packed scales
     float gs;
-    int K, pairs, topk;
+    int K, tokens, topk;
 };
 
-// Two CTAs of 256 threads per SM at most, each walking the blocks of the whole batch: launched early, the kernel waits beside
-// whatever else still needs the SMs.  With a thread per block (896 CTAs for 64 tokens x 8 experts) the waiting CTAs kept the
-// shared expert on the layer's second stream out until they had run, 28 us of a layer at batch 64.  The quantisation
-// without divisions (quant16) takes this kernel from 10.3 to 8.7 us and the SwiGLU one from 7.7 to 6.5 (512 rows, cold).
-constexpr int kGatherDepth = 2;   // blocks of a thread whose loads are in flight together
-constexpr int kGatherCtasPerSm = 2;
+// A thread quantises one block of 16 values of a token and stores it to the rows of all the token's pairs: they differ in nothing
+// else.  (A thread per block of a pair did that arithmetic, and read the token, topk times.)  Launched early, the kernel waits
+// beside whatever else still needs the SMs: no more CTAs than leave the shared expert's second projection, a CTA per weight tile,
+// its SMs (56 of 148 at 7168 dims).  With two CTAs on every SM that projection came behind the gather: mHC pre to the routed experts,
+// layer at batch 64 / 128 36 / 49 -> 27 / 37 us with the shared expert's even cuts.
+constexpr int kGatherThreads = 768;       // of a CTA where there are many blocks; a sixth of them where there are few
+constexpr int kGatherRows = 4;            // rows of a token that are looked up together
+inline int gather_ctas(int sms) { return sms * 5 / 8 > 0 ? sms * 5 / 8 : 1; }
 
-__global__ void __launch_bounds__(kQuantThreads) moe_gather_quant_kernel(GatherParams p) {
+__global__ void __launch_bounds__(kGatherThreads) moe_gather_quant_kernel(GatherParams p) {
     pdl_launch_dependents();
     pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
-    const int blocks = p.K / 16, total = p.pairs * blocks, stride = gridDim.x * kQuantThreads;
+    const int blocks = p.K / 16, total = p.tokens * blocks, stride = gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    for (int item0 = blockIdx.x * kQuantThreads + threadIdx.x; item0 - lane < total; item0 += kGatherDepth * stride) {
-        int pair[kGatherDepth], row[kGatherDepth];
+    for (int item = blockIdx.x * blockDim.x + threadIdx.x; item - lane < total; item += stride) {
+        const int token = item / blocks, b = item - token * blocks;
+        const bool live = item < total;
+        const int32_t* rows = p.pair_row + static_cast<int64_t>(token) * p.topk;
+        uint32_t packed[2] = {0u, 0u}, sf = 0u;
+        int row[kGatherRows];
 #pragma unroll
-        for (int u = 0; u < kGatherDepth; ++u) {
-            pair[u] = (item0 + u * stride) / blocks;
-            row[u] = pair[u] < p.pairs ? __ldcg(p.pair_row + pair[u]) : -1;
+        for (int u = 0; u < kGatherRows; ++u) row[u] = live && u < p.topk ? __ldcg(rows + u) : -1;
+        if (live) {
+            const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(token) * p.K + b * 16);
+            const uint4 lo = __ldcg(src), hi = __ldcg(src + 1);   // activations of a kernel of the same chain
+            float v[16];
+            unpack_bf16x8(lo, v);
+            unpack_bf16x8(hi, v + 8);
+            quant16(v, p.gs, packed, &sf);
         }
-        uint4 lo[kGatherDepth], hi[kGatherDepth];
+        const uint32_t word = sf_word(sf);
+        for (int first = 0; first < p.topk; first += kGatherRows) {
+            int next[kGatherRows];
 #pragma unroll
-        for (int u = 0; u < kGatherDepth; ++u) {
-            if (row[u] < 0) continue;
-            const int b = item0 + u * stride - pair[u] * blocks;
-            const uint4* src = reinterpret_cast<const uint4*>(p.x + static_cast<int64_t>(pair[u] / p.topk) * p.K + b * 16);
-            lo[u] = __ldcg(src), hi[u] = __ldcg(src + 1);   // activations of a kernel of the same chain
-        }
+            for (int u = 0; u < kGatherRows; ++u) next[u] = live && first + kGatherRows + u < p.topk ? __ldcg(rows + first + kGatherRows + u) : -1;
 #pragma unroll
-        for (int u = 0; u < kGatherDepth; ++u) {
-            if (item0 - lane + u * stride >= total) break;   // the same for the whole warp
-            uint32_t packed[2] = {0u, 0u}, sf = 0u;
-            const bool live = row[u] >= 0;
-            if (live) {
-                float v[16];
-                unpack_bf16x8(lo[u], v);
-                unpack_bf16x8(hi[u], v + 8);
-                quant16(v, p.gs, packed, &sf);
+            for (int u = 0; u < kGatherRows; ++u) {
+                if (row[u] >= 0) store_block(p.a4, p.a_sf, row[u], b, blocks, packed, word);
+                row[u] = next[u];
             }
-            store_block(p.a4, p.a_sf, row[u], item0 + u * stride - pair[u] * blocks, blocks, packed, sf, live);
         }
     }
 }
@@ -349,7 +352,8 @@ __global__ void __launch_bounds__(kQuantThreads) moe_swiglu_quant_kernel(SwigluP
         }
         quant16(v, p.gs, packed, &sf);
     }
-    store_block(p.a4, p.a_sf, row, b, blocks, packed, sf, live);
+    const uint32_t word = sf_word(sf);
+    if (live) store_block(p.a4, p.a_sf, row, b, blocks, packed, word);
 }
 
 // ---------------------------------------------------------------- combine
@@ -578,16 +582,18 @@ extern "C" int wuda_moe_gather_quant_nvfp4(const void* x_bf16, const int32_t* pa
     p.a_sf = static_cast<uint8_t*>(a_sf_packed);
     p.gs = global_scale;
     p.K = k;
-    p.pairs = tokens * topk;
+    p.tokens = tokens;
     p.topk = topk;
-    const long long items = static_cast<long long>(p.pairs) * (k / 16);
-    WUDA_REQUIRE(items < (1ll << 31), "tokens * topk * k / 16 must stay below 2^31");
+    const long long items = static_cast<long long>(tokens) * (k / 16);
+    WUDA_REQUIRE(items * topk < (1ll << 31), "tokens * topk * k / 16 must stay below 2^31");
     DeviceInfo dev;
     const int st = current_device_info(&dev);
     if (st != WUDA_OK) return st;
-    const long long ctas = (items + kQuantThreads - 1) / kQuantThreads, most = static_cast<long long>(kGatherCtasPerSm) * dev.num_sms;
-    WUDA_CUDA(launch_pdl(moe_gather_quant_kernel, dim3(static_cast<unsigned>(ctas < most ? ctas : most)),
-                         dim3(kQuantThreads), 0, static_cast<cudaStream_t>(stream), p));
+    const long long most = gather_ctas(dev.num_sms);
+    const int threads = items > most * (kGatherThreads / 6) ? kGatherThreads : kGatherThreads / 6;
+    const long long ctas = (items + threads - 1) / threads;
+    WUDA_CUDA(launch_pdl(moe_gather_quant_kernel, dim3(static_cast<unsigned>(ctas < most ? ctas : most)), dim3(threads), 0,
+                         static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
 }
 

@@ -172,7 +172,15 @@ class DecoderLayer:
             n = lib.wuda_num_sms()
             first = n * 5 // 16
             attention.sm_split = (first, n - first) if first > 8 else (n, n)
-            self._shared_sms = n - 32 if n > 64 else n
+
+    def _shared_sm_split(self, m):
+        """(SMs of w1|w3, SMs of w2) of the shared expert beside the router."""
+        n, inter = lib.wuda_num_sms(), self.ffn.shared.inter
+        split = 16 if m <= 16 else 12 if m <= 32 else 8 if m <= 64 else 6
+        left, tiles = n - -(-self.ffn.experts_total // 128) * split, -(-2 * inter // 128)
+        up = left // tiles * tiles if left >= tiles else n - 32 if n > 64 else n
+        down = -(-self.hidden // 128)
+        return up, down if inter <= 16 * 128 and down <= up else up
 
     # ---- the C++ launch sequence
     def _init_native(self, dev):
@@ -262,12 +270,8 @@ class DecoderLayer:
                                logits=self.gate_logits[:m])
         self.route_indices = idx
         shared = None
-        if f.shared is not None:   # on the SM share wuda_layer_decode gives the shared expert beside the router
-            lib.wuda_gemm_sm_limit(self._shared_sms)
-            try:
-                shared = f.shared.forward(normed)
-            finally:
-                lib.wuda_gemm_sm_limit(0)
+        if f.shared is not None:   # on the SM shares wuda_layer_decode gives the shared expert beside the router
+            shared = f.shared.forward(normed, sm_split=self._shared_sm_split(m))
         y = self.runner.forward(normed, rw, idx, shared=shared, y=self.y[:m])
         return ops.mhc_post_out(y, x, pre["post"], pre["comb"], self.out[:m])
 

@@ -169,16 +169,25 @@ class SharedExpert:
         self.w13, self.w13_scale, self.w2, self.w2_scale, self.limit = w13, w13_scale, w2, w2_scale, float(swiglu_limit)
         self.inter = w2.size(1)
 
-    def forward(self, x):
-        """x bf16 [M, dim] -> bf16 [M, dim]: quantise, w1|w3 GEMM, SwiGLU + quantise, w2 GEMM (four launches)."""
+    def forward(self, x, sm_split=None):
+        """x bf16 [M, dim] -> bf16 [M, dim]: quantise, w1|w3 GEMM, SwiGLU + quantise, w2 GEMM (four launches).  sm_split = (SMs of
+        the w1|w3 GEMM, SMs of the w2 GEMM) cuts them as wuda_layer_decode does, which makes the sums bit-identical to that call's."""
         x8, xs = ops.act_quant(x, 128, "ue8m0")
-        h = ops.fp8_gemm(x8, xs, self.w13, self.w13_scale)
-        m = x.size(0)
-        a8 = torch.empty(m, self.inter, dtype=torch.float8_e4m3fn, device=x.device)
-        a_s = torch.empty(m, self.inter // 128, dtype=torch.float32, device=x.device)
-        check(lib.wuda_swiglu_quant_fp8(h.data_ptr(), None, a8.data_ptr(), a_s.data_ptr(), m, self.inter, self.limit, 1,
-                                        torch.cuda.current_stream().cuda_stream))
-        return ops.fp8_gemm(a8, a_s, self.w2, self.w2_scale)
+        try:
+            if sm_split is not None:
+                lib.wuda_gemm_sm_limit(int(sm_split[0]))
+            h = ops.fp8_gemm(x8, xs, self.w13, self.w13_scale)
+            m = x.size(0)
+            a8 = torch.empty(m, self.inter, dtype=torch.float8_e4m3fn, device=x.device)
+            a_s = torch.empty(m, self.inter // 128, dtype=torch.float32, device=x.device)
+            check(lib.wuda_swiglu_quant_fp8(h.data_ptr(), None, a8.data_ptr(), a_s.data_ptr(), m, self.inter, self.limit, 1,
+                                            torch.cuda.current_stream().cuda_stream))
+            if sm_split is not None:
+                lib.wuda_gemm_sm_limit(int(sm_split[1]))
+            return ops.fp8_gemm(a8, a_s, self.w2, self.w2_scale)
+        finally:
+            if sm_split is not None:
+                lib.wuda_gemm_sm_limit(0)
 
 
 def moe_block(x, gate_weight, gate_bias, routed, shared, score_func="sqrtsoftplus", route_scale=1.0):
