@@ -206,3 +206,20 @@ def test_argument_checks(wuda):
         wuda.sparse_mla_decode(q, pool, idx, lens)            # more than 128 heads
     with pytest.raises(WudaError):
         wuda.sparse_mla_decode(q[:, :64].contiguous(), pool, idx, lens, softmax_scale=-1.0)
+
+
+def test_query_values_beyond_fp16_saturate(wuda):
+    """The query meets the keys as fp16: what lies beyond its range counts as its largest value, infinities too, and NaN as its lowest."""
+    rng = np.random.default_rng(11)
+    pool = model1_pool(rng, 4, 64)
+    idx = indices(rng, 1, 96, [90], 256)
+    q = rng.standard_normal((1, 128, 512)).astype(np.float32)
+    outs = []
+    for big, low in ((3e38, -3e38), (np.inf, -np.inf), (65536.0, np.nan), (1e30, -65536.0)):
+        v = q.copy()
+        v[0, 3, ::7], v[0, 3, 1::7] = big, low            # dims of the tensor-memory operand and of the shared-memory one
+        v[0, 70, 500], v[0, 70, 20] = low, big
+        out, status = run(wuda, u16(torch.from_numpy(v).bfloat16()), None, (pool, 64, idx, np.array([90], np.int32)), None)
+        assert status == 0
+        outs.append(out)
+    assert all(np.array_equal(outs[0], o) for o in outs[1:])

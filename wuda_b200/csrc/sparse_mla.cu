@@ -58,7 +58,9 @@ constexpr int kIssuerWarp = kSoftmaxWarps + kProducerWarps;   // two warps issue
 constexpr int kIssuerWarpPV = kIssuerWarp + 2;                 // issues P V
 constexpr int kThreads = (kIssuerWarpPV + 1) * 32;
 constexpr float kLog2e = 1.4426950408889634f;
-constexpr int kAhead = 3;             // passes whose records are in flight ahead of the one being stored
+// Passes whose records are in flight ahead of the one being stored.  (With three, 63 registers of a producer thread wait for records and a
+// few of them did not fit: 64 / 128 requests 80.5 / 159.9 us, with two 76.0 / 150.5, with one 73.8 / 146.1.)
+constexpr int kAhead = 1;
 constexpr int kMaxSplits = 32;        // CTAs that may share one request's keys (per output half)
 constexpr float kRescaleStep = 8.0f;   // log2 units the block maximum may exceed the reference by
 
@@ -139,12 +141,17 @@ __device__ __forceinline__ uint32_t e4m3x2_to_f16x2(uint32_t pair, uint32_t scal
     return r;
 }
 
-// two bf16 -> two fp16, saturating at the largest finite fp16 (exact for normal-range values)
+// two bf16 -> two fp16, saturating at the largest finite fp16 (exact for normal-range values); NaN becomes the lowest
 __device__ __forceinline__ uint32_t bf16x2_to_f16x2(uint32_t v) {
-    const float lo = fminf(fmaxf(__uint_as_float(v << 16), -65504.0f), 65504.0f);
-    const float hi = fminf(fmaxf(__uint_as_float(v & 0xffff0000u), -65504.0f), 65504.0f);
-    const __half2 h = __floats2half2_rn(lo, hi);
-    return *reinterpret_cast<const uint32_t*>(&h);
+    uint32_t h;
+    asm("{\n\t"
+        ".reg .b32 t;\n\t"
+        "cvt.rn.f16x2.f32 t, %2, %1;\n\t"
+        "max.f16x2 t, t, %3;\n\t"
+        "min.f16x2 %0, t, %4;\n\t"
+        "}"
+        : "=r"(h) : "f"(__uint_as_float(v << 16)), "f"(__uint_as_float(v & 0xffff0000u)), "r"(0xfbfffbffu), "r"(0x7bff7bffu));
+    return h;
 }
 __device__ __forceinline__ uint4 bf16x8_to_f16x8(uint4 v) {
     return make_uint4(bf16x2_to_f16x2(v.x), bf16x2_to_f16x2(v.y), bf16x2_to_f16x2(v.z), bf16x2_to_f16x2(v.w));
@@ -291,16 +298,20 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
 #pragma unroll
         for (int u = 0; u <= kAhead; ++u) idx[u] = fetch_index(p, b, first_key + u * kPass + row, n_swa, n_total);
     }
-    // The query rows, zero-padded to 128, come in as they lie, 16 bytes per lane and whole lines per warp: rotary dims to their
-    // place in the swizzled K-major operand layout, where the lane that brought a piece converts it, scaled dims to the (still
+    // The query rows, zero-padded to 128, come in as they lie, 16 bytes per lane and whole lines per warp: the last 128 dims
+    // to their place in the swizzled K-major operand layout, the others to the (still
     // unused) key stages, from where a row's thread takes them to tensor memory (row = lane, column = a pair of dims).  (A row
     // per thread straight from global memory touches 32 lines with every load: one request of 1152 keys, the first block's
     // scores 14.7 -> 9.5 us after the CTA's start, with the records asked for ahead of it.)
+    // (half a row per warp and turn, so that a lane's place in its chunk stays)
     const uint8_t* q_bytes = reinterpret_cast<const uint8_t*>(p.q + static_cast<int64_t>(b) * p.heads * kDim);
-    for (int i = threadIdx.x; i < kRows * (kDim / 8); i += kThreads) {
-        const int r = i / (kDim / 8), at = i % (kDim / 8), c = at >> 3;
-        const uint32_t dst = c < kQTmemChunks ? base + kOffOwn + c * kQChunk : base + kOffQ + (c - kQTmemChunks) * kQChunk;
-        cp_async_16(staged<128>(dst, r, at & 7), r < p.heads ? q_bytes + static_cast<int64_t>(i) * 16 : q_bytes, r < p.heads);
+    {
+        auto chunk_addr = [&](int c) { return c < kQTmemChunks ? base + kOffOwn + c * kQChunk : base + kOffQ + (c - kQTmemChunks) * kQChunk; };
+        const uint32_t left = chunk_addr(lane >> 3), right = chunk_addr(4 + (lane >> 3));
+        for (int i = warp; i < kRows * 2; i += kThreads / 32) {
+            const int r = i >> 1;
+            cp_async_16(staged<128>(i & 1 ? right : left, r, lane & 7), r < p.heads ? q_bytes + i * 512 + lane * 16 : q_bytes, r < p.heads);
+        }
     }
     KeyRegs ring[kAhead + 1];
     bool bad = false;
@@ -311,17 +322,11 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
         next_idx = idx[kAhead];
     }
     cp_async_wait_all();
-    for (int i = threadIdx.x; i < kRows * (kDim / 8); i += kThreads) {
-        const int r = i / (kDim / 8), at = i % (kDim / 8), c = at >> 3;
-        if (c < kQTmemChunks) continue;
-        const uint32_t mine = staged<128>(base + kOffQ + (c - kQTmemChunks) * kQChunk, r, at & 7);
-        st_shared_v4(mine, bf16x8_to_f16x8(ld_shared_v4(mine)));
-    }
     tc_fence_before();
     __syncthreads();   // the tensor-memory base address is published, the query has arrived
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    {   // three warps per quarter of the lanes, two chunks each
+    {   // tensor memory: three warps per quarter of the lanes, two chunks each
         static_assert(kQTmemChunks == 6 && kIssuerWarp == 12, "chunks per warp");
         if (warp < kIssuerWarp) {
             const int quarter = warp & 3;
@@ -339,6 +344,9 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
             }
             tmem_st_wait();
         }
+        // the chunks that stay: converted where they lie
+        for (uint32_t at = base + kOffQ + threadIdx.x * 16; at < base + kOffQ + kQSmemBytes; at += kThreads * 16)
+            st_shared_v4(at, bf16x8_to_f16x8(ld_shared_v4(at)));
     }
     fence_proxy_async_smem();
     tc_fence_before();
