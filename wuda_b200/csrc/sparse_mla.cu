@@ -303,7 +303,8 @@ __global__ void __launch_bounds__(kThreads, 1) sparse_mla_kernel(const Params p)
     // unused) key stages, from where a row's thread takes them to tensor memory (row = lane, column = a pair of dims).  (A row
     // per thread straight from global memory touches 32 lines with every load: one request of 1152 keys, the first block's
     // scores 14.7 -> 9.5 us after the CTA's start, with the records asked for ahead of it.)
-    // (half a row per warp and turn, so that a lane's place in its chunk stays)
+    // (half a row per warp and turn, so that a lane's place in its chunk stays; with that, and the last 128 dims converted where they lie
+    // instead of in a walk over all pieces, the query is laid out 1.8 us after it came instead of 3.3: one request 20.6 -> 18.6 us)
     const uint8_t* q_bytes = reinterpret_cast<const uint8_t*>(p.q + static_cast<int64_t>(b) * p.heads * kDim);
     {
         auto chunk_addr = [&](int c) { return c < kQTmemChunks ? base + kOffOwn + c * kQChunk : base + kOffQ + (c - kQTmemChunks) * kQChunk; };
