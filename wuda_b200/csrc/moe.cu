@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kDispatchThreads) moe_dispatch_kernel(Dispatch
     pdl_launch_dependents();
     __shared__ int count[kMaxExperts];
     __shared__ int base[kMaxExperts];       // first row of the expert that no earlier round has handed out
-    __shared__ uint16_t before[kDispatchWarps][kMaxExperts];   // a round's pairs of the expert in this warp, then in the warps before it
+    __shared__ alignas(16) uint16_t before[kDispatchWarps][kMaxExperts];   // a round's pairs of the expert in this warp, then in the warps before it
     __shared__ int total_groups;
     const int pairs = p.tokens * p.k;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
