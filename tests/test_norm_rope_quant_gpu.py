@@ -238,3 +238,16 @@ def test_rope_rows_cut_over_ctas(wuda, tokens, heads, head_dim, rope_dim, scale_
     assert torch.equal(s, scale)
     codes = (v / scale[..., None]).clamp(-448, 448).view(tokens, -1).to(torch.float8_e4m3fn)
     assert torch.equal(y8.view(torch.uint8), codes.view(torch.uint8))
+
+
+@pytest.mark.parametrize("rows,dim", [(297, 8192), (149, 13568), (449, 9216)])
+def test_norm_of_many_wide_rows(wuda, rows, dim):
+    """From these counts on the rows are taken with fewer registers: the same bits as a few rows at a time."""
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    x = torch.randn(rows, dim, generator=gen, device="cuda").bfloat16()
+    gamma = torch.rand(dim, generator=gen, device="cuda") + 0.5
+    whole = wuda.rmsnorm_quant(x, gamma)
+    parts = [wuda.rmsnorm_quant(x[i:i + 100], gamma) for i in range(0, rows, 100)]
+    for t, got in enumerate(whole):
+        want = torch.cat([p[t].view(torch.uint8) for p in parts])
+        assert torch.equal(got.view(torch.uint8), want)

@@ -25,6 +25,7 @@ namespace wuda {
 namespace nrq {
 
 constexpr int kMaxChunks = 3;   // 16-byte chunks per thread (rows up to 3 * 1024 * 8 = 24576 elements)
+constexpr int kHintRows = 64;
 
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
     uint16_t lo, hi;
@@ -118,16 +119,18 @@ struct NormParams {
     int rows, dim, pow2;
 };
 
-__global__ void __launch_bounds__(1024, 1) rmsnorm_quant_kernel(const NormParams p) {
+template <int kRegisters>
+__global__ void __maxnreg__(kRegisters) rmsnorm_quant_kernel(const NormParams p) {
     pdl_launch_dependents();
     __shared__ float warp_part[32];
     const int row = blockIdx.x;
     const int chunks = p.dim >> 3;                     // 16-byte chunks in the row
     const __nv_bfloat16* x = p.x + static_cast<int64_t>(row) * p.x_stride;
     // The weights' way to L2 starts before the wait (a hint: nothing is read yet), and row and weights are one round of loads:
-    // 1 to 100 rows of 7168 4.6 -> 3.6 us, 256 rows 6.1 -> 5.2
+    // 1 to 100 rows of 7168 4.6 -> 3.6 us, 256 rows 6.1 -> 5.2.  The hint comes from the first rows alone: L2 needs it once, and from every row
+    // it costs more than the rows do (fp32 weights, 4096 / 16384 x 512: 9.5 / 28.9 us, from the first 64 rows 6.1 / 17.4).
     const uint4* gamma = static_cast<const uint4*>(p.gamma);
-    if (p.gamma) {
+    if (p.gamma && blockIdx.x < kHintRows) {
 #pragma unroll
         for (int c = 0; c < kMaxChunks; ++c) {
             const int ch = c * blockDim.x + threadIdx.x;
@@ -354,7 +357,16 @@ extern "C" int wuda_rmsnorm_quant_fp8(const void* x_bf16, int64_t x_row_stride, 
     int threads = (chunks + kMaxChunks - 1) / kMaxChunks;
     threads = (threads + 31) / 32 * 32;
     if (threads > 1024) threads = 1024;
-    WUDA_CUDA(launch_pdl(rmsnorm_quant_kernel, dim3(rows), dim3(threads), 0, static_cast<cudaStream_t>(stream), p));
+    // With 64 registers a row and its weights stay in them; with 56 a few do not, but one more CTA may fit on an SM.  That pays where
+    // CTAs are so large that no more than two fit and the rows fill them: 300 / 1024 x 8192 6.8 -> 6.1 / 14.7 -> 12.1 us, 256 / 1024 x 13568
+    // 8.2 -> 6.3 / 26.5 -> 19.2; 7168 (three fit either way) 1024 rows 11.0 -> 11.2.
+    DeviceInfo dev;
+    const int st = current_device_info(&dev);
+    if (st != WUDA_OK) return st;
+    const auto fit = [&](int registers) { return 65536 / (registers * threads); };
+    const bool dense = fit(64) <= 2 && fit(56) > fit(64) && rows > dev.num_sms * fit(64);
+    WUDA_CUDA(launch_pdl(dense ? rmsnorm_quant_kernel<56> : rmsnorm_quant_kernel<64>, dim3(rows), dim3(threads), 0,
+                         static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
 }
 
