@@ -251,3 +251,19 @@ def test_norm_of_many_wide_rows(wuda, rows, dim):
     for t, got in enumerate(whole):
         want = torch.cat([p[t].view(torch.uint8) for p in parts])
         assert torch.equal(got.view(torch.uint8), want)
+
+
+@pytest.mark.parametrize("tokens", [1, 61, 148, 1776, 1777])
+@pytest.mark.parametrize("heads", [12, 43])
+def test_rope_cut_of_the_rows(wuda, tokens, heads):
+    """One token and many, rows of less than a round and of several: quantised (and its BF16 rows), and BF16 alone."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens + heads)
+    x = torch.randn(tokens, heads, 384, generator=gen, device="cuda").bfloat16()
+    pos = torch.randint(0, 512, (tokens,), generator=gen, device="cuda")
+    cos, sin = torch.randn(2, 512, 32, generator=gen, device="cuda")
+    want = oracle.rope_bf16(u16(x), pos.cpu().numpy(), cos.cpu().numpy(), sin.cpu().numpy(), 64)
+    want_q, want_s = oracle.act_quant_fp8(want.reshape(tokens, -1), 128, round_scale=False)
+    y16, y8, sc = wuda.rope_quant(x, pos, cos, sin, 64, return_bf16=True)
+    alone, _, _ = wuda.rope_quant(x, pos, cos, sin, 64, quant=False, return_bf16=True)
+    assert np.array_equal(u16(y16), want) and np.array_equal(u16(alone), want)
+    assert np.array_equal(y8.cpu().view(torch.uint8).numpy(), want_q) and np.array_equal(sc.cpu().numpy(), want_s)

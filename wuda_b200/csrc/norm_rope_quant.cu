@@ -203,8 +203,9 @@ __global__ void __maxnreg__(kRegisters) rmsnorm_quant_kernel(const NormParams p)
 // A CTA of 256 threads takes one round of two chunks per thread and is gone: five fit on an SM, and the loads of the next overlap the
 // arithmetic of the ones there.  (Four chunks per thread in one wave of CTAs loaded in step and computed in step: 64 / 256 tokens of
 // 128 heads x 192 4.6 -> 4.3 / 10.2 -> 9.2 us, x 512 6.7 -> 5.6 / 21.0 -> 17.4; with four or six CTAs per SM 4.1 / 9.2, 5.7 / 18.5 and
-// 4.3 / 9.6, 6.6 / 18.0.)
-constexpr int kRopeThreads = 256, kRopeDepth = 2;
+// 4.3 / 9.6, 6.6 / 18.0.)  Without quantisation there is next to no arithmetic, and four chunks per thread in one wave are better: 64 / 256 / 1000
+// tokens x 512 with two chunks 4.1 / 11.3 / 53.5 us, with four 3.8 / 10.1 / 48.5.
+constexpr int kRopeThreads = 256;
 
 struct RopeParams {
     const __nv_bfloat16* x;
@@ -217,7 +218,8 @@ struct RopeParams {
     int tokens, heads, head_dim, rope_dim, max_pos, inverse, pow2;
 };
 
-__global__ void __launch_bounds__(kRopeThreads, 5) rope_quant_kernel(const RopeParams p) {
+template <int kRopeDepth>       // 16-byte chunks of a thread whose loads are in flight together
+__global__ void __launch_bounds__(kRopeThreads, kRopeDepth > 2 ? 4 : 5) rope_quant_kernel(const RopeParams p) {
     pdl_launch_dependents();
     pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
     const int t = blockIdx.x;
@@ -404,16 +406,28 @@ extern "C" int wuda_rope_quant_fp8(const void* x_bf16, const int64_t* positions,
     p.inverse = inverse;
     p.pow2 = scale_mode;
     const int chunks = heads * head_dim / 8;
-    // A row is cut over as many CTAs as it has rounds of kRopeDepth 16-byte chunks per thread (a quantisation group is 16
-    // consecutive threads, so any multiple of the block size is a valid cut, and whole 16-thread groups stay in step).  With
-    // few tokens it is cut further, down to a chunk per thread, up to two CTAs per SM: one token of 128 heads x 192 / x 512
-    // 3.6 -> 2.6 / 4.0 -> 2.6 us.
+    // A quantisation group is 16 consecutive threads, so a row may be cut over CTAs at any multiple of their threads, and whole 16-thread
+    // groups stay in step.  They are cut into rounds of two chunks per thread, until there are so many rows that CTAs come and go
+    // for longer than a CTA per row takes (1500 tokens x 192 / x 512 40.6 / 95.9 us cut, 39.8 / 92.6 whole; both outputs
+    // 44.1 / 107.1 cut, 44.2 / 110.4 whole; 2048 tokens 54.8 / 130.4 cut, 49.5 / 112.2 whole).  Rows that are not quantised and fill two CTAs per SM are
+    // cut into rounds of four instead, as long as all CTAs are there together.  Few rows are cut further, down to a chunk per
+    // thread, up to two CTAs per SM: one token of 128 heads x 192 / x 512 3.6 -> 2.6 / 4.0 -> 2.6 us.
+    DeviceInfo dev;
+    const int st = current_device_info(&dev);
+    if (st != WUDA_OK) return st;
     const int threads = chunks < kRopeThreads ? (chunks + 31) / 32 * 32 : kRopeThreads;
-    const int rounds = (chunks + kRopeDepth * threads - 1) / (kRopeDepth * threads), most = (chunks + threads - 1) / threads;
-    const int few = 2 * 148 / tokens < most ? 2 * 148 / tokens : most;
-    int splits = rounds > few ? rounds : few;
+    const auto rounds = [&](int depth) { return (chunks + depth * threads - 1) / (depth * threads); };
+    const bool deep = !y_fp8 && rounds(2) > 1 && static_cast<long long>(tokens) * rounds(4) >= 2 * dev.num_sms;
+    int splits = 1;
+    if (!deep)
+        splits = tokens <= 12 * dev.num_sms ? rounds(2) : 1;
+    else
+        while (splits < rounds(4) && static_cast<long long>(tokens) * splits * 2 <= 5 * dev.num_sms) splits *= 2;
+    const int few = 2 * dev.num_sms / tokens < rounds(1) ? 2 * dev.num_sms / tokens : rounds(1);
+    if (splits < few) splits = few;
     if (splits > 65535) splits = 65535;      // (the loop takes what is left)
-    WUDA_CUDA(launch_pdl(rope_quant_kernel, dim3(dim3(tokens, splits)), dim3(threads), 0, static_cast<cudaStream_t>(stream), p));
+    WUDA_CUDA(launch_pdl(deep ? rope_quant_kernel<4> : rope_quant_kernel<2>, dim3(tokens, splits), dim3(threads), 0,
+                         static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
 }
 
