@@ -60,7 +60,8 @@ int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dtype, int rank, con
                       const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box,
                       CUtensorMapSwizzle swizzle, CUtensorMapL2promotion promo);
 
-// ---- programmatic dependent launch.  Every kernel of the library is launched with the attribute
+// ---- programmatic dependent launch.  Every kernel of the library but two (moe_route.cu and the SwiGLU of
+// norm_rope_quant.cu say why) is launched with the attribute
 // that lets it start while the kernel before it in the stream is still running; it then runs its
 // prologue (barrier set-up, TMEM allocation, descriptor prefetch) and stops at pdl_wait() until
 // the earlier kernel has completed and its writes are visible, before its first access to global memory.
