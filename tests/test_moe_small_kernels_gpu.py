@@ -79,3 +79,25 @@ def test_gather_and_nvfp4_codes(wuda, tokens, topk, k, gs, values):
 @pytest.mark.parametrize("tokens,topk,k", [(26, 4, 7168), (27, 9, 7168), (160, 2, 7168), (46, 1, 4096), (170, 13, 7168)])
 def test_gather_stores_a_token_to_all_its_rows(wuda, tokens, topk, k):
     test_gather_and_nvfp4_codes(wuda, tokens, topk, k, 1.0 / 448, "normal")
+
+
+def test_gather_of_as_many_blocks_as_it_takes(wuda):
+    """2^31 - 32768 blocks of 16 values, 69 GB: the walk's last steps lie beyond 2^31.  The last token's row is that of a call by itself."""
+    tokens, k = 65535, 1 << 19
+    if torch.cuda.mem_get_info()[0] < 80 << 30:
+        pytest.skip("needs 80 GB")
+    x = torch.empty(tokens, k, dtype=torch.bfloat16, device="cuda")
+    x[-1] = torch.randn(k, device="cuda")
+    rows = torch.full((tokens, 1), -1, dtype=torch.int32, device="cuda")
+    rows[-1] = 0
+    got = []
+    for t in (tokens, 1):
+        a4, sf = (torch.full((n,), 0x5a, dtype=torch.uint8, device="cuda") for n in (16 * k // 2, k // 256 * 2048))
+        check(wuda.lib.wuda_moe_gather_quant_nvfp4(x[-t:].data_ptr(), rows[-t:].data_ptr(), a4.data_ptr(), sf.data_ptr(), 1.0 / 448, t, 1, k,
+                                                   torch.cuda.current_stream().cuda_stream))
+        got.append((a4, sf))
+    torch.cuda.synchronize()
+    del x
+    torch.cuda.empty_cache()
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+    assert bool((got[0][0][:k // 2] != 0x5a).any()) and bool((got[0][0][k // 2:] == 0x5a).all())

@@ -278,10 +278,11 @@ inline int gather_ctas(int sms) { return sms * 5 / 8 > 0 ? sms * 5 / 8 : 1; }
 __global__ void __launch_bounds__(kGatherThreads) moe_gather_quant_kernel(GatherParams p) {
     pdl_launch_dependents();
     pdl_wait();   // nothing of global memory is touched before the kernel ahead has finished
-    const int blocks = p.K / 16, total = p.tokens * blocks, stride = gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    for (int item = blockIdx.x * blockDim.x + threadIdx.x; item - lane < total; item += stride) {
-        const int token = item / blocks, b = item - token * blocks;
+    // (unsigned: the entry takes up to 2^31 - 1 blocks, and a walk goes up to a stride beyond them)
+    const uint32_t blocks = p.K / 16, total = p.tokens * blocks, stride = gridDim.x * blockDim.x;
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t item = blockIdx.x * blockDim.x + threadIdx.x; item - lane < total; item += stride) {
+        const uint32_t token = item / blocks, b = item - token * blocks;
         const bool live = item < total;
         const int32_t* rows = p.pair_row + static_cast<int64_t>(token) * p.topk;
         uint32_t packed[2] = {0u, 0u}, sf = 0u;
