@@ -81,6 +81,12 @@ def test_gather_stores_a_token_to_all_its_rows(wuda, tokens, topk, k):
     test_gather_and_nvfp4_codes(wuda, tokens, topk, k, 1.0 / 448, "normal")
 
 
+# the lines between the grids of a call by itself (at 148 SMs): CTAs of 128 threads and of 768, of 768 and of 256, one walk and more
+@pytest.mark.parametrize("tokens,topk,k", [(84, 2, 7168), (85, 2, 7168), (253, 1, 7168), (254, 2, 7168), (680, 1, 7168)])
+def test_gather_grids(wuda, tokens, topk, k):
+    test_gather_and_nvfp4_codes(wuda, tokens, topk, k, 1.0 / 448, "normal")
+
+
 def test_gather_of_as_many_blocks_as_it_takes(wuda):
     """2^31 - 32768 blocks of 16 values, 69 GB: the walk's last steps lie beyond 2^31.  The last token's row is that of a call by itself."""
     tokens, k = 65535, 1 << 19

@@ -54,6 +54,10 @@ int mhc_pre_as(bool act_quant, const void* hidden_states, const float* weight, c
                void* collapsed_bf16, void* normed_bf16, void* x_fp8, float* x_scales, void* workspace, int64_t workspace_bytes, int m,
                int hidden, void* stream);
 
+// wuda_moe_gather_quant_nvfp4 beside a GEMM of reserved_sms CTAs (0: none) on another stream, which it leaves their SMs.
+int moe_gather_beside(int reserved_sms, const void* x_bf16, const int32_t* pair_row, void* a_fp4, void* a_sf_packed, float global_scale,
+                      int tokens, int topk, int k, void* stream);
+
 // rank-`rank` tiled tensor map. dims/box are innermost-first; strides_bytes has rank-1
 // entries (stride of dims 1..rank-1). Returns a wuda_status.
 int encode_tensor_map(CUtensorMap* map, CUtensorMapDataType dtype, int rank, const void* base,

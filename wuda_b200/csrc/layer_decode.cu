@@ -358,6 +358,7 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
                           w->shared_w13 ? b.s_xs : nullptr, b.pre_ws, wuda_mhc_pre_workspace_bytes(s->m_max, hidden), m, hidden, stream));
     // the shared expert on the side stream, beside router projection, routing, dispatch and gather
     const void* shared_rows = nullptr;
+    int down_sms = 0;
     if (w->shared_w13) {
         const int si = w->shared_inter;
         WUDA_CUDA(cudaEventRecord(side->fork[1], main_stream));
@@ -367,7 +368,7 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
         int st = wuda_gemm_fp8_blockscaled(b.s_x8, b.s_xs, w->shared_w13, w->shared_w13_scales, b.s_h, m, 2 * si, hidden,
                                            b.side_scratch, b.gemm_scratch_bytes, status, side->stream);
         if (st == WUDA_OK) st = wuda_swiglu_quant_fp8(b.s_h, nullptr, b.s_a8, b.s_as, m, si, w->swiglu_limit, 1, side->stream);
-        wuda_gemm_sm_limit(shared_down_sms(up_sms, hidden, si));
+        wuda_gemm_sm_limit(down_sms = shared_down_sms(up_sms, hidden, si));
         if (st == WUDA_OK)
             st = wuda_gemm_fp8_blockscaled(b.s_a8, b.s_as, w->shared_w2, w->shared_w2_scales, b.s_out, m, hidden, si, b.side_scratch,
                                            b.gemm_scratch_bytes, status, side->stream);
@@ -389,7 +390,7 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
                                          w->moe_topk, w->experts_local, w->expert_first, w->experts_total, b.max_groups, status,
                                          stream);
     if (routed == WUDA_OK)
-        routed = wuda_moe_gather_quant_nvfp4(b.f_normed, b.pair_row, b.a1, b.a1_sf, w->act_scale_in, m, w->moe_topk, hidden, stream);
+        routed = moe_gather_beside(down_sms, b.f_normed, b.pair_row, b.a1, b.a1_sf, w->act_scale_in, m, w->moe_topk, hidden, stream);
     if (w->shared_w13) WUDA_CUDA(cudaStreamWaitEvent(main_stream, side->done[1], 0));   // join
     if (routed != WUDA_OK) return routed;
     WUDA_STAGE(wuda_gemm_nvfp4_grouped(b.a1, b.a1_sf, w->act_scale_in, w->w13, w->w13_sf, w->w13_gs, b.group_expert, b.num_groups, b.row_token, b.h,

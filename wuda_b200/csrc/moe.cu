@@ -267,13 +267,32 @@ struct GatherParams {
 };
 
 // A thread quantises one block of 16 values of a token and stores it to the rows of all the token's pairs: they differ in nothing
-// else.  (A thread per block of a pair did that arithmetic, and read the token, topk times.)  Launched early, the kernel waits
-// beside whatever else still needs the SMs: no more CTAs than leave the shared expert's second projection, a CTA per weight tile,
-// its SMs (56 of 148 at 7168 dims).  With two CTAs on every SM that projection came behind the gather: mHC pre to the routed experts,
-// layer at batch 64 / 128 36 / 49 -> 27 / 37 us with the shared expert's even cuts.
-constexpr int kGatherThreads = 768;       // of a CTA where there are many blocks; a sixth of them where there are few
+// else.  (A thread per block of a pair did that arithmetic, and read the token, topk times.)
+constexpr int kGatherThreads = 768;       // most of a CTA
 constexpr int kGatherRows = 4;            // rows of a token that are looked up together
-inline int gather_ctas(int sms) { return sms * 5 / 8 > 0 ? sms * 5 / 8 : 1; }
+
+struct GatherGrid {
+    int ctas, threads;
+};
+// With the GPU to itself: CTAs of 128 threads while two per SM hold all blocks, of 768 while one does, beyond that eight of 256 per SM, whose
+// loads overlap the others' arithmetic (tokens of 7168 values, 8 rows each: 128 / 1024 / 8192 tokens in 92 CTAs of 768 4.9 / 22.6 /
+// 251 us, in one per SM 4.9 / 16.4 / 220, in eight of 256 per SM 4.9 / 12.7 / 229; one row each: 3.2 / 15.1 / 115.8, 3.2 / 11.1 / 74.5, 3.7 / 9.2 / 65.3).
+// Beside a GEMM of `reserved` CTAs on another stream, no more CTAs than leave it its SMs: launched early, they wait there before it comes.  With two
+// on every SM the shared expert's second projection (56 CTAs at 7168 dims) came behind the gather: mHC pre to the routed experts,
+// layer at batch 64 / 128 36 / 49 -> 27 / 37 us with the shared expert's even cuts.
+inline GatherGrid gather_grid(long long blocks, int sms, int reserved) {
+    long long most;
+    int threads;
+    if (reserved > 0) {
+        most = sms - reserved > sms / 8 ? sms - reserved : sms / 8 + 1;
+        threads = blocks > most * 128 ? kGatherThreads : 128;
+    } else {
+        threads = blocks <= 2ll * sms * 128 ? 128 : (blocks <= static_cast<long long>(sms) * kGatherThreads ? kGatherThreads : 256);
+        most = 8ll * sms;
+    }
+    const long long ctas = (blocks + threads - 1) / threads;
+    return {static_cast<int>(ctas < most ? ctas : most), threads};
+}
 
 __global__ void __launch_bounds__(kGatherThreads) moe_gather_quant_kernel(GatherParams p) {
     pdl_launch_dependents();
@@ -568,7 +587,11 @@ extern "C" int wuda_moe_dispatch_range(const int32_t* indices, const float* weig
 
 extern "C" int wuda_moe_gather_quant_nvfp4(const void* x_bf16, const int32_t* pair_row, void* a_fp4, void* a_sf_packed,
                                            float global_scale, int tokens, int topk, int k, void* stream) {
-    using namespace wuda;
+    return wuda::moe_gather_beside(0, x_bf16, pair_row, a_fp4, a_sf_packed, global_scale, tokens, topk, k, stream);
+}
+
+int wuda::moe_gather_beside(int reserved_sms, const void* x_bf16, const int32_t* pair_row, void* a_fp4, void* a_sf_packed,
+                            float global_scale, int tokens, int topk, int k, void* stream) {
     using namespace wuda::moe;
     clear_error();
     WUDA_REQUIRE(tokens >= 1 && topk >= 1 && static_cast<long long>(tokens) * topk <= 65536, "tokens, topk >= 1 and at most 65536 pairs");
@@ -590,11 +613,8 @@ extern "C" int wuda_moe_gather_quant_nvfp4(const void* x_bf16, const int32_t* pa
     DeviceInfo dev;
     const int st = current_device_info(&dev);
     if (st != WUDA_OK) return st;
-    const long long most = gather_ctas(dev.num_sms);
-    const int threads = items > most * (kGatherThreads / 6) ? kGatherThreads : kGatherThreads / 6;
-    const long long ctas = (items + threads - 1) / threads;
-    WUDA_CUDA(launch_pdl(moe_gather_quant_kernel, dim3(static_cast<unsigned>(ctas < most ? ctas : most)), dim3(threads), 0,
-                         static_cast<cudaStream_t>(stream), p));
+    const GatherGrid grid = gather_grid(items, dev.num_sms, reserved_sms);
+    WUDA_CUDA(launch_pdl(moe_gather_quant_kernel, dim3(grid.ctas), dim3(grid.threads), 0, static_cast<cudaStream_t>(stream), p));
     return WUDA_OK;
 }
 
