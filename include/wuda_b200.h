@@ -989,6 +989,11 @@ int64_t wuda_layer_workspace_offset(const wuda_layer_weights* weights, int m_max
 int wuda_layer_decode(const wuda_layer_weights* weights, const wuda_layer_state* state, const wuda_layer_step* step,
                       int m, void* stream);
 
+/* The SMs that wuda_layer_decode gives, on a device of num_sms, to the GEMMs it runs side by side: shares = {front projection
+ * FP8, BF16; router projection; shared expert w1|w3, w2} (wuda_gemm_sm_limit; the router projection takes what it takes on
+ * the whole device).  A caller that enqueues the stages itself gets the same sums in the same order with them. */
+int wuda_layer_sm_shares(int num_sms, int m, int hidden, int shared_inter, int experts_total, int32_t* shares);
+
 /* ------------------------------------------------------------------------------------
  * Host-buffer form of the indexer step: paged MQA logits, then top-k with the request's
  * block table as the page table (page_size = entries_per_block).

@@ -108,3 +108,16 @@ def test_the_documented_build_command_does_not_need_the_library():
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr
     out = subprocess.run([sys.executable, "-m", "wuda_b200.build"], cwd=root, capture_output=True, text=True, timeout=1500)
     assert out.returncode == 0, out.stderr
+
+
+@pytest.mark.parametrize("experts", [16, 256, 384, 512])
+@pytest.mark.parametrize("inter", [256, 2048, 5376, 5504, 16384])
+def test_overlapped_gemms_fit_the_device_together(experts, inter):
+    """A GEMM's CTAs wait for one another, so those that a layer runs at the same time must all have an SM."""
+    import wuda_b200._lib as L
+    for m in range(1, 129):
+        shares = (ctypes.c_int32 * 5)()
+        assert L.lib.wuda_layer_sm_shares(148, m, 7168, inter, experts, shares) == 0
+        front8, front16, router, up, down = shares
+        assert min(shares) >= 1 and front8 + front16 == 148 and router + up <= 148 and down <= up
+    assert L.lib.wuda_layer_sm_shares(148, 129, 7168, inter, experts, shares) == 1

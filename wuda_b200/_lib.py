@@ -193,6 +193,7 @@ SIGNATURES = {
     "wuda_topk": (c_int, [c_vp, c_vp, c_vp, c_vp, c_vp, c_int, c_i64, c_i64, c_int, c_int, c_int, c_vp]),
     "wuda_layer_workspace_bytes": (c_i64, [ctypes.POINTER(LayerWeights), c_int, c_int, c_i64, c_int]),
     "wuda_layer_workspace_offset": (c_i64, [ctypes.POINTER(LayerWeights), c_int, c_int, c_i64, c_int, ctypes.c_char_p]),
+    "wuda_layer_sm_shares": (c_int, [c_int, c_int, c_int, c_int, c_int, c_vp]),
     "wuda_layer_decode": (c_int, [ctypes.POINTER(LayerWeights), ctypes.POINTER(LayerState), ctypes.POINTER(LayerStep),
                                   c_int, c_vp]),
 }

@@ -820,14 +820,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
     }
 }
 
-// Ranges that share a weight tile at most (adding partial sums costs as much as streaming M_PAD / 64 units of weights, so wide
-// tiles are cut into fewer).
-constexpr int max_split(int m_pad) { return m_pad <= 16 ? 16 : (m_pad == 32 ? 12 : (m_pad == 64 ? 8 : 6)); }
-inline int grid_of(long long units, int n_tiles, int m_pad, int sms) {
-    int grid = units < sms ? static_cast<int>(units) : sms;
-    if (static_cast<long long>(n_tiles) * max_split(m_pad) < grid) grid = n_tiles * max_split(m_pad);
-    return grid;
-}
 // Added in slices where every tile is cut into three ranges or more (and the slots suffice: one per CTA and one per tile).  Ranges that
 // hold parts of two tiles take part in two additions, each behind that tile's last CTA: with 17 to 64 rows that pays from five
 // ranges per tile on (FP8 4096 x 7168 at 64 rows, 148 ranges of 32 tiles: in slices 14.1 us, by the CTA with the tile's start 12.7; BF16

@@ -39,6 +39,17 @@ struct DeviceInfo {
 int current_device_info(DeviceInfo* out);
 // SMs the GEMM launches of the calling thread may cover: all of the device's, or fewer after wuda_gemm_sm_limit
 int gemm_sms(const DeviceInfo& dev);
+// How many CTAs they take (their waits for one another count on all of them being there at the same time):
+namespace gemmtc {
+// Ranges that share a weight tile at most (adding partial sums costs as much as streaming M_PAD / 64 units of weights, so wide
+// tiles are cut into fewer).
+constexpr int max_split(int m_pad) { return m_pad <= 16 ? 16 : (m_pad == 32 ? 12 : (m_pad == 64 ? 8 : 6)); }
+inline int grid_of(long long units, int n_tiles, int m_pad, int sms) {
+    int grid = units < sms ? static_cast<int>(units) : sms;
+    if (static_cast<long long>(n_tiles) * max_split(m_pad) < grid) grid = n_tiles * max_split(m_pad);
+    return grid;
+}
+}  // namespace gemmtc
 // Where those launches find their flags: at the front of the scratch, or where wuda_gemm_flags said
 int32_t* gemm_flags(void* scratch);
 

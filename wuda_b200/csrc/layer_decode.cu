@@ -120,24 +120,30 @@ int side_of_current_device(Side** out) {
     return WUDA_OK;
 }
 
-// SM shares (of the device's n): FP8 front segment 5/16 (its weights are 14.7 MB against the BF16 segment's 37.6 MB), BF16 segment
-// the rest.  (16 + 21 tiles, cut into four ranges each by 64 + 84 SMs, would end together and sooner, but the order of these sums
-// moves the experts' 4-bit activations: 1.4e-2 of the output at batch 1.)
-int front8_sms(int n) { return n * 5 / 16 > 8 ? n * 5 / 16 : n; }
-int front16_sms(int n) { return n * 5 / 16 > 8 ? n - n * 5 / 16 : n; }
-// Shared expert, w1|w3: what the router projection (tiles of 128 experts, cut into at most 16 / 12 / 8 / 6 ranges) leaves, as whole
-// ranges per tile: a range that holds parts of two tiles takes part in two exchanges of partial sums.  4096 x 7168 at 1 / 64 / 128
-// rows by itself: 116 SMs 10.0 / 14.4 / 18.7 us, 96 SMs 10.0 / 13.1 / 17.4, 128 SMs 8.7 / 11.2 / 14.2.
-int shared_sms(int n, int m, int inter, int experts) {
-    const int split = m <= 16 ? 16 : (m <= 32 ? 12 : (m <= 64 ? 8 : 6));
-    const int left = n - (experts + 127) / 128 * split, tiles = (2 * inter + 127) / 128;
-    return left >= tiles ? left / tiles * tiles : (n > 64 ? n - 32 : n);
-}
-// w2: a range per tile and no exchange while a tile is no more than 16 units (7168 x 2048 at 1 / 64 / 128 rows: 116 SMs 7.3 / 9.8 / 13.4 us,
-// 56 SMs 7.5 / 9.2 / 11.3), so that the gather beside it finds free SMs.
-int shared_down_sms(int limit, int hidden, int inter) {
-    const int tiles = (hidden + 127) / 128;
-    return inter <= 16 * 128 && tiles <= limit ? tiles : limit;
+// SMs of the GEMMs that run side by side, and of the router projection; n: the device's.  The CTAs of a GEMM wait for one another, so those
+// of one time have to fit the device together: front8 + front16, router + up, the gather beside down.
+struct SmShares {
+    int front8, front16, router, up, down;
+};
+SmShares sm_shares(int n, int m, int hidden, int inter, int experts) {
+    SmShares s;
+    // FP8 front segment 5/16 (its weights are 14.7 MB against the BF16 segment's 37.6 MB), BF16 segment
+    // the rest.  (16 + 21 tiles, cut into four ranges each by 64 + 84 SMs, would end together and sooner, but the order of these sums
+    // moves the experts' 4-bit activations: 1.4e-2 of the output at batch 1.)
+    s.front8 = n * 5 / 16 > 8 ? n * 5 / 16 : n;
+    s.front16 = n * 5 / 16 > 8 ? n - n * 5 / 16 : n;
+    const int m_pad = m <= 16 ? 16 : (m <= 32 ? 32 : (m <= 64 ? 64 : 128)), router_tiles = (experts + 127) / 128;
+    s.router = gemmtc::grid_of(static_cast<long long>(router_tiles) * (hidden / 64), router_tiles, m_pad, n);
+    // Shared expert, w1|w3: what the router projection leaves, as whole
+    // ranges per tile: a range that holds parts of two tiles takes part in two exchanges of partial sums.  4096 x 7168 at 1 / 64 / 128
+    // rows by itself: 116 SMs 10.0 / 14.4 / 18.7 us, 96 SMs 10.0 / 13.1 / 17.4, 128 SMs 8.7 / 11.2 / 14.2.
+    const int left = n - s.router > 0 ? n - s.router : 1, up_tiles = (2 * inter + 127) / 128, wide = n > 64 ? n - 32 : n;
+    s.up = left >= up_tiles && up_tiles > 0 ? left / up_tiles * up_tiles : (left < wide ? left : wide);
+    // w2: a range per tile and no exchange while a tile is no more than 16 units (7168 x 2048 at 1 / 64 / 128 rows: 116 SMs 7.3 / 9.8 / 13.4 us,
+    // 56 SMs 7.5 / 9.2 / 11.3), so that the gather beside it finds free SMs.
+    const int down_tiles = (hidden + 127) / 128;
+    s.down = inter <= 16 * 128 && down_tiles <= s.up ? down_tiles : s.up;
+    return s;
 }
 
 // Lays the buffers out for up to m rows; returns the bytes used, or -1 for a geometry an entry point refuses.
@@ -228,6 +234,16 @@ extern "C" int64_t wuda_layer_workspace_bytes(const wuda_layer_weights* w, int m
     return wuda::layer::carve(w, m_max, topk, logits_stride, window, nullptr, &b);
 }
 
+extern "C" int wuda_layer_sm_shares(int num_sms, int m, int hidden, int shared_inter, int experts_total, int32_t* shares) {
+    using namespace wuda;
+    clear_error();
+    WUDA_REQUIRE(num_sms >= 1 && m >= 1 && m <= 128 && hidden >= 128 && shared_inter >= 0 && experts_total >= 1 && shares,
+                 "num_sms, hidden / 128 and experts_total must be at least 1, m in [1, 128], shared_inter >= 0 and shares given");
+    const layer::SmShares s = layer::sm_shares(num_sms, m, hidden, shared_inter, experts_total);
+    for (int v : {s.front8, s.front16, s.router, s.up, s.down}) *shares++ = v;
+    return WUDA_OK;
+}
+
 #define WUDA_STAGE(call)                 \
     do {                                 \
         const int st__ = (call);         \
@@ -264,15 +280,15 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
     Side* side = nullptr;
     WUDA_STAGE(side_of_current_device(&side));
     cudaStream_t main_stream = static_cast<cudaStream_t>(stream);
-    const int sms = wuda_num_sms();
+    const SmShares shares = sm_shares(wuda_num_sms(), m, hidden, w->shared_w13 ? w->shared_inter : 0, w->experts_total);
     {   // the two segments of the front projection side by side; the fork is joined on every path
         WUDA_CUDA(cudaEventRecord(side->fork[0], main_stream));
         WUDA_CUDA(cudaStreamWaitEvent(side->stream, side->fork[0], 0));
-        wuda_gemm_sm_limit(front16_sms(sms));
+        wuda_gemm_sm_limit(shares.front16);
         int st = wuda_gemm_bf16(b.a_normed, w->front_w16, b.y16, 1, m, kFront16, hidden, b.side_scratch, b.gemm_scratch_bytes, status,
                                 side->stream);
         WUDA_CUDA(cudaEventRecord(side->done[0], side->stream));
-        wuda_gemm_sm_limit(front8_sms(sms));
+        wuda_gemm_sm_limit(shares.front8);
         if (st == WUDA_OK)
             st = wuda_gemm_fp8_blockscaled(b.a_xq, b.a_xsf, w->front_w8, w->front_w8_scales, b.front_out, m, kFront8, hidden,
                                            b.gemm_scratch, b.gemm_scratch_bytes, status, stream);
@@ -358,17 +374,15 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
                           w->shared_w13 ? b.s_xs : nullptr, b.pre_ws, wuda_mhc_pre_workspace_bytes(s->m_max, hidden), m, hidden, stream));
     // the shared expert on the side stream, beside router projection, routing, dispatch and gather
     const void* shared_rows = nullptr;
-    int down_sms = 0;
     if (w->shared_w13) {
         const int si = w->shared_inter;
         WUDA_CUDA(cudaEventRecord(side->fork[1], main_stream));
         WUDA_CUDA(cudaStreamWaitEvent(side->stream, side->fork[1], 0));
-        const int up_sms = shared_sms(sms, m, si, w->experts_total);
-        wuda_gemm_sm_limit(up_sms);
+        wuda_gemm_sm_limit(shares.up);
         int st = wuda_gemm_fp8_blockscaled(b.s_x8, b.s_xs, w->shared_w13, w->shared_w13_scales, b.s_h, m, 2 * si, hidden,
                                            b.side_scratch, b.gemm_scratch_bytes, status, side->stream);
         if (st == WUDA_OK) st = wuda_swiglu_quant_fp8(b.s_h, nullptr, b.s_a8, b.s_as, m, si, w->swiglu_limit, 1, side->stream);
-        wuda_gemm_sm_limit(down_sms = shared_down_sms(up_sms, hidden, si));
+        wuda_gemm_sm_limit(shares.down);
         if (st == WUDA_OK)
             st = wuda_gemm_fp8_blockscaled(b.s_a8, b.s_as, w->shared_w2, w->shared_w2_scales, b.s_out, m, hidden, si, b.side_scratch,
                                            b.gemm_scratch_bytes, status, side->stream);
@@ -390,7 +404,7 @@ extern "C" int wuda_layer_decode(const wuda_layer_weights* w, const wuda_layer_s
                                          w->moe_topk, w->experts_local, w->expert_first, w->experts_total, b.max_groups, status,
                                          stream);
     if (routed == WUDA_OK)
-        routed = moe_gather_beside(down_sms, b.f_normed, b.pair_row, b.a1, b.a1_sf, w->act_scale_in, m, w->moe_topk, hidden, stream);
+        routed = moe_gather_beside(w->shared_w13 ? shares.down : 0, b.f_normed, b.pair_row, b.a1, b.a1_sf, w->act_scale_in, m, w->moe_topk, hidden, stream);
     if (w->shared_w13) WUDA_CUDA(cudaStreamWaitEvent(main_stream, side->done[1], 0));   // join
     if (routed != WUDA_OK) return routed;
     WUDA_STAGE(wuda_gemm_nvfp4_grouped(b.a1, b.a1_sf, w->act_scale_in, w->w13, w->w13_sf, w->w13_gs, b.group_expert, b.num_groups, b.row_token, b.h,

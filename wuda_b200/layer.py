@@ -167,20 +167,16 @@ class DecoderLayer:
             self.pre_ws = torch.empty(lib.wuda_mhc_pre_workspace_bytes(max_batch, hidden), dtype=torch.uint8, device=dev)
             self.gate_logits = torch.empty(max_batch, ffn.experts_total, dtype=torch.float32, device=dev)
             self.y = torch.empty(max_batch, hidden, dtype=torch.bfloat16, device=dev)
-            # the SM shares the C++ sequence gives the GEMMs it runs side by side (wuda_b200/csrc/layer_decode.cu): with
-            # them this Python-sequenced form adds in the same order and is bit-identical to it
-            n = lib.wuda_num_sms()
-            first = n * 5 // 16
-            attention.sm_split = (first, n - first) if first > 8 else (n, n)
+            # the SM shares the C++ sequence gives the GEMMs it runs side by side: with them this Python-sequenced form adds
+            # in the same order and is bit-identical to it
+            attention.sm_split = self._sm_shares(1)[:2]
 
-    def _shared_sm_split(self, m):
-        """(SMs of w1|w3, SMs of w2) of the shared expert beside the router."""
-        n, inter = lib.wuda_num_sms(), self.ffn.shared.inter
-        split = 16 if m <= 16 else 12 if m <= 32 else 8 if m <= 64 else 6
-        left, tiles = n - -(-self.ffn.experts_total // 128) * split, -(-2 * inter // 128)
-        up = left // tiles * tiles if left >= tiles else n - 32 if n > 64 else n
-        down = -(-self.hidden // 128)
-        return up, down if inter <= 16 * 128 and down <= up else up
+    def _sm_shares(self, m):
+        """SMs of the front projection's FP8 and BF16 segment, the router projection, the shared expert's w1|w3 and w2."""
+        shares, shared = (ctypes.c_int32 * 5)(), self.ffn.shared
+        check(lib.wuda_layer_sm_shares(lib.wuda_num_sms(), m, self.hidden, shared.inter if shared is not None else 0,
+                                       self.ffn.experts_total, shares))
+        return tuple(shares)
 
     # ---- the C++ launch sequence
     def _init_native(self, dev):
@@ -271,7 +267,7 @@ class DecoderLayer:
         self.route_indices = idx
         shared = None
         if f.shared is not None:   # on the SM shares wuda_layer_decode gives the shared expert beside the router
-            shared = f.shared.forward(normed, sm_split=self._shared_sm_split(m))
+            shared = f.shared.forward(normed, sm_split=self._sm_shares(m)[3:])
         y = self.runner.forward(normed, rw, idx, shared=shared, y=self.y[:m])
         return ops.mhc_post_out(y, x, pre["post"], pre["comb"], self.out[:m])
 
