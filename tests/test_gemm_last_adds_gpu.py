@@ -26,3 +26,17 @@ def test_exact_bits(wuda, kind, m, n, k):
 @pytest.mark.parametrize("kind", ["bf16", "fp8", "fp8_pow2"])
 def test_order(wuda, kind, m, n, k):
     check_order(wuda, kind, m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", [(8, 1152, 7168), (8, 1280, 7168), (16, 1152, 7168), (16, 1280, 7168), (16, 1408, 7168), (16, 1536, 7168),
+                                   (16, 2048, 4864), (16, 2048, 4608)])
+@pytest.mark.parametrize("kind", KINDS)
+def test_two_quads_per_thread(wuda, kind, m, n, k):
+    """Either side of whole ranges (9 and 10 weight tiles on 148 SMs); general FP8 scales also of 13 ranges per tile and of four units per range."""
+    test_exact_bits(wuda, kind, m, n, k)
+    if kind == "fp8":
+        args, ref = operands(kind, m, n, k, seed=m + n)
+        args = [x.cuda() for x in args]
+        for _ in range(20):
+            got = wuda.fp8_gemm(*args)
+        assert torch.equal(got.cpu(), ref.float().bfloat16())

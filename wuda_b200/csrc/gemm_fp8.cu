@@ -75,6 +75,7 @@ struct Params {
     int a_rows;                // M rounded up to 16
     int stages;
     int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each
+    int last_adds;             // .. or by the one that completes the tile's counter
     int vec_scales;            // rows of a_scales can be read 16 bytes at a time
     // grouped form: weight tile t belongs to group t / group_tiles and reads the activations'
     // columns [group * K, (group + 1) * K); a_kb_total = K blocks in an activation row
@@ -426,7 +427,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 if (p.sliced) {
                     // (the last arrival wraps the tile's counter back to zero: gemm_tc.cuh)
                     const gemmtc::Holders h = unpack_holders(held, seg);
-                    if (M_PAD == 16 && gemmtc::last_adds(p.M, 32 * kEpiWarps)) {
+                    if (M_PAD == 16 && p.last_adds) {
                         if (et == 0) *arrived_last = inc_acq_rel_gpu(p.flags + tile, h.count() - 1) == h.count() - 1;
                         epi_bar_sync();
                         if (*arrived_last)
@@ -543,7 +544,7 @@ gemm_fp8_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant
                 ++tile;
             }
         }
-        if (p.sliced && !(M_PAD == 16 && gemmtc::last_adds(p.M, 32 * kEpiWarps))) {
+        if (p.sliced && !(M_PAD == 16 && p.last_adds)) {
 #pragma unroll 1
             for (int i = 0; i < seg; ++i) {
                 if (et == 0 && alive) await_word(p.flags + tile0 + i, [](int v) { return v == 0; }, abort_flag, p.status);
@@ -591,6 +592,9 @@ static int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, Params& p,
     const int sms = gemm_sms(dev);
     const int grid = gemmtc::grid_of(units, p.n_tiles, M_PAD, sms);
     p.sliced = !p.tp_peer_inbox && gemmtc::slice_wise(grid, p.n_tiles, M_PAD);     // (the two-rank form needs a finished tile in one CTA)
+    // (Nine rows and more: not with 13 ranges per tile either, 1280 / 1408 x 7168 at 16 rows 10.5 / 9.2 us, in slices 8.8 / 9.0; nor with
+    // short ranges, 4096 x 2048 0.5 us longer.)
+    p.last_adds = gemmtc::last_arrival_adds(p.M, 32 * kEpiWarps, grid, p.n_tiles) && (p.M <= 8 || (grid < 13 * p.n_tiles && units >= 4ll * grid));
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(kThreads), smem, stream, w_map, a_map, p));
     return WUDA_OK;
 }

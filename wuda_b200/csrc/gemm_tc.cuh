@@ -22,7 +22,7 @@
 //     CTA with the tile's start adds them in CTA order - it comes to that tile last, the partial was finished first.
 //     Few tiles ("sliced"): every CTA leaves the partial sums of its one or two tiles, and once a tile's counter is
 //     complete each of its CTAs adds one slice of it over all partials - instead of one CTA adding up to fifteen whole
-//     partials one after the other (with few rows the CTA that completes the counter adds the tile, last_adds()).  The order of the additions is CTA order either way and part of the results (it
+//     partials one after the other (with few rows the CTA that completes the counter adds the tile, last_arrival_adds()).  The order of the additions is CTA order either way and part of the results (it
 //     moves single roundings of the fp32 sums, and 4-bit quantisation behind them makes 4e-3 of a layer's output of
 //     that): it depends on the shape and the SM count alone, not on timing.
 //   * before it waits for the kernel ahead (programmatic launch) a CTA asks L2 for its first weight tiles, so a chain
@@ -72,6 +72,7 @@ struct Params {
     int a_rows;                // M rounded up to 16
     int stages;
     int sliced;                // a tile's partial sums are added by all of its CTAs, a slice each (even slices: how many CTAs)
+    int last_adds;             // .. or by the one that completes the tile's counter
     // power-of-two scaled kinds
     const float* a_scales;     // [M, scale_cols]
     const float* w_scales;     // [n_tiles, kb] (FP8 weights)
@@ -270,11 +271,6 @@ __device__ __forceinline__ void add_slice(const float* scratch, int64_t slot_flo
         }
     }
 }
-
-// Few activation rows: a sliced tile has no more than two quads of sums per epilogue thread, which then are one round of loads
-// however few CTAs share them.  The CTA that arrives last at the tile's counter adds the whole tile, right there, and nobody
-// has to wait for the others: FP8 2112 x 7168 at one row, plain calls, 9.0 -> 8.0 us.
-__device__ __forceinline__ bool last_adds(int M, int threads) { return (M + 3) / 4 * kTileN <= 2 * threads; }
 
 template <Kind KIND, int M_PAD>
 __global__ void __launch_bounds__(Layout<KIND, M_PAD>::kThreads, 1)
@@ -731,7 +727,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
                 // The last arrival wraps the tile's counter back to zero, which is what the others wait for, once they have
                 // nothing else to do.  No CTA arrives at a counter twice in a launch, the next launch's arrive after this one.
                 const Holders h = holders(seg);
-                if (M_PAD == 16 && last_adds(p.M, kEpi)) {
+                if (M_PAD == 16 && p.last_adds) {
                     if (et == 0) *arrived_last = inc_acq_rel_gpu(p.flags + tile, h.count() - 1) == h.count() - 1;
                     epi_sync();
                     if (*arrived_last)
@@ -805,7 +801,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
             if (kb == p.kb) kb = 0, ++tile;
             ++seg;
         }
-        if (!kEven && p.sliced && !(M_PAD == 16 && last_adds(p.M, kEpi))) {
+        if (!kEven && p.sliced && !(M_PAD == 16 && p.last_adds)) {
 #pragma unroll 1
             for (uint32_t i = 0; i < seg; ++i) slice(i);
         }
@@ -824,10 +820,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant_
 // hold parts of two tiles take part in two additions, each behind that tile's last CTA: with 17 to 64 rows that pays from five
 // ranges per tile on (FP8 4096 x 7168 at 64 rows, 148 ranges of 32 tiles: in slices 14.1 us, by the CTA with the tile's start 12.7; BF16
 // 2624 x 7168, 102 ranges of 21: 14.0, 13.2), while at 128 rows the slices win from three on (the same two 18.0 / 18.4 and 17.6 / 19.0).
-// The order of additions is the same.
+// The order of additions is the same.  (Either side at 17 to 64 rows of 4096 / 4608 / 5120 x 7168 and 4096 x 2048 / 4096, all formats: in slices
+// 0.4 to 2.2 us longer.)
 inline bool slice_wise(int grid, int n_tiles, int m_pad) {
     const int least = (m_pad == 32 || m_pad == 64) && grid % n_tiles != 0 ? 5 : 3;
     return grid >= least * n_tiles && grid + n_tiles <= kMaxGrid;
+}
+// Few activation rows: a sliced tile has one quad of sums per epilogue thread, which is one round of loads however few CTAs share
+// them.  The CTA that arrives last at the tile's counter adds the whole tile, right there, and nobody has to wait for the
+// others: FP8 2112 x 7168 at one row, plain calls, 9.0 -> 8.0 us; 128 to 4096 wide, 1 to 4 rows (general FP8 scales, with twice the threads, 8),
+// 0.2 to 1.3 us.  With two quads the second round over up to sixteen partials costs more than the one wait of a CTA whose range is part of
+// one tile (up to 1152 x 7168, 5 to 8 rows, 0.3 to 0.9 us), but less than the two waits of one that holds parts of two tiles
+// (1280 to 4096 x 7168 0.3 to 0.9 us).
+inline bool last_arrival_adds(int m, int threads, int grid, int n_tiles) {
+    const int quads = (m + 3) / 4 * kTileN;
+    return quads <= threads || (quads <= 2 * threads && grid % n_tiles != 0);
 }
 // Even slices: CTAs per tile, as many as the SMs hold when that is at least three (and every one gets a unit), else none.
 inline int even_split(int n_tiles, int kb, int sms) {
@@ -858,6 +865,7 @@ int launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const CUtensorMap
     } else {
         p.sliced = !p.group_expert && slice_wise(grid, p.n_tiles, M_PAD);
     }
+    p.last_adds = last_arrival_adds(p.M, 32 * L::kEpiWarps, grid, p.n_tiles);
     WUDA_CUDA(launch_pdl(kernel, dim3(grid), dim3(L::kThreads), L::total(stages, p.a_rows), stream, w_map, a_map, wsf_map, asf_map, p));
     return WUDA_OK;
 }
