@@ -18,4 +18,5 @@ def _running_the_build_module():
 if not _running_the_build_module():
     from ._lib import WudaError, lib, LIB_PATH  # noqa: F401
     from .ops import *  # noqa: F401,F403
+    from .ops import _fast  # noqa: F401
     from .shims import *  # noqa: F401,F403

@@ -14,9 +14,6 @@ if not os.path.exists(LIB_PATH):
         "wuda_b200: %s is missing. Build it with `python -m wuda_b200.build` "
         "(needs nvcc); there is no fallback implementation." % LIB_PATH)
 
-if not os.path.exists(os.path.join(_HERE, "_fast.so")):
-    raise ImportError("wuda_b200: _fast.so is missing. Build it with `python -m wuda_b200.build`.")
-
 lib = ctypes.CDLL(LIB_PATH)
 
 c_int, c_i64, c_vp, c_float = ctypes.c_int, ctypes.c_int64, ctypes.c_void_p, ctypes.c_float

@@ -4,8 +4,8 @@ nvcc cross-compiles without a GPU, so this runs anywhere the CUDA toolkit is pre
 The library links the static CUDA runtime and resolves the one driver function it needs
 (cuTensorMapEncodeTiled) at run time, so it also loads where no driver is installed.
 
-wuda_b200/_fast.so (csrc/fast_ops.cpp, g++) is the operators' native call path from Python; it is built against the installed
-torch and loads the library's entry points by name.
+wuda_b200/_fast.<interpreter>-<torch>.so (csrc/fast_ops.cpp, g++) is the operators' native call path from Python; it is built against
+the installed torch, which its name says, and loads the library's entry points by name.
 """
 import os
 import subprocess
@@ -14,7 +14,6 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libwuda_b200.so")
-FAST = os.path.join(HERE, "_fast.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 NVCC_FLAGS = [
@@ -36,21 +35,23 @@ def headers():
 
 
 def build_fast(force=False):
-    src = os.path.join(CSRC, "fast_ops.cpp")
-    newest = max(os.path.getmtime(p) for p in (src, os.path.join(HERE, "..", "include", "wuda_b200.h")))
-    if not force and os.path.exists(FAST) and os.path.getmtime(FAST) >= newest:
-        return FAST
+    import runpy
     import sysconfig
     import torch
+    fast = os.path.join(HERE, runpy.run_path(os.path.join(HERE, "native_calls.py"))["file_name"]())   # (the package may not import yet)
+    src = os.path.join(CSRC, "fast_ops.cpp")
+    newest = max(os.path.getmtime(p) for p in (src, os.path.join(HERE, "..", "include", "wuda_b200.h")))
+    if not force and os.path.exists(fast) and os.path.getmtime(fast) >= newest:
+        return fast
     root = os.path.dirname(os.path.abspath(torch.__file__))
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     cmd = ([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
             "-D_GLIBCXX_USE_CXX11_ABI=%d" % torch._C._GLIBCXX_USE_CXX11_ABI] +
            ["-I" + p for p in (root + "/include", root + "/include/torch/csrc/api/include", cuda + "/include",
                                sysconfig.get_paths()["include"])] +
-           [src, "-o", FAST, "-L" + root + "/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
+           [src, "-o", fast, "-L" + root + "/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"])
     subprocess.check_call(cmd)
-    return FAST
+    return fast
 
 
 def build(force=False, verbose=False):

@@ -11,7 +11,7 @@ import functools
 
 import torch
 
-from . import _fast, _lib
+from . import _lib, native_calls
 from ._lib import WudaError, check, lib
 from .scratch import Scratch
 
@@ -23,6 +23,7 @@ __all__ = ["mqa_logits_fp4_decode_out", "mqa_logits_fp4_decode", "mqa_logits_fp8
 
 # The operators that a server calls by themselves try csrc/fast_ops.cpp first: checks, outputs and launch in one native call,
 # which does nothing and returns None for whatever it does not know or would have to refuse.
+_fast = native_calls.load()
 _fast.bind(lib._handle)
 
 NUM_INDEX_HEADS = 64
