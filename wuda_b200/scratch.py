@@ -41,7 +41,7 @@ class Scratch:
 
     def __init__(self, zeroed):
         self.zeroed = zeroed
-        self._streams = {}      # (device index, stream) -> what get() returns
+        self._streams = {}      # (device index, stream) -> what get() returns; csrc/fast_ops.cpp reads it, too
         self._flags = {}        # device index -> (blocks, flags handed out)
         self._captures = {}     # (device index, stream, capture) -> address of its flags
 
