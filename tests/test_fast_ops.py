@@ -27,7 +27,7 @@ def test_leaves_what_it_does_not_know_to_python(name):
         wuda.rmsnorm_quant(host, None)
 
 
-PYTHON = {"act_quant of a column slice", "fp8 exponent bytes"}      # cases of _cases() that the native path leaves to Python
+PYTHON = {"act_quant of a column slice", "fp8 exponent bytes", "fp4 exponent bytes"}      # cases of _cases() that the native path leaves to Python
 
 
 class Recorder:
@@ -73,6 +73,7 @@ def _cases():
     yield "fp4 given output", lambda: wuda.fp4_gemm(a, a_s, w4, w4_s, out=torch.empty(5, 256, device="cuda", dtype=torch.bfloat16))
     yield "bf16 given output", lambda: wuda.bf16_gemm(x, rnd(64, 1024).fill_(0.5).bfloat16(), out=torch.empty(5, 64, device="cuda"), status_word=status)
     yield "fp8 exponent bytes", lambda: wuda.fp8_gemm(a, a_s.to(torch.float8_e8m0fnu), w, w_s.to(torch.float8_e8m0fnu))
+    yield "fp4 exponent bytes", lambda: wuda.fp4_gemm(a, a_s.to(torch.float8_e8m0fnu), w4, w4_s)
     yield "fp8 parameter", lambda: wuda.fp8_gemm(a, a_s, torch.nn.Parameter(w, requires_grad=False), w_s)
     yield "fp4", lambda: wuda.fp4_gemm(a, a_s, w4, w4_s)
     yield "bf16", lambda: wuda.bf16_gemm(x, rnd(64, 1024).fill_(0.5).bfloat16())

@@ -292,11 +292,16 @@ PyObject* rope_quant(PyObject* const* a) {
 }
 
 // ---------------------------------------------------------------- GEMMs
+// Scales that are not fp32 (exponent bytes) are the Python functions' to convert: said without an exception, which costs 2.4 us of such a call's
+// 41 (fp8_gemm) or 26 (fp4_gemm).
+bool fp32_scales(PyObject* o) { return THPVariable_CheckExact(o) && THPVariable_Unpack(o).scalar_type() == ScalarType::Float; }
+
 // C of [.., n] for A of [.., k]; a given one is taken as the Python function takes it
 PyObject* result(PyObject* given, const Tensor& made) { return given == Py_None ? THPVariable_Wrap(made) : same(given); }
 
 // a, a_s, b, b_s, out, status_word, pow2_scales, streams
 PyObject* fp8_gemm(PyObject* const* p) {
+    if (!fp32_scales(p[1]) || !fp32_scales(p[3])) return same(Py_None);
     const Tensor& a = dense(p[0], ScalarType::Float8_e4m3fn);
     const Tensor& a_s = dense(p[1], ScalarType::Float);
     const Tensor& b = dense(p[2], ScalarType::Float8_e4m3fn);
@@ -316,6 +321,7 @@ PyObject* fp8_gemm(PyObject* const* p) {
 
 // a, a_s, b, b_s, out, status_word, streams
 PyObject* fp4_gemm(PyObject* const* p) {
+    if (!fp32_scales(p[1])) return same(Py_None);
     const Tensor& a = dense(p[0], ScalarType::Float8_e4m3fn);
     const Tensor& a_s = dense(p[1], ScalarType::Float);
     const Tensor& b = cuda_tensor(p[2]);
